@@ -145,6 +145,8 @@ struct anc_instance {
     std::vector<int8_t> dense;                    // host copy of dense couplings (tensor engine packs lazily)
     anc::TensorInstance tensor;                   // tensor-engine operands (built on first use)
     bool tensor_ready = false;
+    anc::PlanesInstance planes4;                  // operands of the planes kernel (built on first use)
+    bool planes4_ready = false;
     int per_wave[4] = {-1, -1, -1, -1};           // anneals per wave of each engine (ANC_ENGINE_*; -1: not queried)
     int cluster16_wave = -1;                      // anneals one wave of 16-CTA clusters runs (-1: not queried)
     uint64_t uid = g_next_uid.fetch_add(1);       // identifies the instance to the tables' flip record
@@ -458,6 +460,11 @@ int tuned_variant(anc_instance* I, int kernel, int nchains) {
     return it == g_kernel_tune.end() ? 0 : std::max(0, it->second.variant);
 }
 
+// Whether the planes kernel can run this instance, and whether AUTO considers it (not where the fp4 kernel runs).
+bool planes_candidate(const anc_instance* I) {
+    return !I->dense.empty() && anc::planes_supported(I->n, I->info.maxabs, I->info.hmax + int64_t(I->info.bmax));
+}
+
 // Flip fraction AUTO assumes: the caller's hint, else what the last host-output run of these tables on this instance
 // saw, else the prior.
 double flip_fraction(const anc_instance* I, const anc_tables* tb, const anc_run_opts* o) {
@@ -466,13 +473,27 @@ double flip_fraction(const anc_instance* I, const anc_tables* tb, const anc_run_
     return kPhiPrior;
 }
 
+// Engine of a launch. planes is set when the tensor engine is picked with the planes kernel: by AUTO, unless the caller
+// asked for an operand format, a compiled variant or a profile of the other kernels, or by tensor_kind.
 int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts* o, double* us = nullptr,
-                double* phi_used = nullptr) {
+                double* phi_used = nullptr, bool* planes = nullptr) {
     const int e = o ? o->engine : ANC_ENGINE_AUTO;
+    if (planes) *planes = e == ANC_ENGINE_TENSOR && o->tensor_kind == ANC_TENSOR_PLANES;
     if (e == ANC_ENGINE_PLAIN || e == ANC_ENGINE_TENSOR || e == ANC_ENGINE_CLUSTER) return e;
     const double phi = flip_fraction(I, tb, o);
     double est[4];
-    const int best = estimate_engines(I->n, I->K, nchains, tb->S, phi, fp4_candidate(I), engine_waves(I), est);
+    int best = estimate_engines(I->n, I->K, nchains, tb->S, phi, fp4_candidate(I), engine_waves(I), est);
+    const bool free_choice = !o || (o->tensor_kind == ANC_TENSOR_AUTO && o->kernel_variant == 0 && !o->profile);
+    if ((free_choice || o->tensor_kind == ANC_TENSOR_PLANES) && planes_candidate(I) && !fp4_candidate(I)) {
+        const double t = tb->S * anc::planes_step_us(I->n, I->info.maxabs, nchains);
+        if (t >= 0 && (est[ANC_ENGINE_TENSOR] < 0 || t < est[ANC_ENGINE_TENSOR])) {
+            est[ANC_ENGINE_TENSOR] = t;
+            if (est[best] < 0 || t < est[best] || best == ANC_ENGINE_TENSOR) {
+                best = ANC_ENGINE_TENSOR;
+                if (planes) *planes = true;
+            }
+        }
+    }
     if (us) std::copy(est, est + 4, us);
     if (phi_used) *phi_used = phi;
     return best;
@@ -488,6 +509,16 @@ int ensure_tensor(anc_instance* I) {
     return ANC_OK;
 }
 
+int ensure_planes(anc_instance* I, cudaStream_t st) {
+    if (I->planes4_ready) return ANC_OK;
+    std::string why;
+    const int rc = anc::planes_build(I->planes.p, I->K, I->nwj, I->n, I->bias.empty() ? nullptr : I->bias.data(),
+                                     I->info.maxabs, &I->planes4, st, &why);
+    if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "planes kernel setup: %s", why.c_str());
+    I->planes4_ready = true;
+    return ANC_OK;
+}
+
 // Launch on device outputs; no synchronisation. S_probe > 0 runs only the first S_probe steps of the schedule (the
 // run-time tuners' probes).
 int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, int nchains, const anc_run_opts* o,
@@ -498,20 +529,20 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
     int32_t hclamp = 0;
     int rc = resolve_clamp(I, tb, o, &hclamp);
     if (rc) return rc;
-    const int engine = pick_engine(I, tb, nchains, o);
+    bool planes = false;
+    const int engine = pick_engine(I, tb, nchains, o, nullptr, nullptr, &planes);
     if (engine == ANC_ENGINE_TENSOR) {
-        if (!anc::tensor_supported(I->n, I->K, nchains))
+        if (planes ? !planes_candidate(I) : !anc::tensor_supported(I->n, I->K, nchains))
             return fail(ANC_EINVAL, "tensor engine does not support n=%d K=%d", I->n, I->K);
-        rc = ensure_tensor(I);
+        rc = planes ? ensure_planes(I, st) : ensure_tensor(I);
         if (rc) return rc;
         const int forced = o ? o->kernel_variant : 0;
-        if (forced > anc::kF4Variants)
-            return fail(ANC_EINVAL, "kernel_variant %d out of range: the fp4 kernel has %d variants", forced,
-                        anc::kF4Variants);
+        if (forced > (planes ? 0 : anc::kF4Variants))
+            return fail(ANC_EINVAL, "kernel_variant %d out of range: the %s kernel has %d variants", forced,
+                        planes ? "planes" : "fp4", planes ? 0 : anc::kF4Variants);
         anc::TensorRun r{};
         r.tab = dev_tables(tb);
         if (S_probe > 0) r.tab.S = std::min(r.tab.S, S_probe);
-        r.variant = forced > 0 ? forced - 1 : tuned_variant(I, ANC_KERNEL_TENSOR_FP4, nchains);
         r.seed = seed;
         r.trial_offset = off;
         r.nchains = nchains;
@@ -523,9 +554,18 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
         r.out_flips = reinterpret_cast<int64_t*>(out.fl);
         r.out_trace = out.trace;
         r.out_h = out.h;
+        r.wait_ns = g_wait_ns.load();
+        if (planes) {
+            I->prof_ctas = 0;
+            std::string why;
+            rc = anc::planes_run(&I->planes4, r, st, &why);
+            if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "tensor engine: %s", why.c_str());
+            g_last_kernel = ANC_KERNEL_TENSOR_PLANES;
+            return ANC_OK;
+        }
+        r.variant = forced > 0 ? forced - 1 : tuned_variant(I, ANC_KERNEL_TENSOR_FP4, nchains);
         r.prof = nullptr;
         r.kind = o ? o->tensor_kind : ANC_TENSOR_AUTO;
-        r.wait_ns = g_wait_ns.load();
         I->prof_ctas = 0;
         if (o && o->profile) {
             anc::TensorGeometry geo;
@@ -640,7 +680,9 @@ int tune_sparse(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
 int tune_kernel(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, int nchains, const anc_run_opts* o,
                 const OutPtrs& out) {
     if (o && o->kernel_variant > 0) return ANC_OK;
-    const int engine = pick_engine(I, tb, nchains, o);
+    bool planes = false;
+    const int engine = pick_engine(I, tb, nchains, o, nullptr, nullptr, &planes);
+    if (planes) return ANC_OK;     // one compiled variant per geometry
     int kernel = 0, nv = 1, nprobe = nchains;
     if (engine == ANC_ENGINE_PLAIN && I->K != 0) {
         size_t smem = 0;
@@ -688,7 +730,7 @@ int tune_kernel(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
             CK(cudaEventElapsedTime(&ms, I->ev0, I->ev1));
             if (I->tensor_ready && I->tensor.last_err) {
                 std::string why;
-                rc = anc::tensor_check_error(&I->tensor, st, &why);
+                rc = anc::tensor_check_error(I->tensor.last_err, st, &why);
                 I->tensor.last_err = nullptr;
                 if (rc == -3) return fail(ANC_ETIMEOUT, "tensor engine (tuning probe): %s", why.c_str());
                 if (rc) return fail(ANC_ECUDA, "tensor engine (tuning probe): %s", why.c_str());
@@ -749,8 +791,15 @@ int run_host_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, 
     }
     if (I->tensor_ready && I->tensor.last_err) {
         std::string why;
-        rc = anc::tensor_check_error(&I->tensor, st, &why);
+        rc = anc::tensor_check_error(I->tensor.last_err, st, &why);
         I->tensor.last_err = nullptr;
+        if (rc == -3) return fail(ANC_ETIMEOUT, "tensor engine: %s", why.c_str());
+        if (rc) return fail(ANC_ECUDA, "tensor engine: %s", why.c_str());
+    }
+    if (I->planes4.last_err) {
+        std::string why;
+        rc = anc::tensor_check_error(I->planes4.last_err, st, &why);
+        I->planes4.last_err = nullptr;
         if (rc == -3) return fail(ANC_ETIMEOUT, "tensor engine: %s", why.c_str());
         if (rc) return fail(ANC_ECUDA, "tensor engine: %s", why.c_str());
     }
@@ -1049,7 +1098,10 @@ int anc_instance_get_info(const anc_instance* I, anc_instance_info* info) {
 }
 
 void anc_instance_destroy(anc_instance* I) {
-    if (I) anc::tensor_free_instance(&I->tensor);
+    if (I) {
+        anc::tensor_free_instance(&I->tensor);
+        anc::planes_free(&I->planes4);
+    }
     delete I;
 }
 

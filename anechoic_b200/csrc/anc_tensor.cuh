@@ -30,7 +30,7 @@ struct TensorInstance {
 constexpr int kTensorProfSlots = 56;
 
 // Operand format of the field update: int8 (any |J| <= 127) or packed fp4 e2m1 (|J| <= 1, NP = 2048).
-constexpr int TENSOR_KIND_AUTO = 0, TENSOR_KIND_INT8 = 1, TENSOR_KIND_FP4 = 2;
+constexpr int TENSOR_KIND_AUTO = 0, TENSOR_KIND_INT8 = 1, TENSOR_KIND_FP4 = 2, TENSOR_KIND_PLANES = 3;
 
 struct TensorRun {
     DevTables tab;
@@ -76,8 +76,27 @@ void stream_permutation(int np, std::vector<int>* p);
 int stream_width();
 int stream_wave_chains();
 int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm, cudaStream_t st, std::string* why);
+// Planes kernel (tensor_planes.cu): J on chip as one (|J| <= 4) or two e2m1 planes, NP = 2048 .. 6144 (one plane) or
+// 4096 (two).
+struct PlanesInstance {
+    int n = 0, R = 0, W = 0;
+    uint8_t* d_J = nullptr;      // [W][256 RP][128 RP] packed e2m1
+    int32_t* d_bias = nullptr;   // bias at permuted column
+    void* d_ws = nullptr;        // error word, flags, exchange buffers
+    size_t ws_bytes = 0;
+    int* last_err = nullptr;     // error word of the last launch
+};
+// field_bound: max_y sum_x |J_xy| + max |b|
+bool planes_supported(int n, int maxabs, int64_t field_bound);
+// measured device time of one step of nchains anneals (all waves), in microseconds
+double planes_step_us(int n, int maxabs, int nchains);
+// from the plain engine's bit planes on the device ([K][np][nwj])
+int planes_build(const uint32_t* bits, int K, int nwj, int n, const int32_t* bias, int maxabs, PlanesInstance* out,
+                 cudaStream_t st, std::string* why);
+int planes_run(PlanesInstance* pi, const TensorRun& r, cudaStream_t st, std::string* why);
+void planes_free(PlanesInstance* pi);
 // After the stream has reached the launch: -3 if a bounded device wait expired, 0 otherwise.
-int tensor_check_error(TensorInstance* ti, cudaStream_t st, std::string* why);
+int tensor_check_error(const int* err, cudaStream_t st, std::string* why);
 void tensor_free_instance(TensorInstance* ti);
 
 }  // namespace anc

@@ -43,6 +43,10 @@ extern "C" {
                                an 8-CTA cluster too (gpu/onsager_v2_20261007/src/sca_gpu.cu:223-295) */
 
 #define ANC_TENSOR_AUTO 0   /* fp4 when exact for the instance (NP = 2048, |J| <= 1, small fields), else int8 */
+#define ANC_TENSOR_PLANES 3 /* kind::mxf4 with J as one or two e2m1 planes kept in shared memory (|J| <= 4: n <= 6144;
+                              |J| <= 7: n <= 4096; max_y sum_x |J_xy| + max |b| < 2^16, EINVAL otherwise); exact.
+                              ANC_ENGINE_AUTO picks it where it is estimated fastest; ANC_ENGINE_TENSOR runs it only
+                              when this kind is asked for */
 #define ANC_TENSOR_INT8 1   /* tcgen05.mma kind::i8, int32 accumulation (any K) */
 #define ANC_TENSOR_FP4 2    /* tcgen05.mma kind::mxf4 on packed e2m1 with unit block scales, fp32 accumulation;
                               exact because J in {-1,0,1}, dS in {0,+-1,+-2} and |h| < 2^14 (EINVAL otherwise) */
@@ -311,6 +315,7 @@ ANC_API double anc_last_device_ms(void);
 #define ANC_KERNEL_PLAIN 1        /* bit-column engine */
 #define ANC_KERNEL_TENSOR_INT8 2  /* tcgen05 kind::i8 engine */
 #define ANC_KERNEL_TENSOR_FP4 3   /* tcgen05 kind::mxf4 engine */
+#define ANC_KERNEL_TENSOR_PLANES 5 /* tcgen05 kind::mxf4 engine, J as one or two e2m1 planes */
 #define ANC_KERNEL_PLAIN_CLUSTER 4 /* bit-column engine, one anneal per 8-CTA cluster */
 ANC_API int anc_last_kernel(void);
 
