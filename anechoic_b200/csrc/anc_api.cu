@@ -90,6 +90,9 @@ int pad_np(int n) { return std::max(2048, ((n + 255) / 256) * 256); }
 //            streaming 99.5 (measured 99.5 at NP = 10240 and 98 at NP = 16384: bound by its step latency, not by
 //            reading J)
 // Each engine advances a fixed number of anneals at once (per_wave); a launch of more takes further waves.
+// Least step AUTO assumes for the fp4 kernel (3.5 - 4.6 us measured up to four replica groups): a 1-bit batch that flips
+// few spins (the temperature-scaled schedules, phi about 0.11) stays on the plain engine, whose estimate is 5.9 us there.
+constexpr double kFp4FloorUs = 5.95;
 constexpr double kPhiPrior = 0.25;   // flip fraction assumed before any run of these tables on this instance
 
 double plain_step_us(int n, int K, double phi) {
@@ -402,7 +405,8 @@ int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t 
     return ANC_OK;
 }
 
-// Whether the tensor engine would run this instance on the fp4 kernel (tensor_fp4_eligible, from the host statistics).
+// Whether the tensor engine runs this instance on the fp4 kernel (the planes kernel at NP = 2048 with J in {-1, 0, 1} and
+// fields below 2^14).
 bool fp4_candidate(const anc_instance* I) {
     return !I->dense.empty() && I->np == 2048 && I->info.maxabs <= 1 &&
            I->info.hmax + int64_t(I->info.bmax) < (int64_t(1) << 14);
@@ -418,8 +422,8 @@ const int* engine_waves(anc_instance* I) {
         if (plain_residency(I, plain_P(I->np), &smem, &stream, &per_sm) == ANC_OK) w[ANC_ENGINE_PLAIN] = per_sm * I->sms;
         int t = 0;
         if (!I->dense.empty() && anc::tensor_supported(I->n, I->K, 1) &&
-            anc::tensor_wave_chains(I->n, fp4_candidate(I), &t) == 0)
-            w[ANC_ENGINE_TENSOR] = std::max(0, t);
+            anc::tensor_wave_chains(I->n, &t) == 0)
+            w[ANC_ENGINE_TENSOR] = std::max(0, fp4_candidate(I) ? anc::planes_wave_chains(I->n, 1) : t);
         int c = 0;
         if (anc::plain_cluster_supported(I->K, I->np) && anc::plain_cluster_max_active(&c) == 0)
             w[ANC_ENGINE_CLUSTER] = std::max(0, c);
@@ -484,13 +488,16 @@ int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts
     double est[4];
     int best = estimate_engines(I->n, I->K, nchains, tb->S, phi, fp4_candidate(I), engine_waves(I), est);
     const bool free_choice = !o || (o->tensor_kind == ANC_TENSOR_AUTO && o->kernel_variant == 0 && !o->profile);
-    if ((free_choice || o->tensor_kind == ANC_TENSOR_PLANES) && planes_candidate(I) && !fp4_candidate(I)) {
-        const double t = tb->S * anc::planes_step_us(I->n, I->info.maxabs, nchains);
+    if ((free_choice || o->tensor_kind == ANC_TENSOR_PLANES) && planes_candidate(I)) {
+        // where the fp4 kernel runs, it is the planes kernel by another name: only its estimate changes, and not below
+        // kFp4Floor
+        const bool fp4 = fp4_candidate(I) && (!o || o->tensor_kind != ANC_TENSOR_PLANES);
+        const double t = tb->S * std::max(fp4 ? kFp4FloorUs : 0.0, anc::planes_step_us(I->n, I->info.maxabs, nchains));
         if (t >= 0 && (est[ANC_ENGINE_TENSOR] < 0 || t < est[ANC_ENGINE_TENSOR])) {
             est[ANC_ENGINE_TENSOR] = t;
             if (est[best] < 0 || t < est[best] || best == ANC_ENGINE_TENSOR) {
                 best = ANC_ENGINE_TENSOR;
-                if (planes) *planes = true;
+                if (planes) *planes = !fp4;
             }
         }
     }
@@ -534,7 +541,12 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
     if (engine == ANC_ENGINE_TENSOR) {
         if (planes ? !planes_candidate(I) : !anc::tensor_supported(I->n, I->K, nchains))
             return fail(ANC_EINVAL, "tensor engine does not support n=%d K=%d", I->n, I->K);
-        rc = planes ? ensure_planes(I, st) : ensure_tensor(I);
+        const int kind = o ? o->tensor_kind : ANC_TENSOR_AUTO;
+        if (kind == ANC_TENSOR_FP4 && !fp4_candidate(I))
+            return fail(ANC_EINVAL, "tensor engine: the fp4 kernel needs NP = 2048, |J| <= 1 and max|b| + max_y sum_x "
+                                    "|J_xy| < 16384");
+        const bool fp4 = !planes && fp4_candidate(I) && kind != ANC_TENSOR_INT8;
+        rc = planes || fp4 ? ensure_planes(I, st) : ensure_tensor(I);
         if (rc) return rc;
         const int forced = o ? o->kernel_variant : 0;
         if (forced > (planes ? 0 : anc::kF4Variants))
@@ -555,22 +567,13 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
         r.out_trace = out.trace;
         r.out_h = out.h;
         r.wait_ns = g_wait_ns.load();
-        if (planes) {
-            I->prof_ctas = 0;
-            std::string why;
-            rc = anc::planes_run(&I->planes4, r, st, &why);
-            if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "tensor engine: %s", why.c_str());
-            g_last_kernel = ANC_KERNEL_TENSOR_PLANES;
-            return ANC_OK;
-        }
-        r.variant = forced > 0 ? forced - 1 : tuned_variant(I, ANC_KERNEL_TENSOR_FP4, nchains);
+        r.variant = !fp4 ? 0 : forced > 0 ? forced - 1 : tuned_variant(I, ANC_KERNEL_TENSOR_FP4, nchains);
         r.prof = nullptr;
-        r.kind = o ? o->tensor_kind : ANC_TENSOR_AUTO;
         I->prof_ctas = 0;
         if (o && o->profile) {
             anc::TensorGeometry geo;
             if (anc::tensor_geometry(I->n, nchains, &geo) != 0) return fail(ANC_ECUDA, "tensor geometry query failed");
-            const int ctas = std::max(geo.ctas, 16 * ((nchains + 127) / 128));
+            const int ctas = std::max(geo.ctas, anc::planes_max_ctas());
             CK(I->w_prof.ensure(size_t(ctas) * anc::kTensorProfSlots));
             CK(cudaMemsetAsync(I->w_prof.p, 0, size_t(ctas) * anc::kTensorProfSlots * sizeof(long long), st));
             r.prof = I->w_prof.p;
@@ -578,10 +581,14 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
             I->prof_S = tb->S;
         }
         std::string why;
-        rc = anc::tensor_run(&I->tensor, r, st, &why);
+        rc = planes || fp4 ? anc::planes_run(&I->planes4, r, st, &why) : anc::tensor_run(&I->tensor, r, st, &why);
         if (rc == -3) return fail(ANC_ETIMEOUT, "tensor engine: %s", why.c_str());
         if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "tensor engine: %s", why.c_str());
-        g_last_kernel = I->tensor.last_kind == anc::TENSOR_KIND_FP4 ? ANC_KERNEL_TENSOR_FP4 : ANC_KERNEL_TENSOR_INT8;
+        if (planes || fp4) {
+            I->tensor.last_ctas = I->planes4.last_ctas;     // the profile's geometry fields
+            I->tensor.last_cluster = 1;
+        }
+        g_last_kernel = planes ? ANC_KERNEL_TENSOR_PLANES : fp4 ? ANC_KERNEL_TENSOR_FP4 : ANC_KERNEL_TENSOR_INT8;
         return ANC_OK;
     }
     anc::PlainJob job = make_job(I, tb, seed, off, nchains, hclamp, out);
@@ -728,10 +735,10 @@ int tune_kernel(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
             CK(cudaEventRecord(I->ev1, st));
             CK(cudaEventSynchronize(I->ev1));
             CK(cudaEventElapsedTime(&ms, I->ev0, I->ev1));
-            if (I->tensor_ready && I->tensor.last_err) {
+            if (I->planes4.last_err) {
                 std::string why;
-                rc = anc::tensor_check_error(I->tensor.last_err, st, &why);
-                I->tensor.last_err = nullptr;
+                rc = anc::tensor_check_error(I->planes4.last_err, st, &why);
+                I->planes4.last_err = nullptr;
                 if (rc == -3) return fail(ANC_ETIMEOUT, "tensor engine (tuning probe): %s", why.c_str());
                 if (rc) return fail(ANC_ECUDA, "tensor engine (tuning probe): %s", why.c_str());
             }

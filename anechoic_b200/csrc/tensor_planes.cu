@@ -1,6 +1,5 @@
 // Batched engine for replicas sharing a dense J with J held on chip as one or two packed e2m1 planes: NP = 2048 ..
-// 6144 in any multiple of 256, couplings up to 4 bits. It generalises the fp4 kernel (tensor_engine.cu: NP = 2048,
-// |J| <= 1, 16 lanes per CTA) over the number of rounds, the lanes per CTA and the planes.
+// 6144 in any multiple of 256, couplings up to 4 bits. At NP = 2048 with |J| <= 1 it is what the API calls the fp4 kernel.
 //
 // Planes. Every |J| in {0, 1, 2, 3, 4, 6} is one e2m1 value; 5 = 4 + 1 and 7 = 6 + 1 take a second plane with entries
 // in {0, +-1}. The field update is J dS = J_0 dS + J_1 dS: the same dS tile multiplied by each plane's slice into the
@@ -13,7 +12,7 @@
 // 128*RP bytes = RP tiles of 128 bytes (256 columns); a CTA's J slice (N = 2 CH rows per plane, CH = LT*RP padded to 8)
 // stays in shared memory for the whole launch. A group takes 128 / LT CTAs, so the grid holds 148 LT / 128 groups.
 //
-// Per step (the golden model's step, sca_ref_bias.hpp:44-68), as the fp4 kernel does it: decide from the f32 fields in
+// Per step (the golden model's step, sca_ref_bias.hpp:44-68): decide from the f32 fields in
 // TMEM; publish dS nibbles and an n_lin byte per thread through L2; make the next step's draws; fetch the group's dS tile
 // by tile (cp.async, an NS-deep ring, the own tile first) as the tiles' publications appear in the poller warp's shared
 // mirror; 4 MMAs per tile and plane. Each tile has one counter, which every CTA owning columns of it increments with
@@ -32,6 +31,8 @@
 //   n_lin as coalesced reductions into 8 sums per replica, wider dS stores                                   9.1 / 5.9
 //   two MMA warps, each with its own accumulator (the decision adds the two)                                 7.4 / 5.2
 //   fewer lanes per thread where the groups fit                                                              7.4 / 4.6
+// n = 2000, +-1, 1024 anneals: 8.7 us a step with the fp4 kernel before (one MMA thread, decision warps waiting for their
+// copies), 6.15 here.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -84,6 +85,7 @@ struct PlanesParams {
     int32_t* out_trace;
     int32_t* out_h;
     int* err;
+    long long* prof;                    // [CTAs][kTensorProfSlots] clock64 totals of thread 0 and the first MMA warp, or null
 };
 
 template <int RP_, int LT_, int W_>
@@ -161,8 +163,11 @@ __device__ __forceinline__ void draw(Xoshiro (&rng)[G::LT], uint32_t (&pk)[G::CC
     }
 }
 
-// Decisions of the thread's columns 32 E .. of at most 32 (the fp4 kernel's arithmetic, f4_decide in tensor_engine.cu):
-// flip mask fm and mask lm of the linear band. The conversion 1.5*2^23 + x is exact for |x| < 2^22.
+// Decisions of the thread's columns 32 E .. of at most 32: flip mask fm and mask lm of the linear band -2T < z < 2T.
+//   r = floor((u16 - 32768) * 4T / 65536) = mulhi((u16 - 32768) << 16, 4T);
+//   s*h: the field in f32 with its sign flipped for s = -1 (bit 31 of ~sw), clamped when the range plan asks;
+//   z = s*h*65536 + q -/+ corr through the exact conversion 1.5*2^23 + x (|x| < 2^22): the low 16 bits of that encoding are
+//   x, so encoding << 16 = x * 65536 modulo 2^32.
 template <class G, int E, bool CLAMP>
 __device__ __forceinline__ void decide(uint32_t taddr, const uint32_t (&pk)[G::CC / 2], uint32_t sw, uint32_t dw,
                                        int32_t xs, int32_t twocorr, int32_t fourT, int32_t c1, uint32_t lw, float hclf,
@@ -365,6 +370,16 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int r = (warp & 3) * 32 + lane, hf = warp >> 2;
     uint32_t hph = 0u, q = 0;
     bool jready = false;
+    const bool prof = P.prof != nullptr;
+    long long pc[5] = {0, 0, 0, 0, 0}, pt = 0;     // phase totals (slots of kTensorProfSlots), the last mark
+    const long long loop0 = clock64();
+    auto mark = [&](int i) {
+        if (prof) {
+            const long long now = clock64();
+            if (i >= 0) pc[i] += now - pt;
+            pt = now;
+        }
+    };
 
     for (int g = gs0, gi = 0; g < P.ngroups; g += gstride, ++gi) {
         const uint32_t tbase = uint32_t(gi) * uint32_t(S + 2);
@@ -432,9 +447,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int t = m < S ? m : S - 1;
                 const int32_t fourT = __ldg(P.fourT + t), qv = __ldg(P.q + t), kconst = __ldg(P.kconst + t);
                 const int64_t kcorr = __ldg(P.kcorr + t);
+                mark(-1);
                 if (ok) ok = __all_sync(0xffffffffu, mbar_wait_for(bar_h, hph & 1u, err, kErrHready, P.wait_ns));
                 ++hph;
                 tc_fence_after();
+                mark(0);
                 const int32_t nlin_prev = nlin_next;
                 if (m >= 1 && writer && cs == 0 && hf == 0 && P.out_trace) P.out_trace[size_t(chain) * S + (m - 1)] = nlin_prev;
                 if (m == S) {
@@ -506,14 +523,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                     atomicAdd(P.nls + ((size_t(g) * 3 + uint32_t(m) % 3u) * kNlCopies + cs % kNlCopies) * kM + r, nl);
                 }
                 tc_fence_before();
+                mark(1);
                 asm volatile("bar.sync 1, %0;" ::"r"(kDW * 32) : "memory");
                 publish<G>(P, g, cs, tid);
+                mark(2);
                 const bool eok2 = !err_set(err);
                 if (active && m + 1 < S) draw<G>(rng, pk, R);
                 ok = ok && __all_sync(0xffffffffu, eok2);
+                mark(3);
                 nlin_next = exchange<G>(P, g, m, smem_u32(stages), bar_full, bar_empty, q, tid, r, rows, active,
                                                s_tile, tbase, rot, ok);
                 q += RP;
+                mark(4);
                 // every CTA of the group has published step m, so none reads step m - 1's sums any more; they become
                 // step m + 2's, whose writers wait for this CTA's publication of step m + 1
                 if (cs < kNlCopies && hf == 0)
@@ -538,12 +559,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int m = -1; m < S; ++m) {
                 mok = mok && __all_sync(0xffffffffu, !err_set(err));
                 int tk = tk0 < RP ? tk0 : tk0 - RP;
+                const long long c0 = prof ? clock64() : 0;
 #pragma unroll 1
                 for (int t0 = 0; t0 < RP; t0 += NS, q += NS) {
 #pragma unroll
                     for (int s0 = 0; s0 < NS; s0 += kMmaWarps) {
                         const uint32_t s = uint32_t(s0) + a;
+                        mark(-1);
                         if (mok) mok = __all_sync(0xffffffffu, mbar_wait_for(bar_full + 8 * s, (q / NS) & 1u, err, kErrFull, P.wait_ns));
+                        mark(0);
                         tc_fence_after();
                         if (lead) {
                             if (mok) {
@@ -566,6 +590,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 if (lead) mma_commit(bar_h);
                 __syncwarp();
+                if (prof) pc[1] += clock64() - c0;
             }
         } else if (warp == kPollWarp) {
             // ---------------- poller: lane t mirrors the counter of tile t ----------------
@@ -606,6 +631,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!jready) mbar_wait_for(bar_j, 0u, nullptr, 0, kWaitNs);
         mma_commit(bar_fin);
         mbar_wait_for(bar_fin, 0u, nullptr, 0, kWaitNs);
+    }
+    if (prof && lane == 0 && (warp == 0 || warp == kMmaWarp)) {
+        long long* dst = P.prof + size_t(blockIdx.x) * kTensorProfSlots;
+        if (warp == 0) {
+            for (int i = 0; i < 5; ++i) dst[i] = pc[i];
+        } else {
+            dst[5] = pc[0];
+            dst[6] = pc[1];
+            dst[8] = clock64() - loop0;
+        }
     }
     cp_async_wait(0);     // no copy may land in shared memory the CTA has released
     __syncthreads();
@@ -707,6 +742,15 @@ int sm_count() {
     return sms;
 }
 
+// Geometry of a launch: variant 0 by rule, 1 .. 3 force LT = 8, 4 or 2 (NP = 2048, one plane).
+const Config* launch_config(int R, int W, int ngroups, int sms, int variant) {
+    if (variant == 0) return planes_config(R, W, ngroups, sms);
+    const Config* cfg = planes_configs();
+    for (int i = 0; i < kConfigs; ++i)
+        if (cfg[i].rp == (R + 3) / 4 * 4 && cfg[i].w == W && cfg[i].lt == 16 >> variant && group_slots(cfg[i], sms) > 0) return &cfg[i];
+    return nullptr;
+}
+
 int planes_of(int maxabs) { return maxabs <= 4 ? 1 : 2; }
 
 }  // namespace
@@ -722,6 +766,14 @@ double planes_step_us(int n, int maxabs, int nchains) {
     const Config* c = planes_config(rounds_of(n), planes_of(maxabs), ngroups, sms);
     return c ? double((ngroups + group_slots(*c, sms) - 1) / group_slots(*c, sms)) * c->us : -1.0;
 }
+
+int planes_wave_chains(int n, int maxabs) {
+    const int sms = sm_count();
+    const Config* c = planes_config(rounds_of(n), planes_of(maxabs), 1 << 20, sms);     // many groups: the largest LT
+    return c ? group_slots(*c, sms) * kM : 0;
+}
+
+int planes_max_ctas() { return sm_count(); }
 
 int planes_build(const uint32_t* bits, int K, int nwj, int n, const int32_t* bias, int maxabs, PlanesInstance* out,
                  cudaStream_t st, std::string* why) {
@@ -753,7 +805,7 @@ int planes_build(const uint32_t* bits, int K, int nwj, int n, const int32_t* bia
 
 int planes_run(PlanesInstance* pi, const TensorRun& r, cudaStream_t st, std::string* why) {
     const int ngroups = (r.nchains + kM - 1) / kM, words = pi->R * 8, sms = sm_count();
-    const Config* pc = planes_config(pi->R, pi->W, ngroups, sms);
+    const Config* pc = launch_config(pi->R, pi->W, ngroups, sms, r.variant);
     if (!pc) {
         if (why) *why = "the planes kernel cannot be co-resident on this device";
         return -2;
@@ -822,6 +874,7 @@ int planes_run(PlanesInstance* pi, const TensorRun& r, cudaStream_t st, std::str
     P.out_trace = r.out_trace;
     P.out_h = r.out_h;
     P.err = reinterpret_cast<int*>(base);
+    P.prof = r.prof;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
@@ -838,6 +891,7 @@ int planes_run(PlanesInstance* pi, const TensorRun& r, cudaStream_t st, std::str
         return -2;
     }
     pi->last_err = P.err;
+    pi->last_ctas = nsl * slots;
     return 0;
 }
 

@@ -539,7 +539,6 @@ int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm,
         return -2;
     }
     ti->last_err = err;
-    ti->last_kind = TENSOR_KIND_INT8;
     ti->last_ctas = kSSlices;
     ti->last_cluster = 1;
     return 0;

@@ -142,7 +142,8 @@ ANC_API int anc_sparse_tuning(const anc_instance* inst, int* variant, double* pr
  * The run-time tuner of the dense kernels' compiled variants:
  *   ANC_KERNEL_PLAIN (dense instances): rows of bit planes a thread counts per batch -- K = 1: 0 = 8 rows with the
  *     next 8 fetched ahead, 1 = 8 rows, 2 = 16 rows; K = 2: 0 = 8 rows, 1 = 16 rows; K = 4 and NP > 8192: one variant;
- *   ANC_KERNEL_TENSOR_FP4: the depth of the shared-memory ring of dS tiles -- 0 = 4 stages, 1 = 6, 2 = 5, 3 = 3.
+ *   ANC_KERNEL_TENSOR_FP4: RNG lanes per decision thread -- 0 = by the number of replica groups (the fewest waves, then the
+ *     fewest lanes), 1 = 8 (16 CTAs per replica group), 2 = 4 (32 CTAs), 3 = 2 (64 CTAs).
  * The first synchronous run (anc_run / anc_run_fields) that uses one of these kernels for a (device, kernel, NP, K,
  * replica groups) key not yet tuned runs each variant on the first min(S, 256) steps of that run's anneals (one wave
  * of the plain engine, every replica group of the fp4 kernel) into the handle's own workspaces -- three times, the
