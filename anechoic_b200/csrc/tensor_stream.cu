@@ -358,50 +358,54 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 }
             }
         } else if (warp == kSMmaWarp) {
-            // ---------------- MMA thread ----------------
-            if (lane == 0) {
-                if (!err_set(err)) mbar_wait(bar_init, uint32_t(pr) & 1u, err, kErrInit);
-                tc_fence_after();
-                for (int m = -1; m < S; ++m) {
-                    const long long t0 = prof ? clock64() : 0;
-                    if (m >= 0) {
-                        if (!err_set(err)) mbar_wait(bar_rd, rph & 1u, err, kErrRead);
-                        ++rph;
-                        tc_fence_after();
-                    }
-                    for (int c = 0; c < kSChunks; ++c, ++q) {
-                        const int s = int(q % kSStages);
-                        const uint32_t u = q / kSStages;
-                        const long long w0 = prof ? clock64() : 0;
-                        const bool ok = !err_set(err) && mbar_wait(bar_full + 8 * s, u & 1u, err, kErrFull);
-                        if (prof) pa += clock64() - w0;
-                        tc_fence_after();
-                        if (ok) {
-                            const uint32_t b0 = smem_u32(stages + size_t(s) * kSStage);
-                            if (c < kSSlices) {
+            // ---------------- MMA warp: converged, one elected lane issues (as a loop run by one lane, an MMA takes about
+            // 80 cycles to issue: its operands move to uniform registers one by one) ----------------
+            const bool iok = !err_set(err) && mbar_wait(bar_init, uint32_t(pr) & 1u, err, kErrInit);
+            (void)__all_sync(0xffffffffu, iok);
+            tc_fence_after();
+            const uint32_t utmem = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint64_t st0 = sw128_desc(smem_u32(stages)), bo = sw128_desc(smem_u32(ones));
+            const bool lead = elect_one();
+#pragma unroll 1
+            for (int m = -1; m < S; ++m) {
+                const long long t0 = prof ? clock64() : 0;
+                bool ok = __all_sync(0xffffffffu, !err_set(err));
+                if (m >= 0) {
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait(bar_rd, rph & 1u, err, kErrRead));
+                    ++rph;
+                    tc_fence_after();
+                }
+#pragma unroll 1
+                for (int c = 0; c < kSChunks; ++c, ++q) {
+                    const uint32_t s = q % kSStages;
+                    const long long w0 = prof ? clock64() : 0;
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, (q / kSStages) & 1u, err, kErrFull));
+                    if (prof) pa += clock64() - w0;
+                    tc_fence_after();
+                    if (lead) {
+                        const uint64_t b0 = st0 + uint64_t(s * (kSStage >> 4));
+                        if (ok && c < kSSlices) {
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk) {
-                                    const uint64_t bj = sw128_desc(b0 + 32 * kk);
-                                    mma_i8(tmem, sw128_desc(b0 + kSTile + 32 * kk), bj, IDESC_H, 1u);
-                                    mma_i8(tmem + 128u, sw128_desc(b0 + 2 * kSTile + 32 * kk), bj, IDESC_H, 1u);
-                                }
-                            } else {
-                                const uint32_t o = smem_u32(ones);
+                            for (int kk = 0; kk < 4; ++kk) {
+                                const uint64_t bj = b0 + uint64_t(2 * kk);
+                                mma_i8(utmem, bj + uint64_t(kSTile >> 4), bj, IDESC_H, 1u);
+                                mma_i8(utmem + 128u, bj + uint64_t(2 * (kSTile >> 4)), bj, IDESC_H, 1u);
+                            }
+                        } else if (ok) {
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk) {
-                                    const uint64_t bo = sw128_desc(o + 32 * kk);
-                                    mma_i8(tmem + 256u, sw128_desc(b0 + kSTile + 32 * kk), bo, IDESC_NL, 1u);
-                                    mma_i8(tmem + 272u, sw128_desc(b0 + 2 * kSTile + 32 * kk), bo, IDESC_NL, 1u);
-                                }
+                            for (int kk = 0; kk < 4; ++kk) {
+                                const uint64_t bj = b0 + uint64_t(2 * kk);
+                                mma_i8(utmem + 256u, bj + uint64_t(kSTile >> 4), bo + uint64_t(2 * kk), IDESC_NL, 1u);
+                                mma_i8(utmem + 272u, bj + uint64_t(2 * (kSTile >> 4)), bo + uint64_t(2 * kk), IDESC_NL, 1u);
                             }
                         }
                         mma_commit(bar_empty + 8 * s);
                     }
-                    mma_commit(bar_h);
-                    if (prof) pb += clock64() - t0;
+                    __syncwarp();
                 }
-            } else {
-                q += uint32_t(S + 1) * kSChunks;
+                if (lead) mma_commit(bar_h);
+                __syncwarp();
+                if (prof) pb += clock64() - t0;
             }
             __syncwarp();
         }
