@@ -480,9 +480,10 @@ double flip_fraction(const anc_instance* I, const anc_tables* tb, const anc_run_
 // Engine of a launch. planes is set when the tensor engine is picked with the planes kernel: by AUTO, unless the caller
 // asked for an operand format, a compiled variant or a profile of the other kernels, or by tensor_kind.
 int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts* o, double* us = nullptr,
-                double* phi_used = nullptr, bool* planes = nullptr) {
+                double* phi_used = nullptr, bool* planes = nullptr, bool* stream = nullptr) {
     const int e = o ? o->engine : ANC_ENGINE_AUTO;
     if (planes) *planes = e == ANC_ENGINE_TENSOR && o->tensor_kind == ANC_TENSOR_PLANES;
+    if (stream) *stream = false;
     if (e == ANC_ENGINE_PLAIN || e == ANC_ENGINE_TENSOR || e == ANC_ENGINE_CLUSTER) return e;
     const double phi = flip_fraction(I, tb, o);
     double est[4];
@@ -501,16 +502,27 @@ int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts
             }
         }
     }
+    // sizes no other tensor kernel takes: the streaming kernel, which ANC_ENGINE_TENSOR runs above NP = 8192 only
+    if (free_choice && est[ANC_ENGINE_TENSOR] < 0 && !I->dense.empty() && anc::stream_runs(I->n)) {
+        const double t = tb->S * anc::stream_step_us(I->n, nchains);
+        est[ANC_ENGINE_TENSOR] = t;
+        if (est[best] < 0 || t < est[best]) {
+            best = ANC_ENGINE_TENSOR;
+            if (stream) *stream = true;
+        }
+    }
     if (us) std::copy(est, est + 4, us);
     if (phi_used) *phi_used = phi;
     return best;
 }
 
-int ensure_tensor(anc_instance* I) {
+int ensure_tensor(anc_instance* I, cudaStream_t st) {
     if (I->tensor_ready) return ANC_OK;
     if (I->dense.empty()) return fail(ANC_EINVAL, "the tensor engine needs dense couplings");
     std::string why;
-    const int rc = anc::tensor_build_instance(I->dense.data(), I->n, &I->tensor, &why);
+    const int rc = !anc::tensor_supported(I->n, I->K, 1) || anc::stream_supported(I->n)
+                       ? anc::stream_build(I->planes.p, I->K, I->nwj, I->n, &I->tensor, st, &why)
+                       : anc::tensor_build_instance(I->dense.data(), I->n, &I->tensor, &why);
     if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "tensor engine setup: %s", why.c_str());
     I->tensor_ready = true;
     return ANC_OK;
@@ -536,17 +548,17 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
     int32_t hclamp = 0;
     int rc = resolve_clamp(I, tb, o, &hclamp);
     if (rc) return rc;
-    bool planes = false;
-    const int engine = pick_engine(I, tb, nchains, o, nullptr, nullptr, &planes);
+    bool planes = false, streamed = false;
+    const int engine = pick_engine(I, tb, nchains, o, nullptr, nullptr, &planes, &streamed);
     if (engine == ANC_ENGINE_TENSOR) {
-        if (planes ? !planes_candidate(I) : !anc::tensor_supported(I->n, I->K, nchains))
+        if (planes ? !planes_candidate(I) : !streamed && !anc::tensor_supported(I->n, I->K, nchains))
             return fail(ANC_EINVAL, "tensor engine does not support n=%d K=%d", I->n, I->K);
         const int kind = o ? o->tensor_kind : ANC_TENSOR_AUTO;
         if (kind == ANC_TENSOR_FP4 && !fp4_candidate(I))
             return fail(ANC_EINVAL, "tensor engine: the fp4 kernel needs NP = 2048, |J| <= 1 and max|b| + max_y sum_x "
                                     "|J_xy| < 16384");
         const bool fp4 = !planes && fp4_candidate(I) && kind != ANC_TENSOR_INT8;
-        rc = planes || fp4 ? ensure_planes(I, st) : ensure_tensor(I);
+        rc = planes || fp4 ? ensure_planes(I, st) : ensure_tensor(I, st);
         if (rc) return rc;
         const int forced = o ? o->kernel_variant : 0;
         if (forced > (planes ? 0 : anc::kF4Variants))
@@ -689,7 +701,7 @@ int tune_kernel(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
     if (o && o->kernel_variant > 0) return ANC_OK;
     bool planes = false;
     const int engine = pick_engine(I, tb, nchains, o, nullptr, nullptr, &planes);
-    if (planes) return ANC_OK;     // one compiled variant per geometry
+    if (planes) return ANC_OK;     // its geometry follows from the launch
     int kernel = 0, nv = 1, nprobe = nchains;
     if (engine == ANC_ENGINE_PLAIN && I->K != 0) {
         size_t smem = 0;

@@ -10,7 +10,7 @@ namespace anc {
 
 struct TensorInstance {
     int n = 0, np = 0;
-    int npp = 0;                 // permuted width of J_perm (np, or 16384 for the streaming kernel)
+    int npp = 0;                 // permuted width of J_perm (np, or 256 x the padded rounds for the streaming kernel)
     bool stream = false;         // 32 < NP/256 <= 64: J streamed from HBM (tensor_stream.cu)
     std::vector<int> perm;       // slot i -> permuted index (CTA-contiguous slot slices)
     int8_t* d_J = nullptr;       // J_perm [np][np] int8 (row = y, contiguous x)
@@ -59,10 +59,13 @@ bool tensor_supported(int n, int K, int nchains);
 int tensor_wave_chains(int n, int* out);
 int tensor_build_instance(const int8_t* J, int n, TensorInstance* out, std::string* why);
 int tensor_run(TensorInstance* ti, const TensorRun& r, cudaStream_t st, std::string* why);
-// Streaming kernel for NP in (8192, 16384] (tensor_stream.cu): support test, slot permutation, permuted width, launch.
+// Streaming kernel for NP in (8192, 16384] (tensor_stream.cu): support test, build from the plain engine's bit planes, launch.
 bool stream_supported(int n);
-void stream_permutation(int np, std::vector<int>* p);
-int stream_width();
+// Whether the kernel can run n at all: NP in (4096, 16384] (AUTO uses it below 8193 where no other tensor kernel runs), and the
+// measured device time of one step of nchains anneals, in microseconds.
+bool stream_runs(int n);
+double stream_step_us(int n, int nchains);
+int stream_build(const uint32_t* bits, int K, int nwj, int n, TensorInstance* out, cudaStream_t st, std::string* why);
 int stream_wave_chains();
 int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm, cudaStream_t st, std::string* why);
 // Planes kernel (tensor_planes.cu): J on chip as one (|J| <= 4) or two e2m1 planes, NP = 2048 .. 6144 (one plane) or

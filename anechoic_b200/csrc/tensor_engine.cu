@@ -935,21 +935,16 @@ bool tensor_supported(int n, int K, int nchains) {
 int tensor_build_instance(const int8_t* J, int n, TensorInstance* out, std::string* why) {
     const int np = std::max(2048, ((n + 255) / 256) * 256);
     const int R = np / 256, nc = 16 * R;
-    if (!(R == 8 || R == 12 || R == 16 || stream_supported(n))) {
+    if (!(R == 8 || R == 12 || R == 16)) {
         if (why) *why = "tensor engine supports NP in {2048, 3072, 4096} and (8192, 16384]";
         return -1;
     }
-    const bool big = stream_supported(n);
     std::vector<int> p(np);
-    if (big) {
-        stream_permutation(np, &p);
-    } else {
-        for (int i = 0; i < np; ++i) {
-            const int l = i % 256, k = i / 256, cc = l / 16, jl = l % 16;
-            p[i] = cc * nc + jl * R + k;
-        }
+    for (int i = 0; i < np; ++i) {
+        const int l = i % 256, k = i / 256, cc = l / 16, jl = l % 16;
+        p[i] = cc * nc + jl * R + k;
     }
-    const int npp = big ? stream_width() : np;
+    const int npp = np;
     std::vector<int8_t> Jp(size_t(npp) * npp, 0);
     for (int x = 0; x < n; ++x) {
         for (int y = 0; y < n; ++y) {
@@ -960,7 +955,6 @@ int tensor_build_instance(const int8_t* J, int n, TensorInstance* out, std::stri
     out->n = n;
     out->np = np;
     out->npp = npp;
-    out->stream = big;
     out->perm.assign(p.begin(), p.end());
     cudaError_t e = cudaMalloc(&out->d_J, Jp.size());
     if (e == cudaSuccess) e = cudaMemcpy(out->d_J, Jp.data(), Jp.size(), cudaMemcpyHostToDevice);

@@ -1,17 +1,17 @@
-// Batched engine for large dense instances (NP in (8192, 16384], up to 64 rounds): J is too large to keep resident
-// (16384^2 int8 = 256 MB), so every step streams it from HBM once and applies it to two replica groups at a time.
+// Batched engine for large dense instances (NP in (4096, 16384], 17 to 64 rounds): J is too large to keep on chip (16384^2
+// int8 = 256 MB), so every step streams it from HBM or L2 once and applies it to two replica groups at a time.
 //
-// Layout. 128 CTAs, one per y-slice of 128 permuted columns. Slice cs owns RNG lanes 2cs and 2cs + 1, all rounds:
-// slot i = k*256 + l sits at permuted column p(i) = (l / 2) * 128 + (l % 2) * 64 + k (k < R <= 64; columns with
-// k >= R are padding, never decided, with zero couplings). J_perm[p(y)][p(x)] = J[x][y] (int8).
+// Layout. 128 CTAs, one per y-slice of 2 RP permuted columns, RP = the rounds R padded to 48 or 64. Slice cs owns RNG lanes
+// 2cs and 2cs + 1, all rounds: slot i = k*256 + l sits at permuted column p(i) = l*RP + k (columns with k >= R are padding,
+// never decided, with zero couplings). J_perm[p(y)][p(x)] = J[x][y] (int8).
 // Per step (the golden model's step, sca_ref_bias.hpp:44-68; decision as in anc_common.cuh):
 //   16 decision warps: warp w decides group w / 8, replica (w % 4) * 32 + lane (its TMEM lane), RNG lane
-//     2cs + (w / 4) % 2, the lane's R rounds in order (fields from TMEM, int32). It writes the replica's 64 update
+//     2cs + (w / 4) % 2, the lane's R rounds in order (fields from TMEM, int32). It writes the replica's RP update
 //     bytes dS in {0, +-1, +-2} of its lane and its n_lin partial byte; the CTA then publishes flag[cs] = m + 2.
-//   3 producer warps: chunk c of a step = J_perm rows [128 cs, +128) x columns [128 c, +128) (HBM, no dependency;
-//     issued first) plus the two groups' dS tiles of slice c (L2; after slice c's flag). Two more chunks carry the
+//   3 producer warps: chunk c of a step = J_perm rows [2 RP cs, +2 RP) x columns [128 c, +128) (HBM, no dependency;
+//     issued first) plus the two groups' dS tiles of these columns (L2; after the flags of the slices they hold). Two more chunks carry the
 //     n_lin partials (256 bytes per replica: 2 per slice).
-//   1 MMA thread: per dS chunk, 4 x 2 tcgen05.mma kind::i8 (M 128 replicas, N 128 columns, K 32) into each group's
+//   1 MMA warp: per dS chunk, 4 x 2 tcgen05.mma kind::i8 (M 128 replicas, N 2 RP columns, K 32) into each group's
 //     int32 field accumulator; per n_lin chunk 4 x 2 i8 MMAs against a ones row into the n_lin accumulators.
 // Every wait is bounded (2 s); on expiry the kernel records an error code and skips the remaining work.
 #include <cuda.h>
@@ -30,15 +30,23 @@ using namespace ptx;
 
 constexpr int kSM = 128;                   // replicas per group (MMA M, TMEM lanes)
 constexpr int kSSlices = 128;              // y-slices (CTAs)
-constexpr int kSCols = 128;                // permuted columns per slice (MMA N)
-constexpr int kSNPP = kSSlices * kSCols;   // permuted width 16384
 constexpr int kSDW = 16, kSPW = 3;
 constexpr int kSMmaWarp = kSDW + kSPW;
 constexpr int kSThreads = (kSDW + kSPW + 1) * 32;
 constexpr int kSStages = 4;
-constexpr uint32_t kSTile = 128 * 128;     // 16 KB
-constexpr uint32_t kSStage = 3 * kSTile;   // J tile + two dS tiles
-constexpr int kSChunks = kSSlices + 2;     // dS chunks + 2 n_lin chunks per step
+constexpr uint32_t kSTile = 128 * 128;     // dS tile, 16 KB
+
+// Geometry for RP columns per RNG lane (the rounds padded to a multiple of 16): a slice of two lanes has 2 RP columns.
+template <int RP_>
+struct SGeo {
+    static constexpr int RP = RP_;
+    static constexpr int COLS = 2 * RP;                        // columns per slice (MMA N)
+    static constexpr int NPP = kSSlices * COLS;                // permuted width
+    static constexpr int TILES = NPP / 128;                    // dS chunks of 128 columns per step
+    static constexpr int CHUNKS = TILES + 2;                   // and two n_lin chunks
+    static constexpr uint32_t JT = uint32_t(COLS) * 128;       // J tile: COLS rows x 128 bytes
+    static constexpr uint32_t STAGE = JT + 2 * kSTile;
+};
 constexpr int kErrFull = 1, kErrEmpty = 2, kErrHready = 3, kErrFlag = 4, kErrInit = 6, kErrRead = 7;
 
 struct StreamParams {
@@ -66,14 +74,17 @@ struct StreamParams {
     long long* prof;
 };
 
+template <class G>
 __global__ void __launch_bounds__(kSThreads, 1)
     tensor_stream_kernel(const __grid_constant__ CUtensorMap mapJ, const __grid_constant__ CUtensorMap mapD,
                          const __grid_constant__ CUtensorMap mapNL, const __grid_constant__ StreamParams P) {
+    constexpr int kSCols = G::COLS, kSNPP = G::NPP, kSChunks = G::CHUNKS, RP = G::RP;
+    constexpr uint32_t kSStage = G::STAGE;
     constexpr uint32_t IDESC_H = (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(kSCols >> 3) << 17) | (uint32_t(kSM >> 4) << 24);
     constexpr uint32_t IDESC_NL = (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(16 >> 3) << 17) | (uint32_t(kSM >> 4) << 24);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* stages = smem;                                 // kSStages x (J, dS0, dS1)
+    uint8_t* stages = smem;                                 // kSStages x (dS0, dS1, J)
     uint8_t* ones = stages + kSStages * kSStage;            // 2 KB: row 0 = 128 x int8(1)
     uint64_t* bars = reinterpret_cast<uint64_t*>(ones + 2048);   // full[4], empty[4], hready, init, fields read
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSStages + 3);
@@ -111,7 +122,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // TMEM columns: group g fields [128 g, +128), group g n_lin accumulator [256 + 16 g, +16)
+    // TMEM columns: group g fields [128 g, +2 RP), group g n_lin accumulator [256 + 16 g, +16)
 
     const bool prof = P.prof != nullptr;
     long long pa = 0, pb = 0, pc = 0;
@@ -127,7 +138,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
             const int chain = (2 * pr + g) * kSM + r;
             const bool writer = chain < P.nchains;
             const uint32_t tl = uint32_t((warp & 3) * 32) << 16;
-            const uint32_t fcol = uint32_t(128 * g + 64 * jl);   // this thread's 64 field columns
+            const uint32_t fcol = uint32_t(128 * g + RP * jl);   // this thread's RP field columns
             const size_t drow0 = size_t(g * 2) * kSM + r;       // row of parity 0 in the dS buffer
             Xoshiro rng;
             rng_seed(rng, P.seed, P.trial_offset + uint32_t(chain), uint32_t(l));
@@ -136,10 +147,12 @@ __global__ void __launch_bounds__(kSThreads, 1)
             uint32_t nlacc_prev = 0;
             long long flips = 0;
             {
-                uint32_t dwords[16];
+                uint32_t dwords[RP / 4];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) dwords[e] = 0u;
-                for (int k = 0; k < R; ++k) {
+                for (int e = 0; e < RP / 4; ++e) dwords[e] = 0u;
+#pragma unroll
+                for (int k = 0; k < RP; ++k) {
+                    if (k >= R) break;
                     const uint32_t rv = rng_next(rng);
                     const int i = k * 256 + l;
                     const bool valid = i < n;
@@ -150,18 +163,18 @@ __global__ void __launch_bounds__(kSThreads, 1)
                     const uint32_t b = valid ? (up ? 0x01u : 0xFFu) : 0u;
                     dwords[k >> 2] |= b << (8 * (k & 3));
                 }
-                int8_t* dst = P.dbuf + ((drow0 + kSM) * kSNPP) + cs * kSCols + jl * 64;   // parity 1
+                int8_t* dst = P.dbuf + ((drow0 + kSM) * kSNPP) + cs * kSCols + jl * RP;   // parity 1
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
+                for (int e = 0; e < RP / 16; ++e)
                     reinterpret_cast<uint4*>(dst)[e] =
                         make_uint4(dwords[4 * e], dwords[4 * e + 1], dwords[4 * e + 2], dwords[4 * e + 3]);
                 P.nlx[(drow0 + kSM) * 256 + 2 * cs + jl] = 0;
                 uint32_t v[16];
 #pragma unroll
-                for (int h4 = 0; h4 < 4; ++h4) {
+                for (int h4 = 0; h4 < RP / 16; ++h4) {
 #pragma unroll
                     for (int e = 0; e < 16; ++e)
-                        v[e] = P.bias_perm ? uint32_t(P.bias_perm[cs * kSCols + 64 * jl + 16 * h4 + e]) : 0u;
+                        v[e] = P.bias_perm ? uint32_t(P.bias_perm[cs * kSCols + RP * jl + 16 * h4 + e]) : 0u;
                     tmem_st16(tmem + tl + fcol + uint32_t(16 * h4), v);
                 }
                 if (jl == 0) {
@@ -203,19 +216,20 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 nlin_prev = nlin;
                 if (m == S) {
                     long long sh = 0, bs = 0;
-                    for (int half = 0; half < 2; ++half) {
-                        uint32_t hv[32];
-                        tmem_ld32(tmem + tl + fcol + uint32_t(32 * half), hv);
+#pragma unroll 1
+                    for (int c16 = 0; c16 < RP / 16; ++c16) {
+                        uint32_t hv[16];
+                        tmem_ld16(tmem + tl + fcol + uint32_t(16 * c16), hv);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) {
-                            const int k = 32 * half + e, i = k * 256 + l;
+                        for (int e = 0; e < 16; ++e) {
+                            const int k = 16 * c16 + e, i = k * 256 + l;
                             if (k >= R || i >= n) continue;
                             const bool up = (sw >> k) & 1u;
                             const int32_t h = int32_t(hv[e]);
                             sh += up ? h : -h;
                             if (P.bias_perm) {
-                                const int32_t b = P.bias_perm[cs * kSCols + 64 * jl + k];
+                                const int32_t b = P.bias_perm[cs * kSCols + RP * jl + k];
                                 bs += up ? b : -b;
                             }
                             if (writer) {
@@ -237,15 +251,16 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 const int32_t xs = qv - corr, twocorr = 2 * corr, c1 = twoT - 1;
                 uint64_t fm = 0, lm = 0;
                 const int par = m & 1;
-                int8_t* dst = P.dbuf + ((drow0 + size_t(par) * kSM) * kSNPP) + cs * kSCols + jl * 64;
-                for (int half = 0; half < 2; ++half) {
-                    uint32_t hv[32];
-                    tmem_ld32(tmem + tl + fcol + uint32_t(32 * half), hv);
+                int8_t* dst = P.dbuf + ((drow0 + size_t(par) * kSM) * kSNPP) + cs * kSCols + jl * RP;
+#pragma unroll
+                for (int c16 = 0; c16 < RP / 16; ++c16) {
+                    uint32_t hv[16];
+                    tmem_ld16(tmem + tl + fcol + uint32_t(16 * c16), hv);
                     tmem_wait_ld();
                     uint32_t fmh = 0, lmh = 0;
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) {
-                        const int k = 32 * half + e;
+                    for (int e = 0; e < 16; ++e) {
+                        const int k = 16 * c16 + e;
                         if (k >= R) break;
                         const uint32_t u = rng_next(rng);
                         const bool up = (sw >> k) & 1u;
@@ -257,16 +272,16 @@ __global__ void __launch_bounds__(kSThreads, 1)
                         if (zt < thr) fmh |= 1u << e;
                         if (uint32_t(zt + c1) < lw) lmh |= 1u << e;
                     }
-                    fm |= uint64_t(fmh) << (32 * half);
-                    lm |= uint64_t(lmh) << (32 * half);
+                    fm |= uint64_t(fmh) << (16 * c16);
+                    lm |= uint64_t(lmh) << (16 * c16);
                 }
                 fm &= vmask;
                 lm &= vmask;
                 flips += __popcll(fm);
                 // dS bytes: flipped up -> down = -2 (0xFE), down -> up = +2 (0x02)
-                uint32_t dwords[16];
+                uint32_t dwords[RP / 4];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
+                for (int e = 0; e < RP / 4; ++e) {
                     uint32_t wv = 0u;
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
@@ -276,7 +291,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                     dwords[e] = wv;
                 }
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
+                for (int e = 0; e < RP / 16; ++e)
                     reinterpret_cast<uint4*>(dst)[e] =
                         make_uint4(dwords[4 * e], dwords[4 * e + 1], dwords[4 * e + 2], dwords[4 * e + 3]);
                 P.nlx[(drow0 + size_t(par) * kSM) * 256 + 2 * cs + jl] = int8_t(__popcll(lm));
@@ -314,16 +329,18 @@ __global__ void __launch_bounds__(kSThreads, 1)
                         if (!__shfl_sync(0xffffffffu, w, 0)) continue;
                     }
                     uint8_t* st_base = stages + size_t(s) * kSStage;
-                    const bool dchunk = c < kSSlices;
+                    const bool dchunk = c < G::TILES;
                     if (lane == 0) {
                         mbar_arrive_expect_tx(bar_full + 8 * s, dchunk ? kSStage : 2 * kSTile);
-                        if (dchunk) tma_load_2d(smem_u32(st_base), &mapJ, c * 128, cs * kSCols, bar_full + 8 * s);
+                        if (dchunk) tma_load_2d(smem_u32(st_base + 2 * kSTile), &mapJ, c * 128, cs * kSCols, bar_full + 8 * s);
                     }
-                    // slices that must have published: c (dS chunk) or all (n_lin chunks)
+                    // slices that must have published: those with columns of the chunk (dS) or all (n_lin)
+                    const int lo = dchunk ? c * 128 / kSCols : 0, hi = dchunk ? (c * 128 + 127) / kSCols : kSSlices - 1;
                     bool ok = true;
-                    for (int wdw = 0; wdw < 4 && ok; ++wdw) {
-                        const uint32_t need = dchunk ? ((c >> 5) == wdw ? (1u << (c & 31)) : 0u) : 0xffffffffu;
-                        if (!need || (ready[wdw] & need) == need) continue;
+                    for (int wdw = lo >> 5; wdw <= hi >> 5 && ok; ++wdw) {
+                        const int a = max(lo - 32 * wdw, 0), b = min(hi - 32 * wdw, 31);      // window bits a .. b
+                        const uint32_t need = (0xffffffffu >> (31 - (b - a))) << a;
+                        if ((ready[wdw] & need) == need) continue;
                         ok = false;
                         const uint64_t t0 = globaltimer();
                         for (uint32_t k = 1;; ++k) {
@@ -346,12 +363,12 @@ __global__ void __launch_bounds__(kSThreads, 1)
                         asm volatile("fence.proxy.async.global;" ::: "memory");
                         const int ay0 = (0 * 2 + par) * kSM, ay1 = (1 * 2 + par) * kSM;
                         if (dchunk) {
-                            tma_load_2d(smem_u32(st_base + kSTile), &mapD, c * 128, ay0, bar_full + 8 * s);
-                            tma_load_2d(smem_u32(st_base + 2 * kSTile), &mapD, c * 128, ay1, bar_full + 8 * s);
+                            tma_load_2d(smem_u32(st_base), &mapD, c * 128, ay0, bar_full + 8 * s);
+                            tma_load_2d(smem_u32(st_base + kSTile), &mapD, c * 128, ay1, bar_full + 8 * s);
                         } else {
-                            const int x = (c - kSSlices) * 128;
-                            tma_load_2d(smem_u32(st_base + kSTile), &mapNL, x, ay0, bar_full + 8 * s);
-                            tma_load_2d(smem_u32(st_base + 2 * kSTile), &mapNL, x, ay1, bar_full + 8 * s);
+                            const int x = (c - G::TILES) * 128;
+                            tma_load_2d(smem_u32(st_base), &mapNL, x, ay0, bar_full + 8 * s);
+                            tma_load_2d(smem_u32(st_base + kSTile), &mapNL, x, ay1, bar_full + 8 * s);
                         }
                     }
                     __syncwarp();
@@ -384,19 +401,19 @@ __global__ void __launch_bounds__(kSThreads, 1)
                     tc_fence_after();
                     if (lead) {
                         const uint64_t b0 = st0 + uint64_t(s * (kSStage >> 4));
-                        if (ok && c < kSSlices) {
+                        if (ok && c < G::TILES) {
 #pragma unroll
                             for (int kk = 0; kk < 4; ++kk) {
-                                const uint64_t bj = b0 + uint64_t(2 * kk);
-                                mma_i8(utmem, bj + uint64_t(kSTile >> 4), bj, IDESC_H, 1u);
-                                mma_i8(utmem + 128u, bj + uint64_t(2 * (kSTile >> 4)), bj, IDESC_H, 1u);
+                                const uint64_t d0 = b0 + uint64_t(2 * kk), bj = d0 + uint64_t(2 * (kSTile >> 4));
+                                mma_i8(utmem, d0, bj, IDESC_H, 1u);
+                                mma_i8(utmem + 128u, d0 + uint64_t(kSTile >> 4), bj, IDESC_H, 1u);
                             }
                         } else if (ok) {
 #pragma unroll
                             for (int kk = 0; kk < 4; ++kk) {
-                                const uint64_t bj = b0 + uint64_t(2 * kk);
-                                mma_i8(utmem + 256u, bj + uint64_t(kSTile >> 4), bo + uint64_t(2 * kk), IDESC_NL, 1u);
-                                mma_i8(utmem + 272u, bj + uint64_t(2 * (kSTile >> 4)), bo + uint64_t(2 * kk), IDESC_NL, 1u);
+                                const uint64_t d0 = b0 + uint64_t(2 * kk);
+                                mma_i8(utmem + 256u, d0, bo + uint64_t(2 * kk), IDESC_NL, 1u);
+                                mma_i8(utmem + 272u, d0 + uint64_t(kSTile >> 4), bo + uint64_t(2 * kk), IDESC_NL, 1u);
                             }
                         }
                         mma_commit(bar_empty + 8 * s);
@@ -425,7 +442,46 @@ __global__ void __launch_bounds__(kSThreads, 1)
     }
 }
 
-size_t stream_smem_bytes() { return 1024 + size_t(kSStages) * kSStage + 2048 + (2 * kSStages + 3) * 8 + 16; }
+size_t stream_smem_bytes(uint32_t stage) { return 1024 + size_t(kSStages) * stage + 2048 + (2 * kSStages + 3) * 8 + 16; }
+
+using StreamKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const StreamParams);
+struct StreamConfig {
+    int rp, cols, npp;
+    uint32_t stage;
+    StreamKernel fn;
+};
+template <int RP>
+StreamConfig stream_config_t() {
+    using G = SGeo<RP>;
+    return {RP, G::COLS, G::NPP, G::STAGE, tensor_stream_kernel<G>};
+}
+// The columns a lane's R rounds are padded to: 32, 48 or 64. The kernel is bound by shared-memory bandwidth (an MMA reads 128
+// rows of dS and 2 RP of J, 32 bytes each; TMA writes both), so padding costs in full: n = 10000 (R = 40), 256 anneals: 59.4 us
+// a step with 48 columns, 81.9 with 64.
+StreamConfig stream_config(int R) {
+    return R <= 32 ? stream_config_t<32>() : R <= 48 ? stream_config_t<48>() : stream_config_t<64>();
+}
+
+// The plain engine's bit planes -> J_perm (int8, permuted rows and columns; padding zero). One block per permuted row y.
+__global__ void stream_pack_kernel(const uint32_t* __restrict__ bits, int K, int np, int nwj, int n, int RP, int8_t* __restrict__ out) {
+    const int py = blockIdx.x, ky = py % RP, y = ky * 256 + py / RP, npp = 256 * RP, R = np / 256;
+    const size_t bplane = size_t(np) * nwj;
+    const uint32_t* row = bits + size_t(y) * nwj;
+    for (int px = threadIdx.x; px < npp; px += blockDim.x) {
+        const int kx = px % RP, x = kx * 256 + px / RP;
+        int v = 0;
+        if (ky < R && kx < R && y < n && x < n && x != y) {
+            const uint32_t b0 = (row[x >> 5] >> (x & 31)) & 1u;
+            if (K == 1) {
+                v = b0 ? 1 : -1;
+            } else {
+                for (int p = 1; p < K; ++p) v |= int((row[bplane * p + (x >> 5)] >> (x & 31)) & 1u) << (p - 1);
+                if (b0) v = -v;
+            }
+        }
+        out[size_t(py) * npp + px] = int8_t(v);
+    }
+}
 
 }  // namespace
 
@@ -435,15 +491,41 @@ bool stream_supported(int n) {
     return R > 32 && R <= 64;
 }
 
-void stream_permutation(int np, std::vector<int>* p) {
-    p->resize(np);
-    for (int i = 0; i < np; ++i) {
-        const int l = i % 256, k = i / 256;
-        (*p)[i] = (l / 2) * kSCols + (l % 2) * 64 + k;
-    }
+bool stream_runs(int n) {
+    const int R = ((n + 255) / 256);
+    return R > 16 && R <= 64;
 }
 
-int stream_width() { return kSNPP; }
+double stream_step_us(int n, int nchains) {
+    const int R = (n + 255) / 256;
+    const double us = R <= 32 ? 40.0 : R <= 48 ? 59.4 : 80.0;
+    return us * ((nchains + 2 * kSM - 1) / (2 * kSM));
+}
+
+// J_perm from the plain engine's bit planes on the device (slot k*256 + l at permuted column l*RP + k).
+int stream_build(const uint32_t* bits, int K, int nwj, int n, TensorInstance* out, cudaStream_t st, std::string* why) {
+    const int np = std::max(2048, ((n + 255) / 256) * 256), R = np / 256;
+    const StreamConfig c = stream_config(R);
+    out->n = n;
+    out->np = np;
+    out->npp = c.npp;
+    out->stream = true;
+    out->perm.resize(np);
+    for (int i = 0; i < np; ++i) out->perm[i] = (i % 256) * c.rp + i / 256;
+    out->bytes = size_t(c.npp) * c.npp;
+    cudaError_t e = cudaMalloc(&out->d_J, out->bytes);
+    if (e == cudaSuccess) {
+        stream_pack_kernel<<<c.npp, 256, 0, st>>>(bits, K, np, nwj, n, c.rp, out->d_J);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);      // other streams may run this instance next
+    if (e != cudaSuccess) {
+        if (why) *why = std::string("J: ") + cudaGetErrorString(e);
+        tensor_free_instance(out);
+        return -2;
+    }
+    return 0;
+}
 
 // The kernel advances one pair of replica groups at a time across all its CTAs.
 int stream_wave_chains() { return 2 * kSM; }
@@ -453,9 +535,11 @@ int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm,
     const int ngroups = (r.nchains + kSM - 1) / kSM;
     const int npairs = (ngroups + 1) / 2;
     int per_sm = 0, dev = 0, sms = 0;
-    const size_t smem = stream_smem_bytes();
-    cudaError_t e = cudaFuncSetAttribute(tensor_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tensor_stream_kernel, kSThreads, smem);
+    const StreamConfig c = stream_config(R);
+    const int kSNPP = c.npp;
+    const size_t smem = stream_smem_bytes(c.stage);
+    cudaError_t e = cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, c.fn, kSThreads, smem);
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess || per_sm * sms < kSSlices) {
@@ -483,7 +567,7 @@ int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm,
     int8_t* dbuf = reinterpret_cast<int8_t*>(base + 256 + fbytes);
     int8_t* nlx = dbuf + dbytes;
     CUtensorMap mapJ, mapD, mapNL;
-    if (!make_map_2d(&mapJ, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, ti->d_J, kSNPP, kSNPP, 128, 128) ||
+    if (!make_map_2d(&mapJ, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, ti->d_J, kSNPP, kSNPP, 128, uint32_t(c.cols)) ||
         !make_map_2d(&mapD, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dbuf, kSNPP, 4 * kSM, 128, 128) ||
         !make_map_2d(&mapNL, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, nlx, 256, 4 * kSM, 128, 128)) {
         if (why) *why = "cuTensorMapEncodeTiled failed";
@@ -537,7 +621,7 @@ int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm,
     cfg.blockDim = dim3(kSThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    e = cudaLaunchKernelEx(&cfg, tensor_stream_kernel, mapJ, mapD, mapNL, P);
+    e = cudaLaunchKernelEx(&cfg, c.fn, mapJ, mapD, mapNL, P);
     if (e != cudaSuccess) {
         if (why) *why = std::string("launch: ") + cudaGetErrorString(e);
         return -2;

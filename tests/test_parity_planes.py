@@ -85,3 +85,19 @@ def test_planes_limits_and_expiry(cuda, oracle):
         L.anc_set_wait_ns(old)
     _same(A.run(dev, tb, 3, 0, 130, trace=True, engine="tensor", tensor_kind="planes"),
           oracle.run_batch(2500, oracle.tables(**sc), 3, 0, 130, dense=inst.dense), "after expiry")
+
+
+@pytest.mark.parametrize("n,K,chains", [(4100, 4, 130), (8192, 4, 3), (7000, 1, 300)])
+def test_auto_streams_between_the_other_kernels(cuda, oracle, n, K, chains):
+    """Sizes above the planes kernel's (two planes n > 4096, one plane n > 6144) up to 8192: AUTO runs the streaming kernel
+    (32 columns per lane, 17 to 32 rounds); ANC_ENGINE_TENSOR still refuses them."""
+    inst = _instance(n, K, 5)
+    dev = A.DeviceInstance(inst)
+    sc = dict(S=4, t0=float(1.0 + 0.5 * np.sqrt(n) * (1 << (K - 1))), t1=1.0, q=2.0, lam=0.7, ramp=True)
+    tb = A.Tables.from_schedule(A.Schedule(**sc))
+    r = A.run(dev, tb, 5, 40, chains, trace=True, fields=True, flip_fraction=0.5)
+    assert r.kernel == "tensor-int8"
+    _same(r, oracle.run_batch(n, oracle.tables(**sc), 5, 40, chains, dense=inst.dense, bias=inst.bias), f"n={n} K={K}")
+    assert np.array_equal(r.fields[-1], inst.fields(r.spins[-1]))
+    with pytest.raises(A.AncError):
+        A.run(dev, tb, 5, 40, 2, engine="tensor")
