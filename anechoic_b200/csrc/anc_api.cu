@@ -138,12 +138,16 @@ struct anc_instance {
     anc_instance_info info{};
     std::vector<int32_t> bias;                    // host copy (empty = none)
     DevBuf<uint32_t> planes;
-    DevBuf<int32_t> row_ptr;
-    DevBuf<uint32_t> adj;
-    // the CSR rows with 16-bit edges, two per word (every J_xy = +-1 and n < 32767; else empty): half the fetches
-    DevBuf<int32_t> row_ptr16;
-    DevBuf<uint32_t> adj16;
+    DevBuf<uint32_t> csr;                         // the rows of a sparse instance in all their forms, as one block:
+    const int32_t* row_ptr = nullptr;
+    const uint32_t* adj = nullptr;
+    // with 16-bit edges, two per word (every J_xy = +-1 and np <= kEdgePad; else null): half the fetches
+    const int32_t* row_ptr16 = nullptr;
+    const uint32_t* adj16 = nullptr;
     bool csr16 = false;
+    const uint32_t *slices = nullptr, *row_counts = nullptr;     // for launches in groups (PlainJob::slices), or null
+    const uint2* slice_info = nullptr;
+    DevBuf<int32_t> w_group;                      // fields of the grouped sparse launch (large instances)
     DevBuf<int32_t> d_bias;
     std::vector<int8_t> dense;                    // host copy of dense couplings (tensor engine packs lazily)
     anc::TensorInstance tensor;                   // tensor-engine operands (built on first use)
@@ -314,9 +318,12 @@ anc::PlainJob make_job(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t 
     j.nwj = I->nwj;
     j.K = I->K;
     j.planes = I->planes.p;
-    j.row_ptr = I->csr16 ? I->row_ptr16.p : I->row_ptr.p;
-    j.adj = I->csr16 ? I->adj16.p : I->adj.p;
+    j.row_ptr = I->csr16 ? I->row_ptr16 : I->row_ptr;
+    j.adj = I->csr16 ? I->adj16 : I->adj;
     j.csr16 = I->csr16 ? 1 : 0;
+    j.slices = I->slices;
+    j.slice_info = I->slice_info;
+    j.row_counts = I->row_counts;
     j.bias = I->bias.empty() ? nullptr : I->d_bias.p;
     j.tab = dev_tables(tb);
     j.seed = seed;
@@ -338,7 +345,8 @@ int plain_residency(const anc_instance* I, int P, size_t* smem, bool* stream, in
     *smem = anc::plain_smem_plan(I->np, I->K == 0 ? I->nw : I->nwj, I->K, P, stream);
     if (*smem > 227 * 1024)
         return fail(ANC_EINVAL, "instance too large for the plain engine (%zu B shared memory)", *smem);
-    const int rc = anc::plain_max_blocks_per_sm(I->K, P, *smem, per_sm, *stream);
+    const int rc = I->K == 0 ? anc::sparse_max_blocks_per_sm(I->np, per_sm)
+                             : anc::plain_max_blocks_per_sm(I->K, P, *smem, per_sm, *stream);
     if (rc) return cuda_fail(cudaError_t(rc), "occupancy");
     if (*per_sm < 1) return fail(ANC_EINVAL, "plain engine cannot be resident (smem %zu)", *smem);
     return ANC_OK;
@@ -348,7 +356,7 @@ int plain_residency(const anc_instance* I, int P, size_t* smem, bool* stream, in
 constexpr int kKinds[4] = {0, 1, 2, 4};     // CSR, then dense K = 1 / 2 / 4
 int kind_index(int K) { return K == 0 ? 0 : K == 1 ? 1 : K == 2 ? 2 : 3; }
 struct KindPlan {
-    int np_max = 0, nwj_max = 0, P = 0, per_sm = 0;
+    int np_max = 0, np_min = 0, nwj_max = 0, P = 0, per_sm = 0;
     size_t smem = 0;
     bool stream = false;
 };
@@ -362,7 +370,8 @@ int plan_kind(int K, int np_max, int nwj_max, int sms, KindPlan* out) {
     if (p.smem > 227 * 1024)
         return fail(ANC_EINVAL, "batch instance too large for the plain engine (n padded to %d needs %zu B of shared "
                                 "memory)", np_max, p.smem);
-    const int rc = anc::plain_max_blocks_per_sm(K, p.P, p.smem, &p.per_sm, p.stream);
+    const int rc = K == 0 ? anc::sparse_max_blocks_per_sm(np_max, &p.per_sm)
+                          : anc::plain_max_blocks_per_sm(K, p.P, p.smem, &p.per_sm, p.stream);
     if (rc) return cuda_fail(cudaError_t(rc), "occupancy");
     if (p.per_sm < 1) return fail(ANC_EINVAL, "plain engine cannot be resident (%zu B shared memory)", p.smem);
     *out = p;
@@ -370,6 +379,9 @@ int plan_kind(int K, int np_max, int nwj_max, int sms, KindPlan* out) {
 }
 
 int tuned_variant(anc_instance* I, int kernel, int nchains);
+
+// Mean edges per row of a sparse instance.
+double row_degree(const anc_instance* I) { return double(I->info.nnz) / std::max(1, I->n); }
 
 // One launch of the one-CTA plain engine; variant >= 0 forces the CSR pass variant (sparse instances) or the dense
 // pass variant (dense instances), else the tuned one.
@@ -390,6 +402,14 @@ int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t 
     if (rc) return rc;
     if (I->K == 0) {
         L.sparse_variant = variant >= 0 ? variant : std::max(0, I->sparse_variant);
+        if (job.slices && anc::sparse_groups(I->np, row_degree(I), job.ntrials, I->sms)) {
+            L.groups = 1;
+            L.clamp = job.hclamp > 0;
+            L.nitems = (job.ntrials + anc::kGroupReplicas - 1) / anc::kGroupReplicas;
+            const size_t words = anc::sparse_group_scratch(I->np, L.nitems, I->sms);
+            CK(I->w_group.ensure(words));
+            L.group_h = I->w_group.p;
+        }
     } else {
         const int nv = anc::dense_variants(I->K, stream);
         if (variant >= nv)
@@ -400,7 +420,7 @@ int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t 
     L.stream = stream ? 1 : 0;
     const int grid = std::max(1, std::min(job.ntrials, per_sm * I->sms));
     CK(cudaMemsetAsync(I->counter.p, 0, sizeof(int), st));
-    rc = anc::plain_launch(L, I->K, P, grid, smem, st);
+    rc = I->K == 0 ? anc::sparse_launch(L, per_sm, I->sms, st) : anc::plain_launch(L, I->K, P, grid, smem, st);
     if (rc) return cuda_fail(cudaError_t(rc), "plain engine launch");
     return ANC_OK;
 }
@@ -627,15 +647,16 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
         return ANC_OK;
     }
     if (I->K == 0 && o && o->kernel_variant > 0) {
-        // CSR edge format: 1 = 32-bit edges, 2 = 16-bit edges (unit weights and n < 32767 only)
+        // CSR edge format: 1 = 32-bit edges, 2 = 16-bit edges (unit weights and np <= kEdgePad only)
         if (o->kernel_variant > 2 || (o->kernel_variant == 2 && !I->csr16))
             return fail(ANC_EINVAL, "kernel_variant %d: CSR instances take 1 (32-bit edges) or, with unit weights "
-                                    "and n < 32767, 2 (16-bit edges)", o->kernel_variant);
+                                    "and n <= 32512, 2 (16-bit edges)", o->kernel_variant);
         if (o->kernel_variant == 1) {
-            job.row_ptr = I->row_ptr.p;
-            job.adj = I->adj.p;
+            job.row_ptr = I->row_ptr;
+            job.adj = I->adj;
             job.csr16 = 0;
         }
+        job.slices = nullptr;      // a forced edge format runs the kernels that take either
     }
     const int forced = o ? (I->K == 0 ? o->sparse_variant : o->kernel_variant) : 0;
     rc = launch_plain_single(I, job, st, forced > 0 ? forced - 1 : -1);
@@ -1079,32 +1100,92 @@ int anc_instance_create_csr(int n, const int32_t* row_ptr, const int32_t* col, c
     compute_info(I.get(), row_ptr, col, val);
     int rc = finish_common(I.get(), bias);
     if (rc) return rc;
-    cudaError_t e = I->row_ptr.ensure(size_t(n) + 1);
-    if (e == cudaSuccess) e = cudaMemcpy(I->row_ptr.p, row_ptr, (size_t(n) + 1) * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = I->adj.ensure(std::max<int64_t>(nnz, 1));
-    if (e == cudaSuccess && nnz) e = cudaMemcpy(I->adj.p, adj.data(), size_t(nnz) * 4, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_fail(e, "upload CSR");
-    // unit weights and n < 32767: the same rows with 16-bit edges y | [J = -1] << 15, two per word, each row padded
-    // to a whole word with the skip edge 0x7fff; the CSR pass then fetches half the words
-    bool unit = n < 0x7fff;
+    // every form of the rows goes to the device as one block of words
+    std::vector<uint32_t> block;
+    auto put = [&](const void* p, size_t words) {
+        const size_t at = block.size();
+        block.resize(at + (std::max<size_t>(words, 1) + 63) / 64 * 64, 0u);
+        if (words) std::memcpy(block.data() + at, p, words * 4);
+        return at;
+    };
+    const size_t rp_at = put(row_ptr, size_t(n) + 1), adj_at = put(adj.data(), size_t(nnz));
+    size_t rp16_at = 0, adj16_at = 0, slices_at = 0, info_at = 0, counts_at = 0;
+    bool sliced = false;
+    // unit weights and np <= kEdgePad: the same rows with 16-bit edges y | [J = -1] << 15, two per word, each row padded to a
+    // whole word with the edge kEdgePad; the CSR pass then fetches half the words
+    bool unit = I->np <= int(anc::kEdgePad);
     for (int64_t k = 0; unit && k < nnz; ++k) unit = val[k] == 1 || val[k] == -1;
     if (unit) {
         std::vector<int32_t> rp16(size_t(n) + 1, 0);
         for (int x = 0; x < n; ++x) rp16[x + 1] = rp16[x] + (row_ptr[x + 1] - row_ptr[x] + 1) / 2;
-        std::vector<uint32_t> a16(std::max<int32_t>(rp16[n], 1), 0x7fff7fffu);
-        for (int x = 0; x < n; ++x)
+        std::vector<uint32_t> a16(std::max<int32_t>(rp16[n], 1), anc::kEdgePad * 0x10001u);
+        std::vector<int32_t> minus(n, 0);
+        int longest = 0;
+        for (int x = 0; x < n; ++x) {
             for (int k = row_ptr[x]; k < row_ptr[x + 1]; ++k) {
                 const int i = k - row_ptr[x];
                 const uint32_t ed = uint32_t(col[k]) | (val[k] < 0 ? 0x8000u : 0u);
                 uint32_t& wd = a16[size_t(rp16[x]) + i / 2];
                 wd = (i & 1) ? ((wd & 0xffffu) | (ed << 16)) : ((wd & 0xffff0000u) | ed);
+                minus[x] += val[k] < 0;
             }
-        e = I->row_ptr16.ensure(size_t(n) + 1);
-        if (e == cudaSuccess) e = cudaMemcpy(I->row_ptr16.p, rp16.data(), (size_t(n) + 1) * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = I->adj16.ensure(a16.size());
-        if (e == cudaSuccess) e = cudaMemcpy(I->adj16.p, a16.data(), a16.size() * 4, cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return cuda_fail(e, "upload 16-bit CSR");
+            longest = std::max(longest, row_ptr[x + 1] - row_ptr[x]);
+        }
+        std::vector<uint32_t> slices, counts;
+        std::vector<uint2> slice_info;
+        if (longest <= anc::kGroupDegree && I->np <= anc::kGroupNp) {
+            counts.resize(n);
+            for (int x0 = 0; x0 < n; x0 += 32) {
+                const int x1 = std::min(n, x0 + 32);
+                int w[2] = {0, 0};                               // words of the longest + and - part
+                for (int x = x0; x < x1; ++x) {
+                    const int deg = row_ptr[x + 1] - row_ptr[x];
+                    counts[x] = uint32_t(deg) | uint32_t(minus[x]) << 8;
+                    w[0] = std::max(w[0], (deg - minus[x] + 1) / 2);
+                    w[1] = std::max(w[1], (minus[x] + 1) / 2);
+                }
+                const size_t base = slices.size();
+                slice_info.push_back(make_uint2(uint32_t(base), uint32_t(w[0]) | uint32_t(w[1]) << 16));
+                slices.resize(base + size_t(32) * (w[0] + w[1]));
+                for (int i = 0; i < 32; ++i) {
+                    const uint32_t pad = 8u * uint32_t(I->np + i);
+                    for (int e = 0; e < w[0] + w[1]; ++e) slices[base + size_t(32) * e + i] = pad * 0x10001u;
+                    if (x0 + i >= x1) continue;
+                    int at[2] = {0, 2 * w[0]};                   // next edge of the + and the - part
+                    for (int k = row_ptr[x0 + i]; k < row_ptr[x0 + i + 1]; ++k) {
+                        const int j = at[val[k] < 0]++;
+                        uint32_t& wd = slices[base + size_t(32) * (j / 2) + i];
+                        const uint32_t off = 8u * uint32_t(col[k]);
+                        wd = (j & 1) ? ((wd & 0xffffu) | off << 16) : ((wd & 0xffff0000u) | off);
+                    }
+                }
+            }
+            // active rounds reach the next multiple of 256 rows: empty slices
+            while (slice_info.size() % 8) slice_info.push_back(make_uint2(0u, 0u));
+        }
+        rp16_at = put(rp16.data(), rp16.size());
+        adj16_at = put(a16.data(), a16.size());
+        if (!slice_info.empty()) {
+            slices_at = put(slices.data(), slices.size());
+            info_at = put(slice_info.data(), 2 * slice_info.size());
+            counts_at = put(counts.data(), counts.size());
+            sliced = true;
+        }
         I->csr16 = true;
+    }
+    cudaError_t e = I->csr.ensure(block.size());
+    if (e == cudaSuccess) e = cudaMemcpy(I->csr.p, block.data(), block.size() * 4, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_fail(e, "upload CSR");
+    I->row_ptr = reinterpret_cast<const int32_t*>(I->csr.p + rp_at);
+    I->adj = I->csr.p + adj_at;
+    if (I->csr16) {
+        I->row_ptr16 = reinterpret_cast<const int32_t*>(I->csr.p + rp16_at);
+        I->adj16 = I->csr.p + adj16_at;
+    }
+    if (sliced) {
+        I->slices = I->csr.p + slices_at;
+        I->slice_info = reinterpret_cast<const uint2*>(I->csr.p + info_at);
+        I->row_counts = I->csr.p + counts_at;
     }
     *out = I.release();
     return ANC_OK;
@@ -1306,6 +1387,33 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
             if (rc) return rc;
         }
     }
+    // Sparse jobs run as concurrent launches by size and form: classes 0 .. 2 (NP up to 2304, 9216 and above) in groups of
+    // four replicas, classes 3 .. 5 anneal by anneal, so that the largest instance's shared memory does not set how many of
+    // the smaller ones share an SM.
+    constexpr int kClasses = 6;
+    int64_t sparse_anneals = 0;
+    for (int k = 0; k < njobs; ++k)
+        if (jobs[k].inst->K == 0) sparse_anneals += jobs[k].nchains;
+    auto sparse_class = [&](const anc_instance* I) {
+        const bool group = I->slices && anc::sparse_groups(I->np, std::max(8.0, row_degree(I)), sparse_anneals, sms);
+        // few anneals: one launch, one anneal per SM
+        if (sparse_anneals <= 2 * sms) return 3;
+        return (group ? 0 : 3) + (I->np <= 2304 ? 0 : I->np <= 9216 ? 1 : 2);
+    };
+    KindPlan sparse_plans[kClasses];
+    for (int k = 0; k < njobs; ++k) {
+        if (jobs[k].inst->K != 0) continue;
+        KindPlan& sp = sparse_plans[sparse_class(jobs[k].inst)];
+        sp.np_max = std::max(sp.np_max, jobs[k].inst->np);
+        sp.np_min = sp.np_min ? std::min(sp.np_min, jobs[k].inst->np) : jobs[k].inst->np;
+    }
+    for (KindPlan& sp : sparse_plans)
+        if (sp.np_max) {
+            const int np_min = sp.np_min;
+            const int rc = plan_kind(0, sp.np_max, sp.np_max / 32, sms, &sp);
+            if (rc) return rc;
+            sp.np_min = np_min;
+        }
     cudaStream_t st = nullptr;
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     std::unique_ptr<CUstream_st, void (*)(cudaStream_t)> st_guard(st, [](cudaStream_t s) { cudaStreamDestroy(s); });
@@ -1314,70 +1422,159 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
     CK(cudaEventCreate(&e1));
     std::unique_ptr<CUevent_st, void (*)(cudaEvent_t)> g0(e0, [](cudaEvent_t e) { cudaEventDestroy(e); });
     std::unique_ptr<CUevent_st, void (*)(cudaEvent_t)> g1(e1, [](cudaEvent_t e) { cudaEventDestroy(e); });
-    // per-job device outputs
-    struct JobBufs {
-        DevBuf<uint32_t> spins;
-        DevBuf<long long> sh, bs, fl;
-        DevBuf<int32_t> trace;
-    };
-    std::vector<std::unique_ptr<JobBufs>> bufs(njobs);
-    std::vector<anc::PlainJob> pj(njobs);
-    for (const Prepared& p : prep) {
-        const anc_job& j = jobs[p.idx];
-        bufs[p.idx].reset(new JobBufs());
-        JobBufs& b = *bufs[p.idx];
-        CK(b.spins.ensure(size_t(j.inst->nw) * j.nchains));
-        CK(b.sh.ensure(j.nchains));
-        CK(b.bs.ensure(j.nchains));
-        CK(b.fl.ensure(j.nchains));
-        if (j.trace) CK(b.trace.ensure(size_t(j.nchains) * j.tb->S));
-        OutPtrs out{b.spins.p, b.sh.p, b.bs.p, b.fl.p, j.trace ? b.trace.p : nullptr, nullptr};
-        pj[p.idx] = make_job(j.inst, j.tb, j.seed, j.trial_offset, j.nchains, p.hclamp, out);
+    // side streams of the sparse classes beyond the first in use, with their fork and join events
+    struct Side {
+        cudaStream_t st = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr;
+        ~Side() {
+            if (fork) cudaEventDestroy(fork);
+            if (join) cudaEventDestroy(join);
+            if (st) cudaStreamDestroy(st);
+        }
+    } side[kClasses];
+    int main_class = -1;
+    for (int ci = 0; ci < kClasses; ++ci) {
+        if (!sparse_plans[ci].np_max) continue;
+        if (main_class < 0) {
+            main_class = ci;          // the smallest class runs on the call's own stream, after the larger ones
+            continue;
+        }
+        CK(cudaStreamCreateWithFlags(&side[ci].st, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&side[ci].fork, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&side[ci].join, cudaEventDisableTiming));
     }
-    DevBuf<anc::PlainJob> d_jobs;
-    CK(d_jobs.ensure(njobs));
-    CK(cudaMemcpy(d_jobs.p, pj.data(), sizeof(anc::PlainJob) * njobs, cudaMemcpyHostToDevice));
-    DevBuf<int> counters;
-    CK(counters.ensure(4));
-    std::vector<DevBuf<int2>> d_items(4);
-    // from here on work is enqueued: a failure waits for the stream before the buffers above are freed
-    auto drain = [&](int rc) {
-        cudaStreamSynchronize(st);
-        return rc;
-    };
     // work items per kind: a longest-processing-time-first queue, cost ~ np * S per anneal (dense np^2 * S)
-    int nitems[4] = {0, 0, 0, 0};
+    int nitems[4] = {0, 0, 0, 0}, first_item[4] = {0, 0, 0, 0}, class_first[kClasses + 1] = {};
+    std::vector<int2> all_items;
     for (int ki = 0; ki < 4; ++ki) {
         const int K = kKinds[ki];
         std::vector<std::pair<double, int2>> items;
         for (int k = 0; k < njobs; ++k) {
             if (jobs[k].inst->K != K) continue;
             const double cost = double(jobs[k].inst->np) * jobs[k].tb->S * (K == 0 ? 1.0 : double(jobs[k].inst->np));
-            for (int c = 0; c < jobs[k].nchains; ++c) items.push_back({cost, make_int2(k, c)});
+            const int per = K == 0 && sparse_class(jobs[k].inst) < 3 ? anc::kGroupReplicas : 1;
+            for (int c = 0; c < jobs[k].nchains; c += per) items.push_back({cost, make_int2(k, c)});
         }
         if (items.empty()) continue;
         std::stable_sort(items.begin(), items.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-        std::vector<int2> it(items.size());
-        for (size_t i = 0; i < items.size(); ++i) it[i] = items[i].second;
-        cudaError_t e = d_items[ki].ensure(it.size());
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_items[ki].p, it.data(), it.size() * sizeof(int2), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return drain(cuda_fail(e, "work items"));
-        nitems[ki] = int(it.size());
+        if (K == 0) {
+            auto cls = [&](const std::pair<double, int2>& x) { return sparse_class(jobs[x.second.x].inst); };
+            std::stable_sort(items.begin(), items.end(), [&](const auto& a, const auto& b) { return cls(a) < cls(b); });
+            for (const auto& x : items) ++class_first[cls(x) + 1];
+            for (int ci = 0; ci < kClasses; ++ci) class_first[ci + 1] += class_first[ci];
+        }
+        first_item[ki] = int(all_items.size());
+        nitems[ki] = int(items.size());
+        for (const auto& x : items) all_items.push_back(x.second);
     }
+    // the call's device memory is one allocation: results (one copy back), traces, job table and items (one copy in), queue
+    // counters, the group launches' fields
+    size_t need = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = need;
+        need += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    struct JobPlace {
+        size_t sh, bs, fl, spins, trace;
+    };
+    std::vector<JobPlace> at(njobs);
+    for (int k = 0; k < njobs; ++k) {
+        const size_t c = size_t(jobs[k].nchains) * 8;
+        at[k].sh = place(c);
+        at[k].bs = place(c);
+        at[k].fl = place(c);
+        at[k].spins = place(size_t(jobs[k].inst->nw) * jobs[k].nchains * 4);
+    }
+    const size_t result_bytes = need;
+    for (int k = 0; k < njobs; ++k) at[k].trace = jobs[k].trace ? place(size_t(jobs[k].nchains) * jobs[k].tb->S * 4) : 0;
+    const size_t jobs_at = place(sizeof(anc::PlainJob) * njobs), items_at = place(sizeof(int2) * all_items.size());
+    const size_t in_bytes = need - jobs_at;
+    const size_t probe_at = place(sizeof(anc::PlainJob) * njobs);
+    const size_t counters_at = place((4 + kClasses) * sizeof(int));   // one per dense kind (1 .. 3), one per sparse class (4 ..)
+    size_t group_at[3] = {0, 0, 0};
+    for (int ci = 0; ci < 3; ++ci)
+        if (sparse_plans[ci].np_max)
+            group_at[ci] = place(4 * anc::sparse_group_scratch(sparse_plans[ci].np_max, class_first[ci + 1] - class_first[ci], sms));
+    DevBuf<uint8_t> arena;
+    CK(arena.ensure(need));
+    int* const counters = reinterpret_cast<int*>(arena.p + counters_at);
+    int2* const d_items = reinterpret_cast<int2*>(arena.p + items_at);
+    const anc::PlainJob* const d_jobs = reinterpret_cast<const anc::PlainJob*>(arena.p + jobs_at);
+    anc::PlainJob* const d_probe = reinterpret_cast<anc::PlainJob*>(arena.p + probe_at);
+    std::vector<anc::PlainJob> pj(njobs);
+    for (const Prepared& p : prep) {
+        const anc_job& j = jobs[p.idx];
+        const JobPlace& a = at[p.idx];
+        OutPtrs out{reinterpret_cast<uint32_t*>(arena.p + a.spins), reinterpret_cast<long long*>(arena.p + a.sh),
+                    reinterpret_cast<long long*>(arena.p + a.bs), reinterpret_cast<long long*>(arena.p + a.fl),
+                    j.trace ? reinterpret_cast<int32_t*>(arena.p + a.trace) : nullptr, nullptr};
+        pj[p.idx] = make_job(j.inst, j.tb, j.seed, j.trial_offset, j.nchains, p.hclamp, out);
+    }
+    // from here on work is enqueued: a failure waits for the streams before the memory above is freed
+    auto drain = [&](int rc) {
+        for (const Side& sd : side)
+            if (sd.st) cudaStreamSynchronize(sd.st);
+        cudaStreamSynchronize(st);
+        return rc;
+    };
+    std::vector<uint8_t> staging(std::max(in_bytes, result_bytes));
+    std::memcpy(staging.data(), pj.data(), sizeof(anc::PlainJob) * njobs);
+    std::memcpy(staging.data() + (items_at - jobs_at), all_items.data(), sizeof(int2) * all_items.size());
+    {
+        cudaError_t e = cudaMemcpyAsync(arena.p + jobs_at, staging.data(), in_bytes, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);     // staging is used again below
+        if (e != cudaSuccess) return drain(cuda_fail(e, "job table"));
+    }
+    auto launch_sparse = [&](const anc::PlainJob* djobs, int variant) -> int {
+        for (int ci = kClasses - 1; ci >= 0; --ci) {
+            const KindPlan& kp = sparse_plans[ci];
+            if (!kp.np_max) continue;
+            cudaStream_t cst = ci == main_class ? st : side[ci].st;
+            cudaError_t e = cudaSuccess;
+            if (ci != main_class) {
+                e = cudaEventRecord(side[ci].fork, st);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(cst, side[ci].fork, 0);
+            }
+            anc::PlainLaunch L{};
+            L.sparse_variant = variant;
+            L.jobs = djobs;
+            L.items = d_items + first_item[0] + class_first[ci];
+            L.nitems = class_first[ci + 1] - class_first[ci];
+            L.next_item = counters + 4 + ci;
+            L.np_max = kp.np_max;
+            L.nwj_max = kp.np_max / 32;
+            L.np_min = kp.np_min;
+            L.groups = ci < 3;
+            for (const Prepared& p : prep) L.clamp = L.clamp || p.hclamp > 0;
+            L.group_h = L.groups ? reinterpret_cast<int32_t*>(arena.p + group_at[ci]) : nullptr;
+            if (e == cudaSuccess) e = cudaMemsetAsync(L.next_item, 0, sizeof(int), cst);
+            if (e != cudaSuccess) return cuda_fail(e, "sparse launch");
+            const int rc = anc::sparse_launch(L, kp.per_sm, sms, cst);
+            if (rc) return cuda_fail(cudaError_t(rc), "plain engine launch");
+        }
+        for (const Side& sd : side) {
+            if (!sd.st) continue;
+            cudaError_t e = cudaEventRecord(sd.join, sd.st);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(st, sd.join, 0);
+            if (e != cudaSuccess) return cuda_fail(e, "sparse launch");
+        }
+        return ANC_OK;
+    };
     auto launch_kind = [&](int ki, const anc::PlainJob* djobs, int variant) -> int {
+        if (ki == 0) return launch_sparse(djobs, variant);
         const KindPlan& kp = plans[ki];
         anc::PlainLaunch L{};
         L.sparse_variant = variant;
         L.jobs = djobs;
-        L.items = d_items[ki].p;
+        L.items = d_items + first_item[ki];
         L.nitems = nitems[ki];
-        L.next_item = counters.p + ki;
+        L.next_item = counters + ki;
         L.np_max = kp.np_max;
         L.nwj_max = kp.nwj_max;
         L.stream = kp.stream ? 1 : 0;
         const int grid = std::max(1, std::min(L.nitems, kp.per_sm * sms));
-        cudaError_t e = cudaMemsetAsync(counters.p + ki, 0, sizeof(int), st);
+        cudaError_t e = cudaMemsetAsync(counters + ki, 0, sizeof(int), st);
         if (e != cudaSuccess) return cuda_fail(e, "memset");
         const int rc = anc::plain_launch(L, kKinds[ki], kp.P, grid, kp.smem, st);
         return rc ? cuda_fail(cudaError_t(rc), "plain engine launch") : ANC_OK;
@@ -1400,15 +1597,13 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
         if (sparse_variant < 0) {
             std::vector<anc::PlainJob> probe = pj;
             for (int k = 0; k < njobs; ++k) probe[k].tab.S = std::min(probe[k].tab.S, 64);
-            DevBuf<anc::PlainJob> d_probe;
-            CK(d_probe.ensure(njobs));
-            CK(cudaMemcpy(d_probe.p, probe.data(), sizeof(anc::PlainJob) * njobs, cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(d_probe, probe.data(), sizeof(anc::PlainJob) * njobs, cudaMemcpyHostToDevice));
             float best = 0.f;
             for (int v = 0; v < anc::kSparseVariants; ++v) {
                 float ms = 0.f;
                 for (int rep = 0; rep < 2; ++rep) {
                     CK(cudaEventRecord(e0, st));
-                    const int rc = launch_kind(0, d_probe.p, v);
+                    const int rc = launch_kind(0, d_probe, v);
                     if (rc) return drain(rc);
                     CK(cudaEventRecord(e1, st));
                     CK(cudaEventSynchronize(e1));
@@ -1423,22 +1618,25 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
     if (cudaEventRecord(e0, st) != cudaSuccess) return drain(cuda_fail(cudaGetLastError(), "event"));
     for (int ki = 0; ki < 4; ++ki) {
         if (!nitems[ki]) continue;
-        const int rc = launch_kind(ki, d_jobs.p, ki == 0 ? std::max(0, sparse_variant) : 0);
+        const int rc = launch_kind(ki, d_jobs, ki == 0 ? std::max(0, sparse_variant) : 0);
         if (rc) return drain(rc);
     }
     if (cudaEventRecord(e1, st) != cudaSuccess) return drain(cuda_fail(cudaGetLastError(), "event"));
-    for (const Prepared& p : prep) {
-        const anc_job& j = jobs[p.idx];
-        JobBufs& b = *bufs[p.idx];
-        cudaError_t e = cudaMemcpyAsync(j.spins, b.spins.p, size_t(j.inst->nw) * j.nchains * 4, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(j.sum_sh, b.sh.p, size_t(j.nchains) * 8, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess && j.sum_bs) e = cudaMemcpyAsync(j.sum_bs, b.bs.p, size_t(j.nchains) * 8, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess && j.flips) e = cudaMemcpyAsync(j.flips, b.fl.p, size_t(j.nchains) * 8, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess && j.trace)
-            e = cudaMemcpyAsync(j.trace, b.trace.p, size_t(j.nchains) * j.tb->S * 4, cudaMemcpyDeviceToHost, st);
-        if (e != cudaSuccess) return drain(cuda_fail(e, "result copy"));
-    }
+    cudaError_t ce = cudaMemcpyAsync(staging.data(), arena.p, result_bytes, cudaMemcpyDeviceToHost, st);
+    for (int k = 0; k < njobs && ce == cudaSuccess; ++k)
+        if (jobs[k].trace)
+            ce = cudaMemcpyAsync(jobs[k].trace, arena.p + at[k].trace, size_t(jobs[k].nchains) * jobs[k].tb->S * 4,
+                                 cudaMemcpyDeviceToHost, st);
+    if (ce != cudaSuccess) return drain(cuda_fail(ce, "result copy"));
     CK(cudaStreamSynchronize(st));
+    for (int k = 0; k < njobs; ++k) {
+        const anc_job& j = jobs[k];
+        const size_t c = size_t(j.nchains) * 8;
+        std::memcpy(j.spins, staging.data() + at[k].spins, size_t(j.inst->nw) * j.nchains * 4);
+        std::memcpy(j.sum_sh, staging.data() + at[k].sh, c);
+        if (j.sum_bs) std::memcpy(j.sum_bs, staging.data() + at[k].bs, c);
+        if (j.flips) std::memcpy(j.flips, staging.data() + at[k].fl, c);
+    }
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     g_dev_ms = ms;
@@ -1592,7 +1790,8 @@ extern "C" int anc_run_batch_noalloc(int njobs, const anc_device_job* jobs, void
         L.np_max = kp.np_max;
         L.nwj_max = kp.nwj_max;
         L.stream = kp.stream ? 1 : 0;
-        const int rc = anc::plain_launch(L, K, kp.P, std::max(1, std::min(cnt, kp.per_sm * sms)), kp.smem, st);
+        const int rc = K == 0 ? anc::sparse_launch(L, kp.per_sm, sms, st)
+                              : anc::plain_launch(L, K, kp.P, std::max(1, std::min(cnt, kp.per_sm * sms)), kp.smem, st);
         if (rc) return cuda_fail(cudaError_t(rc), "plain engine launch");
     }
     return ANC_OK;

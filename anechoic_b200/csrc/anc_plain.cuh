@@ -34,8 +34,15 @@ struct PlainJob {
     const uint32_t* planes;            // dense: [max(K,1)][np][nwj]
     const int32_t* row_ptr;            // sparse: [n + 1] (csr16: in words of two edges)
     const uint32_t* adj;               // sparse: (y << 8) | uint8(J_xy); csr16: two 16-bit edges per word
-    int csr16;                         // sparse, every J_xy = +-1 and n < 32767: edge = y | [J_xy = -1] << 15, rows
-                                       // padded to whole words with the skip edge 0x7fff
+    int csr16;                         // sparse, every J_xy = +-1 and np <= kEdgePad: edge = y | [J_xy = -1] << 15, rows
+                                       // padded to whole words with the edge kEdgePad
+    // the rows once more, for launches in groups (every J_xy = +-1, at most kGroupDegree edges per row, np <= kGroupNp; else
+    // null): slices of 32 rows, word e of row 32 s + i at slice_info[s].x + 32 e + i, its + edges in the first
+    // slice_info[s].y & 0xffff words and its - edges in the next slice_info[s].y >> 16; a word holds
+    // two edges as byte offsets 8 y (y >= np: no edge)
+    const uint32_t* slices;
+    const uint2* slice_info;
+    const uint32_t* row_counts;        // edges | - edges << 8
     const int32_t* bias;               // [n] or null
     DevTables tab;
     uint64_t seed;
@@ -65,10 +72,21 @@ struct PlainLaunch {
     int nitems;
     int* next_item;                    // queue head (zeroed before launch)
     int np_max, nwj_max;               // shared-memory layout
+    int np_min;                        // sparse batches: the smallest job's np
     int stream;                        // 1: dense counts go into the fields set by set (one result buffer)
     int sparse_variant;                // CSR pass variant (kSparseVariants index; 0 = rows 1 x edges 8 per lane)
+    int groups;                        // sparse: items are groups of kGroupReplicas trials, every job has slices
+    int clamp;                         // sparse groups: some job has hclamp > 0
+    int32_t* group_h;                  // sparse_group_scratch words
     int dense_variant;                 // dense pass variant (dense_variants(K) of them; 0 = the default)
 };
+
+constexpr uint32_t kEdgePad = 0x7fe0;  // padding edge of csr16 rows
+
+// Sparse jobs with unit weights and short rows run several replicas of an instance together (sparse_engine.cu).
+constexpr int kGroupReplicas = 8;
+constexpr int kGroupDegree = 120;      // a row's four byte sums stay below 256
+constexpr int kGroupNp = 7936;         // a slot's byte offset fits 16 bits, padding included
 
 // CSR pass variants the host's tuner chooses among: {lane groups' rows in flight, edges per lane fetched before any
 // is applied}. Every variant computes the same fields (integer atomics into shared memory), only the time differs.
@@ -103,7 +121,13 @@ inline size_t plain_smem_plan(int np_max, int nwj_max, int K, int P, bool* strea
     return *stream ? plain_smem_bytes(np_max, nwj_max, K, P, true) : full;
 }
 
-// Host launcher (plain_engine.cu). Returns a cudaError_t value.
+// Host launchers; they return a cudaError_t value. Sparse jobs (K = 0, sparse_engine.cu): co-resident CTAs per SM of the
+// several-anneals-per-SM form, and the launch, which runs one anneal per SM when the anneals are no more than the SMs.
+int sparse_max_blocks_per_sm(int np_max, int* out);
+int sparse_launch(const PlainLaunch& L, int per_sm, int sms, cudaStream_t stream);
+size_t sparse_group_scratch(int np_max, int nitems, int sms);   // words of L.group_h
+bool sparse_groups(int np, double degree, int64_t anneals, int sms);   // whether a launch of so many anneals runs in groups
+// Dense jobs (plain_engine.cu)
 int plain_launch(const PlainLaunch& L, int K, int P, int grid, size_t smem, cudaStream_t stream);
 int plain_max_blocks_per_sm(int K, int P, size_t smem, int* out, bool stream = false);
 
