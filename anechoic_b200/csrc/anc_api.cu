@@ -12,6 +12,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/anechoic.h"
@@ -70,6 +71,61 @@ struct DevBuf {
         return e;
     }
 };
+
+// Device memory of anc_run_batch calls. One block per device, of at most kKeepBytes, is kept between calls (allocating and
+// freeing 100 MB took up to 20 ms a call); concurrent calls allocate their own. A call has synchronised its streams before it
+// gives its block back. The kept blocks are freed with the last instance.
+class BatchMemory {
+public:
+    ~BatchMemory() { give(); }
+    cudaError_t take(int dev, size_t bytes) {
+        give();
+        dev_ = dev;
+        std::lock_guard<std::mutex> lock(mu_);
+        auto it = kept_.find(dev);
+        if (it != kept_.end() && it->second.second >= bytes) {
+            std::tie(p, n_) = it->second;
+            kept_.erase(it);
+            return cudaSuccess;
+        }
+        n_ = std::max<size_t>(bytes, 1);
+        return cudaMalloc(&p, n_);
+    }
+    static void instance_created() {
+        std::lock_guard<std::mutex> lock(mu_);
+        ++instances_;
+    }
+    static void instance_gone() {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (--instances_ > 0) return;
+        for (auto& k : kept_) cudaFree(k.second.first);
+        kept_.clear();
+    }
+    uint8_t* p = nullptr;
+
+private:
+    static constexpr size_t kKeepBytes = size_t(256) << 20;
+    void give() {
+        if (!p) return;
+        std::lock_guard<std::mutex> lock(mu_);
+        auto it = kept_.find(dev_);
+        if (n_ <= kKeepBytes && instances_ > 0 && (it == kept_.end() || it->second.second < n_)) {
+            if (it != kept_.end()) cudaFree(it->second.first);
+            kept_[dev_] = {p, n_};
+        } else {
+            cudaFree(p);
+        }
+        p = nullptr;
+    }
+    int dev_ = 0;
+    size_t n_ = 0;
+    static std::mutex mu_;
+    static std::map<int, std::pair<uint8_t*, size_t>> kept_;
+    static long instances_;
+};
+std::mutex BatchMemory::mu_;
+std::map<int, std::pair<uint8_t*, size_t>> BatchMemory::kept_;
+long BatchMemory::instances_ = 0;
 
 int pad_np(int n) { return std::max(2048, ((n + 255) / 256) * 256); }
 
@@ -172,7 +228,9 @@ struct anc_instance {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int device = 0, sms = 0;
+    anc_instance() { BatchMemory::instance_created(); }
     ~anc_instance() {
+        BatchMemory::instance_gone();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);
@@ -1070,9 +1128,6 @@ int anc_instance_create_csr(int n, const int32_t* row_ptr, const int32_t* col, c
         if (row_ptr[x + 1] < row_ptr[x]) return fail(ANC_EINVAL, "row_ptr not monotone at %d", x);
     const int64_t nnz = row_ptr[n];
     if (nnz > 0 && (!col || !val)) return fail(ANC_EINVAL, "col and val required");
-    std::vector<std::pair<int64_t, int8_t>> keys, keysT;
-    keys.reserve(nnz);
-    keysT.reserve(nnz);
     std::vector<uint32_t> adj(nnz);
     for (int x = 0; x < n; ++x)
         for (int k = row_ptr[x]; k < row_ptr[x + 1]; ++k) {
@@ -1081,15 +1136,29 @@ int anc_instance_create_csr(int n, const int32_t* row_ptr, const int32_t* col, c
             if (y == x) return fail(ANC_EINVAL, "nonzero diagonal coupling at %d", x);
             if (val[k] == 0) return fail(ANC_EINVAL, "explicit zero coupling in row %d", x);
             if (val[k] == -128) return fail(ANC_EINVAL, "coupling -128 not supported");
-            keys.push_back({int64_t(x) * n + y, val[k]});
-            keysT.push_back({int64_t(y) * n + x, val[k]});
             adj[k] = (uint32_t(y) << 8) | uint8_t(val[k]);
         }
-    std::sort(keys.begin(), keys.end());
-    std::sort(keysT.begin(), keysT.end());
-    if (keys != keysT) return fail(ANC_EINVAL, "J not symmetric (or duplicate entries)");
-    for (size_t i = 1; i < keys.size(); ++i)
-        if (keys[i].first == keys[i - 1].first) return fail(ANC_EINVAL, "duplicate coupling");
+    {
+        // symmetric: the transposed rows, gathered in ascending order of their columns, equal the sorted rows
+        std::vector<int64_t> first(size_t(n) + 1, 0);
+        for (int64_t k = 0; k < nnz; ++k) ++first[col[k] + 1];
+        for (int x = 0; x < n; ++x) first[x + 1] += first[x];
+        std::vector<std::pair<int, int8_t>> tr(nnz), row;
+        std::vector<int64_t> next(first.begin(), first.end() - 1);
+        for (int x = 0; x < n; ++x)
+            for (int k = row_ptr[x]; k < row_ptr[x + 1]; ++k) tr[next[col[k]]++] = {x, val[k]};
+        bool duplicate = false;
+        for (int x = 0; x < n; ++x) {
+            row.clear();
+            for (int k = row_ptr[x]; k < row_ptr[x + 1]; ++k) row.push_back({col[k], val[k]});
+            const auto t0 = tr.begin() + first[x], t1 = tr.begin() + first[x + 1];
+            if (!std::is_sorted(row.begin(), row.end())) std::sort(row.begin(), row.end());
+            if (!std::is_sorted(t0, t1)) std::sort(t0, t1);
+            if (!std::equal(row.begin(), row.end(), t0, t1)) return fail(ANC_EINVAL, "J not symmetric (or duplicate entries)");
+            for (size_t i = 1; i < row.size(); ++i) duplicate = duplicate || row[i].first == row[i - 1].first;
+        }
+        if (duplicate) return fail(ANC_EINVAL, "duplicate coupling");
+    }
     std::unique_ptr<anc_instance> I(new anc_instance());
     I->n = n;
     I->np = pad_np(n);
@@ -1496,8 +1565,8 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
     for (int ci = 0; ci < 3; ++ci)
         if (sparse_plans[ci].np_max)
             group_at[ci] = place(4 * anc::sparse_group_scratch(sparse_plans[ci].np_max, class_first[ci + 1] - class_first[ci], sms));
-    DevBuf<uint8_t> arena;
-    CK(arena.ensure(need));
+    BatchMemory arena;
+    CK(arena.take(dev, need));
     int* const counters = reinterpret_cast<int*>(arena.p + counters_at);
     int2* const d_items = reinterpret_cast<int2*>(arena.p + items_at);
     const anc::PlainJob* const d_jobs = reinterpret_cast<const anc::PlainJob*>(arena.p + jobs_at);
