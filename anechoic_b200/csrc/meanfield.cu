@@ -13,14 +13,18 @@
 
 namespace anc {
 
+namespace {
+struct PsForm;
+}
+
 struct MfContext {
     int n = 0, npad = 0;
     __nv_bfloat16* J = nullptr;       // [npad][npad] (zero padded)
     float* bias = nullptr;            // [npad]
-    float* partial = nullptr;         // [npad / 256][64][npad] split-K partial products
+    float* partial = nullptr;         // [npad / 256][64][npad] split-K partial products (twice in the persistent form)
     float* mring = nullptr;           // forward ring: 3 x [64][npad]
-    __nv_bfloat16* xm = nullptr;      // [3][64][npad]: hi / mid / lo of the m operand
-    __nv_bfloat16* xp = nullptr;      // [3][64][npad]: hi / mid / lo of the adjoint operand
+    __nv_bfloat16* xm = nullptr;      // [3][64][npad]: hi / mid / lo of the m operand (twice in the persistent form)
+    __nv_bfloat16* xp = nullptr;      // [3][64][npad]: hi / mid / lo of the adjoint operand (likewise)
     float* seg_m = nullptr;           // [kMfCheckpoint + 2][64][npad]: m_{t0-1} .. m_{t0+16} of a segment
     float* seg_P = nullptr;           // [kMfCheckpoint][64][npad]
     float* pbar = nullptr;            // [3][64][npad] ring of pbar_t
@@ -29,6 +33,8 @@ struct MfContext {
     float* gparts = nullptr;          // [S][4][nch][64] per-chunk schedule-gradient sums
     int nbuf_steps = 0;
     int* err = nullptr;               // device error word
+    const PsForm* form = nullptr;   // the persistent form, null: the launch sequences
+    unsigned* cnt = nullptr;          // the persistent form's counters
     uint64_t wait_ns = ptx::kWaitNs;  // limit of each device wait before the kernel gives up (recorded in the graphs)
     CUtensorMap mapJ, mapXm[3], mapXp[3];
     // CUDA graphs of the forward and adjoint launch sequences (one step count each), captured on internal buffers:
@@ -352,6 +358,457 @@ __global__ void mf_gsum_kernel(const float* __restrict__ gparts, int S, int nch,
     gsched[e] = v;
 }
 
+// ---------------------------------------------------------------------------------------------- persistent form
+// The whole forward pass, or the whole adjoint, in one cooperative launch: every CTA keeps its tile of J on chip and walks
+// through the steps, where the launch sequences below reload J and pay two launches a step. The arithmetic is that of the
+// kernels above, operation for operation and in their order, so the results are bit-identical.
+//
+// The NR = 64, 32 or 16 replicas of a replica group never meet those of another. Within a group, CTA (rows, K chunk j) has
+// RB = 1 or 2 blocks of 128 rows of J by the 256 columns of chunk j: in TMEM (RB = 1; an MMA then reads only its B tile from
+// shared memory) or in shared memory (RB = 2). The 256 rows of chunk c belong to the GS CTAs of team c, which also share the
+// chunk's elementwise work: unit (replica, c) goes to a quarter of 256 of the CTA's 1024 threads. Two counters per chunk
+// replace the launch boundaries: a_cnt[c], the team's GEMMs done (its partials may be summed), and b_cnt[c], its elementwise
+// steps done (the BF16 terms of chunk c may be multiplied). What a step reads of the other chunks (the soft counts, s_t)
+// was published before the GEMMs whose partials it waited for. Partials and terms are double-buffered: a buffer is written
+// again only after a chain of both waits that covers all of its readers; at the segment ends of the adjoint, where that
+// chain is cut, all CTAs meet (e_cnt).
+// Bound: the chain of a step (counter, terms from L2, 48 MMAs, epilogue, counter, partials, tanh, counter), 13300 cycles at
+// n = 2000, of which the exchange of the partials through L2 takes half.
+constexpr int kPsThreads = 1024;
+constexpr int kPsChunks = 12;              // at most this many chunks: nch^2 CTAs of two row blocks, one CTA per SM
+constexpr int kCntStride = 32;             // counters in lines of their own
+constexpr int kErrA = 13, kErrB = 14, kErrE = 15;
+
+int ps_pad(int nch) { return (nch + 3) / 4 * 4; }
+
+struct PsArgs {
+    int n, npad, S;
+    const float *bias, *beta, *q, *u, *w;
+    float* partial;            // [2][nch][64][nch up to a multiple of 4, zeros][256]: chunk, replica, K chunk, row
+    __nv_bfloat16* xm;         // [2][nch][64][3][256] terms of m: chunk, replica, term, column
+    __nv_bfloat16* xp;         // [2][nch][64][3][256] terms of pbar (adjoint)
+    float* nbuf;               // [S + 1][64][kPsChunks] soft counts per chunk, zero beyond nch
+    unsigned* cnt;             // per replica group a_cnt[nch], b_cnt[nch]; e_cnt (zeroed)
+    int* err;
+    uint64_t wait_ns;
+    const __nv_bfloat16* J;
+    // forward
+    const float *m0, *mprev;
+    float *ring, *ckpt, *m_out;
+    // adjoint
+    const float *ckpt_in, *g_m;
+    float *seg_m, *seg_P, *pbar;
+    float* svec;               // [3][64][kPsChunks], zero beyond nch
+    float* gparts;
+};
+
+__device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc));
+}
+
+__device__ __forceinline__ void ps_ld(uint32_t taddr, uint32_t (&x)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void ps_ld(uint32_t taddr, uint32_t (&x)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void ps_ld(uint32_t taddr, uint32_t (&x)[2]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(x[0]), "=r"(x[1]) : "r"(taddr));
+}
+
+// block_sum's tree over the 8 warps of a quarter of the CTA; the result is valid in the quarter's first warp. Calls
+// alternate between two halves of red, so one barrier a call keeps a half's readers and its next writers apart.
+template <int NV>
+__device__ __forceinline__ void unit_sum(float (&v)[NV], float* red, int unit) {
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) red[k * 8 + warp] = v[k];
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + unit) : "memory");
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            float x = lane < 8 ? red[k * 8 + lane] : 0.f;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            v[k] = x;
+        }
+    }
+}
+
+// Sum of up to kPsChunks values in chunk order, past L1 (other CTAs wrote them during this launch). The zeros that pad the
+// chunks to a multiple of 4 change no bit of it.
+__device__ __forceinline__ float sum_parts_cg(const float* parts, int nch) {
+    const float4* p = reinterpret_cast<const float4*>(parts);
+    float4 a = __ldcg(p), b = make_float4(0.f, 0.f, 0.f, 0.f), c = b;
+    if (nch > 4) b = __ldcg(p + 1);
+    if (nch > 8) c = __ldcg(p + 2);
+    float v = (((0.f + a.x) + a.y) + a.z) + a.w;
+    if (nch > 4) v = (((v + b.x) + b.y) + b.z) + b.w;
+    if (nch > 8) v = (((v + c.x) + c.y) + c.z) + c.w;
+    return v;
+}
+
+template <int RB, int NR>
+constexpr size_t ps_smem() { return 1024 + (RB == 1 ? 0 : RB * 4 * kATile) + 12 * size_t(NR) * 128 + 64; }
+
+template <int RB, int NR, bool ADJOINT>
+__global__ void __launch_bounds__(kPsThreads, 1) mf_steps_kernel(const __grid_constant__ CUtensorMap mapJ, const __grid_constant__ PsArgs A) {
+    constexpr uint32_t IDESC =
+        (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(NR >> 3) << 17) | (uint32_t(kRows >> 4) << 24);
+    constexpr int BT = NR * 128, CW = NR / 8, NG = kRep / NR;   // bytes of a B atom; columns per epilogue warp; groups
+    constexpr uint32_t kACol = 320;                             // TMEM columns: 5 x NR accumulators, J from 320
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    __shared__ float red_s[4][2][24];
+    __shared__ int s_ok;
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sa = smem;                                         // [RB][4] J atoms (RB = 2)
+    uint8_t* sb = sa + (RB == 1 ? 0 : RB * 4 * kATile);         // [3 terms][4] operand atoms
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sb + 12 * BT);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
+    const uint32_t bar_j = smem_u32(bars), bar_done = smem_u32(bars + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, unit = tid >> 8, ut = tid & 255;
+    const int npad = A.npad, nch = npad / kKC, nch4 = (nch + 3) & ~3, n = A.n, S = A.S;
+    const int nrow = RB == 1 ? 2 * nch : nch;             // CTAs per K chunk and replica group
+    const int rg = int(blockIdx.x) % NG, rowi = int(blockIdx.x) / NG % nrow, j = int(blockIdx.x) / NG / nrow;
+    const int c = RB == 1 ? rowi >> 1 : rowi;             // own chunk
+    const int gs = RB == 1 ? 2 * nch : nch, member = RB == 1 ? (rowi & 1) * nch + j : j;
+    const int half = RB == 1 ? (rowi & 1) * kRows : 0;    // first own row within the chunk
+    const size_t plane = size_t(kRep) * npad;
+    unsigned* const a_cnt = A.cnt + (rg * 2 * nch + c) * kCntStride;
+    unsigned* const b_own = a_cnt + nch * kCntStride;
+    const unsigned* const b_in = A.cnt + (rg * 2 * nch + nch + j) * kCntStride;
+    unsigned* const e_cnt = A.cnt + NG * 2 * nch * kCntStride;
+
+    if (tid == 0) {
+        s_ok = 1;
+        mbar_init(bar_j, 1);
+        mbar_init(bar_done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot, tlane = tmem + (uint32_t((warp & 3) * 32) << 16);
+    if constexpr (RB == 1) {
+        // warp w: rows 32 (w % 4) .., BF16 columns 32 (w / 4) .. of the tile, two to a TMEM column
+        const uint4* src = reinterpret_cast<const uint4*>(A.J + size_t(rowi * kRows + (warp & 3) * 32 + lane) * npad + j * kKC +
+                                                          32 * (warp >> 2));
+        uint32_t v[16];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint4 x = __ldg(src + k);
+            v[4 * k] = x.x;
+            v[4 * k + 1] = x.y;
+            v[4 * k + 2] = x.z;
+            v[4 * k + 3] = x.w;
+        }
+        tmem_st16(tlane + kACol + uint32_t(16 * (warp >> 2)), v);
+        tmem_wait_st();
+        tc_fence_before();
+    } else if (tid == 0) {
+        mbar_arrive_expect_tx(bar_j, RB * 4 * kATile);
+        for (int rb = 0; rb < RB; ++rb)
+            for (int a = 0; a < 4; ++a)
+                tma_load_2d(smem_u32(sa + (rb * 4 + a) * kATile), &mapJ, j * kKC + 64 * a, (rowi * RB + rb) * kRows, bar_j);
+        if (!mbar_wait_for(bar_j, 0u, A.err, kErrFull, A.wait_ns)) {
+            mbar_wait_for(bar_j, 0u, nullptr, 0, kWaitNs);
+            s_ok = 0;
+        }
+    }
+    unsigned ng = 0, nb = 0, ne = 0, ns = 0;              // GEMMs, elementwise steps, meetings and sums so far
+    uint32_t done_ph = 0u;
+
+    // Thread 0 waits (bounded) for a counter, everyone behind it; after a wait that gave up the CTA waits for nothing more
+    // and walks on, so that its peers still see every arrival.
+    auto wait_cnt = [&](const unsigned* p, unsigned target, int code) {
+        if (tid == 0 && s_ok) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+            if (v < target) {
+                const uint64_t t0 = globaltimer();
+                for (uint32_t k = 1;; ++k) {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+                    if (v >= target) break;
+                    if (((k & 63u) == 0 || A.wait_ns == 0) && (globaltimer() - t0 >= A.wait_ns || err_set(A.err))) {
+                        atomicCAS(A.err, 0, code);
+                        s_ok = 0;
+                        break;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    };
+    auto arrive = [&](unsigned* p) {
+        __syncthreads();
+        if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+    };
+    // This thread's 16-byte pieces of the operand: piece tid % 32 of rows (replicas) tid / 32 + 32 k of each term
+    constexpr int PIECES = NR >= 32 ? NR / 32 : 1;
+    const uint32_t b_dst = smem_u32(sb) + uint32_t((lane >> 3) * BT + warp * 128 + (((lane & 7) ^ (warp & 7)) << 4));
+    const size_t b_src = (size_t(j * kRep + rg * NR + warp) * 3) * kKC + lane * 8;
+    // partial[ng parity][..][j] = J tile x the three terms x[..][chunk j]
+    auto gemm = [&](const __nv_bfloat16* x) {
+        wait_cnt(b_in, nb * unsigned(gs), kErrB);
+        const __nv_bfloat16* src = x + b_src;
+#pragma unroll
+        for (int term = 0; term < 3; ++term) {
+            if (NR >= 32 || warp < NR)
+#pragma unroll
+                for (int k = 0; k < PIECES; ++k)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(b_dst + uint32_t(term * 4 * BT + k * 32 * 128)),
+                                 "l"(src + (k * 32 * 3 + term) * kKC)
+                                 : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+#pragma unroll
+        for (int rb = 0; rb < RB; ++rb) {
+            const uint32_t ut0 = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint64_t da = sw128_desc(smem_u32(sa)) + uint64_t(rb * 4 * (kATile >> 4)), db = sw128_desc(smem_u32(sb));
+            auto mma = [&](uint32_t d, int term, int a, int kk, uint32_t acc) {
+                const uint64_t b = db + uint64_t((term * 4 + a) * (BT >> 4) + 2 * kk);
+                if constexpr (RB == 1)
+                    mma_f16_ta(d, ut0 + kACol + uint32_t(8 * (4 * a + kk)), b, IDESC, acc);
+                else
+                    mma_f16(d, da + uint64_t(a * (kATile >> 4) + 2 * kk), b, IDESC, acc);
+            };
+            // the leading term's products while the other two terms are on their way
+            if (rb == 0) {
+                asm volatile("cp.async.wait_group 2;" ::: "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncthreads();
+            }
+            if (warp == 0) {
+                tc_fence_after();
+                if (elect_one())
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) mma(ut0 + uint32_t(NR * a), 0, a, kk, kk != 0 ? 1u : 0u);
+                __syncwarp();
+            }
+            if (rb == 0) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncthreads();
+            }
+            if (warp == 0) {
+                if (elect_one()) {
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) {
+                            mma(ut0 + uint32_t(4 * NR), 1, a, kk, (a | kk) != 0 ? 1u : 0u);
+                            mma(ut0 + uint32_t(4 * NR), 2, a, kk, 1u);
+                        }
+                    mma_commit(bar_done);
+                }
+                __syncwarp();
+            }
+            if (!mbar_wait_for(bar_done, done_ph & 1u, A.err, kErrDone, A.wait_ns)) {
+                mbar_wait_for(bar_done, done_ph & 1u, nullptr, 0, kWaitNs);
+                s_ok = 0;
+            }
+            ++done_ph;
+            tc_fence_after();
+            // warp w: rows 32 (w % 4) .. of the block, replicas CW (w / 4) ..
+            const uint32_t tl = tlane + uint32_t(CW * (warp >> 2));
+            uint32_t v[5][CW];
+#pragma unroll
+            for (int a = 0; a < 5; ++a) ps_ld(tl + uint32_t(NR * a), v[a]);
+            tmem_wait_ld();
+            float* dst = A.partial + (size_t(((ng & 1u) * nch + c) * kRep + rg * NR + CW * (warp >> 2)) * nch4 + j) * kKC + half +
+                         rb * kRows + (warp & 3) * 32 + lane;
+#pragma unroll
+            for (int e = 0; e < CW; ++e) {
+                const float s01 = __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
+                const float s23 = __uint_as_float(v[2][e]) + __uint_as_float(v[3][e]);
+                __stcg(dst + e * (nch4 * kKC), (s01 + s23) + __uint_as_float(v[4][e]));
+            }
+            tc_fence_before();
+            if (rb + 1 < RB) __syncthreads();
+        }
+        ++ng;
+        arrive(a_cnt);
+    };
+    // sum of the split-K partials of the last GEMM for one element, in chunk order (the pads are zeros)
+    auto field = [&](int r) {
+        const float* p = A.partial + size_t((((ng - 1u) & 1u) * nch + c) * kRep + r) * (nch4 * kKC) + ut;
+        float v[kPsChunks], H = 0.f;
+#pragma unroll
+        for (int b = 0; b < kPsChunks; b += 4)
+            if (b < nch)
+#pragma unroll
+                for (int k = b; k < b + 4; ++k) v[k] = __ldcg(p + k * kKC);
+#pragma unroll
+        for (int b = 0; b < kPsChunks; b += 4)
+            if (b < nch)
+#pragma unroll
+                for (int k = b; k < b + 4; ++k) H += v[k];
+        return H;
+    };
+    const int i = c * kKC + ut;                           // this thread's column
+    const float bias = A.bias[i];
+    // the replicas of this quarter of the CTA
+    auto each = [&](auto f) {
+        for (int k = member + gs * unit; k < NR; k += 4 * gs) f(rg * NR + k);
+    };
+    auto terms = [&](float v, __nv_bfloat16* x, int r) { split_bf16(v, x + size_t(c * kRep + r) * (3 * kKC) + ut, kKC); };
+    auto red = [&]() { return red_s[unit][ns++ & 1u]; };
+    const size_t xbuf = 3 * plane;                        // elements of one of the two buffers of terms
+    // the BF16 terms and the soft count partials of m_t (mf_prep_kernel), from `m`
+    auto prep = [&](const float* m, int t, __nv_bfloat16* x) {
+        each([&](int r) {
+            const float v = m[size_t(r) * npad + i];
+            terms(v, x, r);
+            float acc[1] = {i < n ? 1.f - v * v : 0.f};
+            unit_sum(acc, red(), unit);
+            if (ut == 0) __stcg(A.nbuf + (size_t(t) * kRep + r) * kPsChunks + c, acc[0]);
+        });
+        ++nb;
+        arrive(b_own);
+    };
+    // one forward step t (mf_fwd_kernel): m_{t+1} into m_next, its terms into x, P_t into P_out when that is not null
+    auto forward = [&](int t, const float* m_cur, const float* m_prev, float* m_next, float* also, __nv_bfloat16* x, float* P_out) {
+        const float beta = __ldg(A.beta + t), q = __ldg(A.q + t), u = __ldg(A.u + t), w = __ldg(A.w + t);
+        wait_cnt(a_cnt, ng * unsigned(gs), kErrA);
+        each([&](int r) {
+            const float gamma = u * sum_parts_cg(A.nbuf + (size_t(t) * kRep + r) * kPsChunks, nch) + w;
+            const size_t idx = size_t(r) * npad + i;
+            const float H = field(r);
+            const float P = H + bias + q * m_cur[idx] - gamma * m_prev[idx];
+            const float mn = i < n ? tanhf(beta * P) : 0.f;
+            m_next[idx] = mn;
+            if (also) also[idx] = mn;
+            terms(mn, x, r);
+            if (P_out) P_out[idx] = P;
+            float acc[1] = {i < n ? 1.f - mn * mn : 0.f};
+            unit_sum(acc, red(), unit);
+            if (ut == 0) __stcg(A.nbuf + (size_t(t + 1) * kRep + r) * kPsChunks + c, acc[0]);
+        });
+        ++nb;
+        arrive(b_own);
+    };
+    __syncthreads();
+    tc_fence_after();
+
+    if constexpr (!ADJOINT) {
+        // m_t in ring slot (t + 1) % 3, touched by its owner threads only; checkpoints of (m_{t-1}, m_t) every 16 steps
+        each([&](int r) {
+            const size_t idx = size_t(r) * npad + i;
+            A.ring[idx] = A.mprev[idx];
+            A.ring[plane + idx] = A.m0[idx];
+        });
+        prep(A.m0, 0, A.xm);
+        for (int t = 0; t < S; ++t) {
+            const float *prev = A.ring + size_t(t % 3) * plane, *cur = A.ring + size_t((t + 1) % 3) * plane;
+            if (t % kMfCheckpoint == 0) {
+                float* ck = A.ckpt + size_t(t / kMfCheckpoint) * 2 * plane;
+                each([&](int r) {
+                    const size_t idx = size_t(r) * npad + i;
+                    ck[idx] = prev[idx];
+                    ck[plane + idx] = cur[idx];
+                });
+            }
+            gemm(A.xm + size_t(t & 1) * xbuf);
+            forward(t, cur, prev, A.ring + size_t((t + 2) % 3) * plane, t == S - 1 ? A.m_out : nullptr,
+                    A.xm + size_t((t + 1) & 1) * xbuf, nullptr);
+        }
+    } else {
+        unsigned pbn = 0;                                 // adjoint steps so far: the buffer of their terms
+        for (int seg = (S + kMfCheckpoint - 1) / kMfCheckpoint - 1; seg >= 0; --seg) {
+            const int t0 = seg * kMfCheckpoint, t1 = min(S, t0 + kMfCheckpoint);
+            // seg_m slot k holds m_{t0 - 1 + k}
+            const float* ck = A.ckpt_in + size_t(seg) * 2 * plane;
+            each([&](int r) {
+                const size_t idx = size_t(r) * npad + i;
+                A.seg_m[idx] = ck[idx];
+                A.seg_m[plane + idx] = ck[plane + idx];
+            });
+            prep(ck + plane, t0, A.xm);
+            for (int t = t0; t < t1; ++t) {
+                const int k = t - t0;
+                gemm(A.xm + size_t(k & 1) * xbuf);
+                forward(t, A.seg_m + size_t(k + 1) * plane, A.seg_m + size_t(k) * plane, A.seg_m + size_t(k + 2) * plane, nullptr,
+                        A.xm + size_t((k + 1) & 1) * xbuf, A.seg_P + size_t(k) * plane);
+            }
+            for (int t = t1 - 1; t >= t0; --t) {
+                const int k = t - t0;
+                const bool last = t == S - 1, far = t + 2 < S;
+                // one adjoint step (mf_bwd_kernel)
+                const float beta = __ldg(A.beta + t), q1 = last ? 0.f : __ldg(A.q + t + 1), u1 = last ? 0.f : __ldg(A.u + t + 1);
+                const float u2 = far ? __ldg(A.u + t + 2) : 0.f, w2 = far ? __ldg(A.w + t + 2) : 0.f;
+                if (!last) {
+                    gemm(A.xp + size_t((pbn - 1u) & 1u) * xbuf);
+                    wait_cnt(a_cnt, ng * unsigned(gs), kErrA);
+                }
+                each([&](int r) {
+                    const float us = last ? 0.f : 2.f * u1 * sum_parts_cg(A.svec + (size_t((t + 1) % 3) * kRep + r) * kPsChunks, nch);
+                    const float g2 = far ? u2 * sum_parts_cg(A.nbuf + (size_t(t + 2) * kRep + r) * kPsChunks, nch) + w2 : 0.f;
+                    const float nt = sum_parts_cg(A.nbuf + (size_t(t) * kRep + r) * kPsChunks, nch);
+                    const size_t idx = size_t(r) * npad + i;
+                    const float mn = A.seg_m[size_t(k + 2) * plane + idx];
+                    float G;
+                    if (last) {
+                        G = A.g_m[idx];
+                    } else {
+                        const float H = field(r);
+                        G = H + q1 * A.pbar[size_t((t + 1) % 3) * plane + idx] + us * mn;
+                        if (far) G -= g2 * A.pbar[size_t((t + 2) % 3) * plane + idx];
+                    }
+                    const float abar = i < n ? G * (1.f - mn * mn) : 0.f;
+                    const float pb = beta * abar;
+                    A.pbar[size_t(t % 3) * plane + idx] = pb;
+                    terms(pb, A.xp + size_t(pbn & 1u) * xbuf, r);
+                    float acc[3] = {abar * A.seg_P[size_t(k) * plane + idx], pb * A.seg_m[size_t(k + 1) * plane + idx],
+                                    pb * A.seg_m[size_t(k) * plane + idx]};
+                    unit_sum(acc, red(), unit);
+                    if (ut == 0) {
+                        __stcg(A.svec + (size_t(t % 3) * kRep + r) * kPsChunks + c, acc[2]);
+                        float* g = A.gparts + size_t(t) * 4 * nch * kRep;
+                        g[(0 * nch + c) * kRep + r] = acc[0];
+                        g[(1 * nch + c) * kRep + r] = acc[1];
+                        g[(2 * nch + c) * kRep + r] = -acc[2] * nt;
+                        g[(3 * nch + c) * kRep + r] = -acc[2];
+                    }
+                });
+                ++pbn;
+                ++nb;
+                arrive(b_own);
+            }
+            if (seg > 0) {
+                ++ne;
+                arrive(e_cnt);
+                wait_cnt(e_cnt, ne * gridDim.x, kErrE);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
 bool check(cudaError_t e, const char* what, std::string* why) {
     if (e == cudaSuccess) return true;
     if (why) *why = std::string(what) + ": " + cudaGetErrorString(e);
@@ -429,10 +886,84 @@ int ensure_steps(MfContext* c, int S, std::string* why) {
         *p = nullptr;
     }
     c->nbuf_steps = 0;
-    if (!check(cudaMalloc(&c->nbuf, size_t(S + 1) * nch(c) * kRep * sizeof(float)), "cudaMalloc", why) ||
+    const size_t nbytes = size_t(S + 1) * (c->form ? kPsChunks : nch(c)) * kRep * sizeof(float);
+    if (!check(cudaMalloc(&c->nbuf, nbytes), "cudaMalloc", why) || !check(cudaMemset(c->nbuf, 0, nbytes), "cudaMemset", why) ||
+        !check(cudaStreamSynchronize(nullptr), "cudaMemset", why) ||
         !check(cudaMalloc(&c->gparts, size_t(S) * 4 * nch(c) * kRep * sizeof(float)), "cudaMalloc", why))
         return -2;
     c->nbuf_steps = S;
+    return 0;
+}
+
+using PsKernel = void (*)(const CUtensorMap, const PsArgs);
+struct PsForm {
+    int rb, nr;                // row blocks per CTA, replicas per group
+    PsKernel fwd, adj;
+    size_t smem;
+    int grid(int nch) const { return (rb == 1 ? 2 : 1) * nch * nch * (kRep / nr); }
+};
+const PsForm kPsForms[] = {
+    {1, 16, mf_steps_kernel<1, 16, false>, mf_steps_kernel<1, 16, true>, ps_smem<1, 16>()},
+    {1, 32, mf_steps_kernel<1, 32, false>, mf_steps_kernel<1, 32, true>, ps_smem<1, 32>()},
+    {1, 64, mf_steps_kernel<1, 64, false>, mf_steps_kernel<1, 64, true>, ps_smem<1, 64>()},
+    {2, 64, mf_steps_kernel<2, 64, false>, mf_steps_kernel<2, 64, true>, ps_smem<2, 64>()},
+};
+
+size_t ps_cnt_bytes(int nch) { return size_t(2 * nch * (kRep / 16) + 1) * kCntStride * sizeof(unsigned); }
+
+// The persistent form: the first one whose CTAs fit one per SM, null (the launch sequences) where none does. Measured, a
+// forward / an adjoint step in us, launch sequence -> persistent: n = 700 10.0 / 18.7 -> 6.6 / 13.1, n = 2000 9.35 / 19.5 ->
+// 7.0 / 16.0, n = 3072 17.0 / 32.8 -> 13.0 / 27.9. One chunk (n <= 256) leaves it 8 CTAs: 8.4 / 15.2 -> 8.0 / 16.9, so it
+// stays with the launch sequences.
+const PsForm* ps_form(int npad) {
+    int dev = 0, sms = 0, coop = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop || npad / kKC < 2 || npad / kKC > kPsChunks)
+        return nullptr;
+    for (const PsForm& f : kPsForms) {
+        if (f.grid(npad / kKC) > sms) continue;
+        bool ok = true;
+        for (PsKernel kernel : {f.fwd, f.adj}) {
+            const void* k = reinterpret_cast<const void*>(kernel);
+            int per_sm = 0;
+            ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(f.smem)) == cudaSuccess &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPsThreads, f.smem) == cudaSuccess && per_sm >= 1;
+        }
+        if (ok) return &f;
+        cudaGetLastError();
+    }
+    return nullptr;
+}
+
+PsArgs ps_args(MfContext* c, int S, const float* beta, const float* q, const float* u, const float* w) {
+    PsArgs a{};
+    a.n = c->n;
+    a.npad = c->npad;
+    a.S = S;
+    a.J = c->J;
+    a.bias = c->bias;
+    a.beta = beta;
+    a.q = q;
+    a.u = u;
+    a.w = w;
+    a.partial = c->partial;
+    a.xm = c->xm;
+    a.xp = c->xp;
+    a.nbuf = c->nbuf;
+    a.cnt = c->cnt;
+    a.err = c->err;
+    a.wait_ns = c->wait_ns;
+    return a;
+}
+
+int ps_launch(MfContext* c, PsKernel kernel, PsArgs& a, cudaStream_t st, std::string* why) {
+    void* args[] = {&c->mapJ, &a};
+    if (!check(cudaMemsetAsync(c->cnt, 0, ps_cnt_bytes(nch(c)), st), "clear counters", why) ||
+        !check(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(c->form->grid(nch(c))),
+                                           dim3(kPsThreads), args, c->form->smem, st),
+               "mean-field steps launch", why))
+        return -2;
     return 0;
 }
 
@@ -456,19 +987,27 @@ int mf_create(const int8_t* J, const int32_t* bias, int n, MfContext** out, std:
     if (bias)
         for (int i = 0; i < n; ++i) bh[i] = float(bias[i]);
     const size_t plane = size_t(kRep) * npad;
+    c->form = ps_form(npad);
+    const size_t nbuf = c->form ? 2 : 1, kch = npad / kKC;
+    const size_t pbytes = (c->form ? 2 * size_t(ps_pad(kch)) : kch) * plane * sizeof(float);
+    const size_t sbytes = 3 * (c->form ? size_t(kPsChunks) : kch) * kRep * sizeof(float);
     bool ok = check(cudaMalloc(&c->J, Jh.size() * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
               check(cudaMemcpy(c->J, Jh.data(), Jh.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice), "upload J",
                     why) &&
               check(cudaMalloc(&c->bias, npad * sizeof(float)), "cudaMalloc", why) &&
               check(cudaMemcpy(c->bias, bh.data(), npad * sizeof(float), cudaMemcpyHostToDevice), "upload bias", why) &&
-              check(cudaMalloc(&c->partial, size_t(npad / kKC) * plane * sizeof(float)), "cudaMalloc", why) &&
+              check(cudaMalloc(&c->partial, pbytes), "cudaMalloc", why) &&
               check(cudaMalloc(&c->mring, 3 * plane * sizeof(float)), "cudaMalloc", why) &&
-              check(cudaMalloc(&c->xm, 3 * plane * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
-              check(cudaMalloc(&c->xp, 3 * plane * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
+              check(cudaMalloc(&c->xm, nbuf * 3 * plane * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
+              check(cudaMalloc(&c->xp, nbuf * 3 * plane * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->seg_m, (kMfCheckpoint + 2) * plane * sizeof(float)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->seg_P, kMfCheckpoint * plane * sizeof(float)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->pbar, 3 * plane * sizeof(float)), "cudaMalloc", why) &&
-              check(cudaMalloc(&c->svec, 3 * size_t(npad / kElemThreads) * kRep * sizeof(float)), "cudaMalloc", why) &&
+              check(cudaMalloc(&c->svec, sbytes), "cudaMalloc", why) &&
+              check(cudaMemset(c->partial, 0, pbytes), "cudaMemset", why) &&
+              check(cudaMemset(c->svec, 0, sbytes), "cudaMemset", why) &&
+              check(cudaStreamSynchronize(nullptr), "cudaMemset", why) &&
+              check(cudaMalloc(&c->cnt, ps_cnt_bytes(kch)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->err, sizeof(int)), "cudaMalloc", why) &&
               check(cudaMemset(c->err, 0, sizeof(int)), "cudaMemset", why);
     if (ok) {
@@ -659,6 +1198,17 @@ int mf_forward(MfContext* c, int S, const float* beta, const float* q, const flo
         if (why) *why = "invalid mean-field forward arguments";
         return -1;
     }
+    if (c->form) {
+        int rc = ensure_steps(c, S, why);
+        if (rc) return rc;
+        PsArgs a = ps_args(c, S, beta, q, u, w);
+        a.m0 = m0;
+        a.mprev = mprev;
+        a.ring = c->mring;
+        a.ckpt = ckpt;
+        a.m_out = m_out;
+        return ps_launch(c, c->form->fwd, a, st, why);
+    }
     int rc = ensure_io(c, S, why);
     if (rc) return rc;
     const size_t plane = size_t(kRep) * c->npad, nseg = (S + kMfCheckpoint - 1) / kMfCheckpoint;
@@ -683,6 +1233,23 @@ int mf_backward(MfContext* c, int S, const float* beta, const float* q, const fl
     if (!c || S < 1 || !beta || !q || !u || !w || !ckpt || !g_m || !gsched) {
         if (why) *why = "invalid mean-field backward arguments";
         return -1;
+    }
+    if (c->form) {
+        int rc = ensure_steps(c, S, why);
+        if (rc) return rc;
+        PsArgs a = ps_args(c, S, beta, q, u, w);
+        a.ckpt_in = ckpt;
+        a.g_m = g_m;
+        a.seg_m = c->seg_m;
+        a.seg_P = c->seg_P;
+        a.pbar = c->pbar;
+        a.svec = c->svec;
+        a.gparts = c->gparts;
+        rc = ps_launch(c, c->form->adj, a, st, why);
+        if (rc) return rc;
+        const int ne = S * 4 * kRep;
+        mf_gsum_kernel<<<(ne + 255) / 256, 256, 0, st>>>(c->gparts, S, nch(c), gsched);
+        return check(cudaGetLastError(), "mean-field gradient sum", why) ? 0 : -2;
     }
     int rc = ensure_io(c, S, why);
     if (rc) return rc;
@@ -741,7 +1308,7 @@ void mf_destroy(MfContext* c) {
                     static_cast<void*>(c->mring), static_cast<void*>(c->xm), static_cast<void*>(c->xp),
                     static_cast<void*>(c->seg_m), static_cast<void*>(c->seg_P), static_cast<void*>(c->pbar),
                     static_cast<void*>(c->svec), static_cast<void*>(c->nbuf), static_cast<void*>(c->gparts),
-                    static_cast<void*>(c->err)})
+                    static_cast<void*>(c->cnt), static_cast<void*>(c->err)})
         if (p) cudaFree(p);
     delete c;
 }
