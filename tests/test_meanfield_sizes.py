@@ -1,6 +1,6 @@
-"""GPU: the mean-field kernels at the sizes where their launch form changes -- one 256-column chunk (launch sequences), two
-and more chunks with 16, 32 and 64 replicas per group, two row blocks per CTA from nine chunks on, launch sequences again
-beyond twelve -- and at the checkpoint edges, against the FP64 recurrence.
+"""GPU: the mean-field kernels at the sizes where their launch form changes -- every number of 256-column chunks from one to
+eight (J in tensor memory; 16, 32 and 64 replicas per group), nine to twelve (two row blocks per CTA), launch sequences
+beyond -- and at the checkpoint edges (a last segment of one step), against the FP64 recurrence.
 
 The schedule keeps the map a contraction, so that rounding is not amplified with the steps: T >= 2 sqrt(n) and
 ||J|| <= 2 sqrt(0.6 n) give beta ||J|| <= 0.39, and beta gamma <= 0.07 with the counted correction. The error of one step
@@ -18,8 +18,8 @@ from tests.test_meanfield import _case, _rel
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,S", [(256, 17), (257, 33), (1000, 16), (1281, 1), (1600, 5), (2048, 18), (2049, 17), (3072, 2),
-                                 (3073, 17)])
+@pytest.mark.parametrize("n,S", [(256, 17), (257, 33), (700, 18), (1000, 16), (1281, 1), (1500, 33), (1600, 5), (2048, 18),
+                                 (2049, 17), (3072, 2), (3073, 17)])
 def test_forms_vs_fp64(cuda, n, S):
     inst = I.random_kbit(n, 2, 900 + n, pzero=0.4, bmax=3)
     theta = (4.0 * math.sqrt(n), math.log(2.0), 1.0, 0.5, 1.05)
