@@ -571,7 +571,7 @@ int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts
         // where the fp4 kernel runs, it is the planes kernel by another name: only its estimate changes, and not below
         // kFp4Floor
         const bool fp4 = fp4_candidate(I) && (!o || o->tensor_kind != ANC_TENSOR_PLANES);
-        const double t = tb->S * std::max(fp4 ? kFp4FloorUs : 0.0, anc::planes_step_us(I->n, I->info.maxabs, nchains));
+        const double t = tb->S * std::max(fp4 ? kFp4FloorUs : 0.0, anc::planes_step_us(I->n, I->info.maxabs, nchains, I->sms));
         if (t >= 0 && (est[ANC_ENGINE_TENSOR] < 0 || t < est[ANC_ENGINE_TENSOR])) {
             est[ANC_ENGINE_TENSOR] = t;
             if (est[best] < 0 || t < est[best] || best == ANC_ENGINE_TENSOR) {
@@ -753,6 +753,7 @@ int tune_sparse(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
     for (int v = 0; v < anc::kSparseVariants; ++v) {
         float ms = 0.f;
         for (int rep = 0; rep < 2; ++rep) {
+            job.tab.S = rep ? Sp : std::min(Sp, 8);       // the first launch loads the kernel and the caches
             CK(cudaEventRecord(I->ev0, st));
             rc = launch_plain_single(I, job, st, v);
             if (rc) return rc;
@@ -1665,21 +1666,23 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
         }
         if (sparse_variant < 0) {
             std::vector<anc::PlainJob> probe = pj;
-            for (int k = 0; k < njobs; ++k) probe[k].tab.S = std::min(probe[k].tab.S, 64);
-            CK(cudaMemcpy(d_probe, probe.data(), sizeof(anc::PlainJob) * njobs, cudaMemcpyHostToDevice));
             float best = 0.f;
-            for (int v = 0; v < anc::kSparseVariants; ++v) {
-                float ms = 0.f;
-                for (int rep = 0; rep < 2; ++rep) {
+            // each variant's first launch, of 8 steps, loads its kernels; all variants' timed launches follow
+            float ms[anc::kSparseVariants] = {};
+            for (int rep = 0; rep < 2; ++rep) {
+                for (int k = 0; k < njobs; ++k) probe[k].tab.S = std::min(pj[k].tab.S, rep ? 64 : 8);
+                CK(cudaMemcpy(d_probe, probe.data(), sizeof(anc::PlainJob) * njobs, cudaMemcpyHostToDevice));
+                for (int v = 0; v < anc::kSparseVariants; ++v) {
                     CK(cudaEventRecord(e0, st));
                     const int rc = launch_kind(0, d_probe, v);
                     if (rc) return drain(rc);
                     CK(cudaEventRecord(e1, st));
                     CK(cudaEventSynchronize(e1));
-                    CK(cudaEventElapsedTime(&ms, e0, e1));
+                    CK(cudaEventElapsedTime(&ms[v], e0, e1));
                 }
-                if (sparse_variant < 0 || ms < best) { best = ms; sparse_variant = v; }
             }
+            for (int v = 0; v < anc::kSparseVariants; ++v)
+                if (sparse_variant < 0 || ms[v] < best) { best = ms[v]; sparse_variant = v; }
             std::lock_guard<std::mutex> lock(g_batch_tune_mu);
             g_batch_tune[key] = sparse_variant;
         }

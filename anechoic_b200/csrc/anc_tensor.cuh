@@ -82,7 +82,7 @@ struct PlanesInstance {
 // field_bound: max_y sum_x |J_xy| + max |b|
 bool planes_supported(int n, int maxabs, int64_t field_bound);
 // measured device time of one step of nchains anneals (all waves), in microseconds
-double planes_step_us(int n, int maxabs, int nchains);
+double planes_step_us(int n, int maxabs, int nchains, int sms);
 // anneals one wave advances at most
 int planes_wave_chains(int n, int maxabs);
 // upper bound of a launch's CTAs on this device

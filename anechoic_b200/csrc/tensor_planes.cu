@@ -761,8 +761,8 @@ bool planes_supported(int n, int maxabs, int64_t field_bound) {
            planes_config(rounds_of(n), planes_of(maxabs), 1, 128) != nullptr;
 }
 
-double planes_step_us(int n, int maxabs, int nchains) {
-    const int sms = sm_count(), ngroups = (nchains + kM - 1) / kM;
+double planes_step_us(int n, int maxabs, int nchains, int sms) {
+    const int ngroups = (nchains + kM - 1) / kM;
     const Config* c = planes_config(rounds_of(n), planes_of(maxabs), ngroups, sms);
     return c ? double((ngroups + group_slots(*c, sms) - 1) / group_slots(*c, sms)) * c->us : -1.0;
 }

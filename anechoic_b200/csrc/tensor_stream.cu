@@ -1,7 +1,7 @@
 // Batched engine for large dense instances (NP in (4096, 16384], 17 to 64 rounds): J is too large to keep on chip (16384^2
 // int8 = 256 MB), so every step streams it from HBM or L2 once and applies it to two replica groups at a time.
 //
-// Layout. 128 CTAs, one per y-slice of 2 RP permuted columns, RP = the rounds R padded to 48 or 64. Slice cs owns RNG lanes
+// Layout. 128 CTAs, one per y-slice of 2 RP permuted columns, RP = the rounds R padded to 32, 48 or 64. Slice cs owns RNG lanes
 // 2cs and 2cs + 1, all rounds: slot i = k*256 + l sits at permuted column p(i) = l*RP + k (columns with k >= R are padding,
 // never decided, with zero couplings). J_perm[p(y)][p(x)] = J[x][y] (int8).
 // Per step (the golden model's step, sca_ref_bias.hpp:44-68; decision as in anc_common.cuh):

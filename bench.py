@@ -272,7 +272,7 @@ def numba_baselines(budget_s: float = 6.0):
 
 
 # ------------------------------------------------------------------------------------------------------ our arm
-KERNEL_NAMES = {"plain": "plain_kernel", "tensor-int8": "tensor_res_kernel", "tensor-fp4": "tensor_fp4_kernel"}
+KERNEL_NAMES = {"plain": "plain_kernel", "tensor-int8": "tensor_res_kernel", "tensor-fp4": "tensor_planes_kernel"}
 
 
 def roofline(kernel: str, t_launch_ms: float, B: int, S: int, mean_flips: float, np_pad: int):
@@ -595,7 +595,7 @@ def run_extra(name: str, args, steps: int = 3, warmup: int = 1, target=None) -> 
                 "exact_engine_judgement": judged,
                 "roofline": {"bound": "tensor", "achieved": ach, "peak": bf16_sus, "unit": "TFLOP/s",
                              "frac": ach / bf16_sus, "peak_kind": f"{peak_kind} bf16 sustained",
-                             "algorithmic_per_launch": fl_f, "kernel": "mf_gemm_kernel (+ mf_fwd_kernel)",
+                             "algorithmic_per_launch": fl_f, "kernel": "mf_tmem_kernel",
                              "adjoint_achieved": ach_b, "adjoint_frac": ach_b / bf16_sus,
                              "note": "2 n^2 R FLOPs per forward step; the adjoint counts 2x that (recompute + J p)"}}
     if name == "sparse51":

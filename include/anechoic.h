@@ -126,7 +126,7 @@ typedef struct {
                            force variant v. Cluster engine: 0 = 16 CTAs per anneal when the anneals fit one wave of
                            16-CTA clusters, else 8; 1 = 8 CTAs; 2 = 16 CTAs. CSR instances on the plain engine: the
                            edge format -- 0 = 16-bit edges (two per fetched word) when every weight is +-1 and
-                           n < 32767, else 32-bit; 1 = 32-bit; 2 = 16-bit (EINVAL when not eligible) */
+                           np <= 32736, else 32-bit; 1 = 32-bit; 2 = 16-bit (EINVAL when not eligible) */
 } anc_run_opts;
 
 /* No counterpart in the reference (its kernel geometry is fixed per build by flags, sca_gpu_bias.cu:637-644). The
@@ -174,10 +174,9 @@ ANC_API int anc_auto_choice(anc_instance* inst, anc_tables* tb, int nchains, con
  *   0 wait for fields, 1 TMEM load + decide + update store, 2 n_lin publish, 3 cluster barrier, 4 n_lin read,
  *   5 MMA waiting for TMA, 6 MMA phase (barrier to last commit), 7 TMA waiting for free stages, 8 whole step;
  * out[9] = CTAs, out[10] = CTAs per cluster, out[11] = co-resident clusters, out[12] = MMA issue, out[13] = MMA
- * commits (cycles per step); fp4 kernel, cycles after the CTA's own publish: out[14] first update tile in shared
- * memory, out[15] last update tile, out[16] n_lin tile, out[17] fields-ready commit, out[18] / out[19] flags of
- * update tile 0 / 7 seen, out[20] / out[21] TMA of tile 0 / 7 issued (slot 3 there is the flag publish alone and
- * slot 4 the fields-ready wake-up after the own publish). Returns the count written (<= max). */
+ * commits (cycles per step; streaming and int8 kernels). The planes kernel, which the fp4 kernel is, fills 0 = wait for
+ * fields, 1 = decide, 2 = publish, 3 = draws, 4 = exchange (counters seen and copies issued), 5 = MMA warp waiting, 6 = its
+ * issue, 8 and 9; out[14 ..] are 0. Returns the count written (<= max). */
 ANC_API int anc_last_profile(double* out, int max);
 
 /* Replaces one launch + readback of sca_gpu / sca_gpu_bias (sca_gpu.cu:699-713, sca_gpu_bias.cu:716-733) and
