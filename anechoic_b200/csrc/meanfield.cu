@@ -21,7 +21,7 @@ struct MfContext {
     int n = 0, npad = 0;
     __nv_bfloat16* J = nullptr;       // [npad][npad] (zero padded)
     float* bias = nullptr;            // [npad]
-    float* partial = nullptr;         // [npad / 256][64][npad] split-K partial products (twice in the persistent form)
+    float* partial = nullptr;         // [npad / 256][64][npad] split-K partial products
     float* mring = nullptr;           // forward ring: 3 x [64][npad]
     __nv_bfloat16* xm = nullptr;      // [3][64][npad]: hi / mid / lo of the m operand (twice in the persistent form)
     __nv_bfloat16* xp = nullptr;      // [3][64][npad]: hi / mid / lo of the adjoint operand (likewise)
@@ -359,33 +359,36 @@ __global__ void mf_gsum_kernel(const float* __restrict__ gparts, int S, int nch,
 }
 
 // ---------------------------------------------------------------------------------------------- persistent form
-// The whole forward pass, or the whole adjoint, in one cooperative launch: every CTA keeps its tiles of J on chip and walks
-// through the steps, where the launch sequences below reload J and pay two launches a step. The arithmetic is that of the
-// kernels above, operation for operation and in their order, so the results are bit-identical.
+// The whole forward pass, or the whole adjoint, in one cooperative launch up to 12 chunks of 256 columns: every CTA keeps its
+// tile of J on chip and walks through the steps, where the launch sequences below reload J and pay two launches a step. The
+// arithmetic is that of the kernels above, operation for operation and in their order, so the results are bit-identical.
 //
-// Nine to twelve chunks (mf_steps_kernel): CTA (chunk c, K chunk j) has the two blocks of 128 rows of chunk c by the 256
-// columns of chunk j in shared memory. The nch CTAs of a chunk also share its 64 x 256 elementwise work: unit (replica, c)
-// goes to a quarter of 256 of a CTA's 1024 threads. Two counters per chunk replace the launch boundaries: a_cnt[c], the
-// GEMMs done (the partials of c may be summed), and b_cnt[c], the elementwise steps done (the BF16 terms of c may be
-// multiplied). What a step reads of the other chunks (the soft counts, s_t) was published before the GEMMs whose partials
-// it waited for. Partials and terms are double-buffered: a buffer is written again only after a chain of both waits that
-// covers all of its readers; at the segment ends of the adjoint, where that chain is cut, all CTAs meet (e_cnt).
-// Bound: the chain of a step (counter, terms from L2, 96 MMAs, epilogue, counter, partials, tanh, counter).
-constexpr int kPsThreads = 1024;
-constexpr int kPsChunks = 12;              // at most this many chunks: nch^2 CTAs, one per SM
+// The NR = 64, 32 or 16 replicas of a replica group never meet those of another. Within a group, CTA (MB = 1 or 2 blocks of
+// 128 rows, K chunk j) keeps its first block's tile of J in TMEM, so that an MMA reads only its B tile from shared memory, and
+// a second block's (from nine chunks on, the two blocks of a chunk) in shared memory. The nch CTAs of the same rows are a
+// team: replica k of the group is summed by its member k mod nch, 128 rows to a quarter of its 512 threads. Two kinds of
+// counters replace the launch boundaries: a_cnt[team], the team's GEMMs done (its partials may be summed), and b_cnt[chunk],
+// the elementwise steps of the chunk's teams done (its BF16 terms may be multiplied). The sizes are compile-time constants.
+//
+// A soft count needs the sum over a chunk's two row blocks, which with MB = 1 two teams hold: the warps publish their sums of
+// 32 rows ([replica][chunk][warp of the chunk]) and each reader applies block_sum's tree over them, bit for bit. Those sums and
+// the thread's own values are loaded while the MMAs run.
+// Before its MMAs a CTA has seen every chunk's last elementwise step, so partials, terms and sums of the step before that have
+// all been read: one buffer of partials and two of terms are enough.
+// Bound: the chain of a step, about 11000 cycles at n = 2000: counter 800, terms from L2 1450, MMAs 2200 (the mid and low
+// terms' 32 in one chain, 45 cycles each), epilogue and store 1000, release and counter 2500, partials 1000, tanh, terms and
+// sums 1000, release 1000. 512 threads with up to 128 registers, because 1024 spilled and left each thread one serial chain.
 constexpr int kCntStride = 32;             // counters in lines of their own
-constexpr int kErrA = 13, kErrB = 14, kErrE = 15;
-
-int ps_pad(int nch) { return (nch + 3) / 4 * 4; }
+constexpr int kErrA = 13, kErrB = 14;
 
 struct PsArgs {
-    int n, npad, S;
+    int n, S;
     const float *bias, *beta, *q, *u, *w;
-    float* partial;            // mf_steps: [2][nch][64][nch up to a multiple of 4, zeros][256] (chunk, replica, K chunk, row)
+    float* partial;            // [row block][64][nch][128]
     __nv_bfloat16* xm;         // [2][nch][64][3][256] terms of m: chunk, replica, term, column
     __nv_bfloat16* xp;         // [2][nch][64][3][256] terms of pbar (adjoint)
-    float* nbuf;               // soft counts. mf_steps: [S + 1][64][kPsChunks] per chunk, zero beyond nch
-    unsigned* cnt;             // the counters (zeroed)
+    float* nbuf;               // [S + 1][64][nch][8] soft counts per warp of 32 rows
+    unsigned* cnt;             // per replica group b_cnt[nch], a_cnt[teams] (zeroed)
     int* err;
     uint64_t wait_ns;
     const __nv_bfloat16* J;
@@ -395,8 +398,8 @@ struct PsArgs {
     // adjoint
     const float *ckpt_in, *g_m;
     float *seg_m, *seg_P, *pbar;
-    float* svec;               // s_t, [3] of them laid out like a soft count
-    float* gparts;
+    float* svec;               // [3][64][nch][8] s_t
+    float* gparts;             // [S][3][64][nch][8]
 };
 
 __device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
@@ -415,384 +418,8 @@ __device__ __forceinline__ void ps_ld(uint32_t taddr, uint32_t (&x)[4]) {
                  : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
                  : "r"(taddr));
 }
-__device__ __forceinline__ void ps_ld(uint32_t taddr, uint32_t (&x)[2]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(x[0]), "=r"(x[1]) : "r"(taddr));
-}
 
-// block_sum's tree over the 8 warps of a quarter of the CTA; the result is valid in the quarter's first warp. Calls
-// alternate between two halves of red, so one barrier a call keeps a half's readers and its next writers apart.
-template <int NV>
-__device__ __forceinline__ void unit_sum(float (&v)[NV], float* red, int unit) {
-    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    }
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) red[k * 8 + warp] = v[k];
-    asm volatile("bar.sync %0, 256;" ::"r"(1 + unit) : "memory");
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            float x = lane < 8 ? red[k * 8 + lane] : 0.f;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            v[k] = x;
-        }
-    }
-}
-
-// Sum of up to kPsChunks values in chunk order, past L1 (other CTAs wrote them during this launch). The zeros that pad the
-// chunks to a multiple of 4 change no bit of it.
-__device__ __forceinline__ float sum_parts_cg(const float* parts, int nch) {
-    const float4* p = reinterpret_cast<const float4*>(parts);
-    float4 a = __ldcg(p), b = make_float4(0.f, 0.f, 0.f, 0.f), c = b;
-    if (nch > 4) b = __ldcg(p + 1);
-    if (nch > 8) c = __ldcg(p + 2);
-    float v = (((0.f + a.x) + a.y) + a.z) + a.w;
-    if (nch > 4) v = (((v + b.x) + b.y) + b.z) + b.w;
-    if (nch > 8) v = (((v + c.x) + c.y) + c.z) + c.w;
-    return v;
-}
-
-constexpr size_t ps_smem() { return 1024 + 8 * size_t(kATile) + 12 * size_t(kBTile) + 64; }
-
-template <bool ADJOINT>
-__global__ void __launch_bounds__(kPsThreads, 1) mf_steps_kernel(const __grid_constant__ CUtensorMap mapJ, const __grid_constant__ PsArgs A) {
-    constexpr uint32_t IDESC =
-        (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(kRep >> 3) << 17) | (uint32_t(kRows >> 4) << 24);
-    constexpr int RB = 2, CW = kRep / 8;                        // row blocks; columns per epilogue warp
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    __shared__ float red_s[4][2][24];
-    __shared__ int s_ok;
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sa = smem;                                         // [RB][4] J atoms
-    uint8_t* sb = sa + RB * 4 * kATile;         // [3 terms][4] operand atoms
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sb + 12 * kBTile);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
-    const uint32_t bar_j = smem_u32(bars), bar_done = smem_u32(bars + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, unit = tid >> 8, ut = tid & 255;
-    const int npad = A.npad, nch = npad / kKC, nch4 = (nch + 3) & ~3, n = A.n, S = A.S;
-    const int c = int(blockIdx.x) % nch, j = int(blockIdx.x) / nch;   // own chunk, K chunk
-    const size_t plane = size_t(kRep) * npad;
-    unsigned* const a_cnt = A.cnt + c * kCntStride;
-    unsigned* const b_own = a_cnt + nch * kCntStride;
-    const unsigned* const b_in = A.cnt + (nch + j) * kCntStride;
-    unsigned* const e_cnt = A.cnt + 2 * nch * kCntStride;
-
-    if (tid == 0) {
-        s_ok = 1;
-        mbar_init(bar_j, 1);
-        mbar_init(bar_done, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                     "r"(512)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot, tlane = tmem + (uint32_t((warp & 3) * 32) << 16);
-    if (tid == 0) {
-        mbar_arrive_expect_tx(bar_j, RB * 4 * kATile);
-        for (int rb = 0; rb < RB; ++rb)
-            for (int a = 0; a < 4; ++a)
-                tma_load_2d(smem_u32(sa + (rb * 4 + a) * kATile), &mapJ, j * kKC + 64 * a, (c * RB + rb) * kRows, bar_j);
-        if (!mbar_wait_for(bar_j, 0u, A.err, kErrFull, A.wait_ns)) {
-            mbar_wait_for(bar_j, 0u, nullptr, 0, kWaitNs);
-            s_ok = 0;
-        }
-    }
-    unsigned ng = 0, nb = 0, ne = 0, ns = 0;              // GEMMs, elementwise steps, meetings and sums so far
-    uint32_t done_ph = 0u;
-
-    // Thread 0 waits (bounded) for a counter, everyone behind it; after a wait that gave up the CTA waits for nothing more
-    // and walks on, so that its peers still see every arrival.
-    auto wait_cnt = [&](const unsigned* p, unsigned target, int code) {
-        if (tid == 0 && s_ok) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-            if (v < target) {
-                const uint64_t t0 = globaltimer();
-                for (uint32_t k = 1;; ++k) {
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-                    if (v >= target) break;
-                    if (((k & 63u) == 0 || A.wait_ns == 0) && (globaltimer() - t0 >= A.wait_ns || err_set(A.err))) {
-                        atomicCAS(A.err, 0, code);
-                        s_ok = 0;
-                        break;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    };
-    auto arrive = [&](unsigned* p) {
-        __syncthreads();
-        if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
-    };
-    // This thread's 16-byte pieces of the operand: piece tid % 32 of rows (replicas) tid / 32 + 32 k of each term
-    const uint32_t b_dst = smem_u32(sb) + uint32_t((lane >> 3) * int(kBTile) + warp * 128 + (((lane & 7) ^ (warp & 7)) << 4));
-    const size_t b_src = (size_t(j * kRep + warp) * 3) * kKC + lane * 8;
-    // partial[ng parity][..][j] = J tile x the three terms x[..][chunk j]
-    auto gemm = [&](const __nv_bfloat16* x) {
-        wait_cnt(b_in, nb * unsigned(nch), kErrB);
-        const __nv_bfloat16* src = x + b_src;
-#pragma unroll
-        for (int term = 0; term < 3; ++term) {
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(b_dst + uint32_t(term * 4 * kBTile + k * 32 * 128)),
-                                 "l"(src + (k * 32 * 3 + term) * kKC)
-                                 : "memory");
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-#pragma unroll
-        for (int rb = 0; rb < RB; ++rb) {
-            const uint32_t ut0 = __shfl_sync(0xffffffffu, tmem, 0);
-            const uint64_t da = sw128_desc(smem_u32(sa)) + uint64_t(rb * 4 * (kATile >> 4)), db = sw128_desc(smem_u32(sb));
-            auto mma = [&](uint32_t d, int term, int a, int kk, uint32_t acc) {
-                const uint64_t b = db + uint64_t((term * 4 + a) * (kBTile >> 4) + 2 * kk);
-                mma_f16(d, da + uint64_t(a * (kATile >> 4) + 2 * kk), b, IDESC, acc);
-            };
-            // the leading term's products while the other two terms are on their way
-            if (rb == 0) {
-                asm volatile("cp.async.wait_group 2;" ::: "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncthreads();
-            }
-            if (warp == 0) {
-                tc_fence_after();
-                if (elect_one())
-#pragma unroll
-                    for (int a = 0; a < 4; ++a)
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) mma(ut0 + uint32_t(kRep * a), 0, a, kk, kk != 0 ? 1u : 0u);
-                __syncwarp();
-            }
-            if (rb == 0) {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncthreads();
-            }
-            if (warp == 0) {
-                if (elect_one()) {
-#pragma unroll
-                    for (int a = 0; a < 4; ++a)
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            mma(ut0 + uint32_t(4 * kRep), 1, a, kk, (a | kk) != 0 ? 1u : 0u);
-                            mma(ut0 + uint32_t(4 * kRep), 2, a, kk, 1u);
-                        }
-                    mma_commit(bar_done);
-                }
-                __syncwarp();
-            }
-            if (!mbar_wait_for(bar_done, done_ph & 1u, A.err, kErrDone, A.wait_ns)) {
-                mbar_wait_for(bar_done, done_ph & 1u, nullptr, 0, kWaitNs);
-                s_ok = 0;
-            }
-            ++done_ph;
-            tc_fence_after();
-            // warp w: rows 32 (w % 4) .. of the block, replicas CW (w / 4) ..
-            const uint32_t tl = tlane + uint32_t(CW * (warp >> 2));
-            uint32_t v[5][CW];
-#pragma unroll
-            for (int a = 0; a < 5; ++a) ps_ld(tl + uint32_t(kRep * a), v[a]);
-            tmem_wait_ld();
-            float* dst = A.partial + (size_t(((ng & 1u) * nch + c) * kRep + CW * (warp >> 2)) * nch4 + j) * kKC +
-                         rb * kRows + (warp & 3) * 32 + lane;
-#pragma unroll
-            for (int e = 0; e < CW; ++e) {
-                const float s01 = __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
-                const float s23 = __uint_as_float(v[2][e]) + __uint_as_float(v[3][e]);
-                __stcg(dst + e * (nch4 * kKC), (s01 + s23) + __uint_as_float(v[4][e]));
-            }
-            tc_fence_before();
-            if (rb + 1 < RB) __syncthreads();
-        }
-        ++ng;
-        arrive(a_cnt);
-    };
-    // sum of the split-K partials of the last GEMM for one element, in chunk order (the pads are zeros)
-    auto field = [&](int r) {
-        const float* p = A.partial + size_t((((ng - 1u) & 1u) * nch + c) * kRep + r) * (nch4 * kKC) + ut;
-        float v[kPsChunks], H = 0.f;
-#pragma unroll
-        for (int b = 0; b < kPsChunks; b += 4)
-            if (b < nch)
-#pragma unroll
-                for (int k = b; k < b + 4; ++k) v[k] = __ldcg(p + k * kKC);
-#pragma unroll
-        for (int b = 0; b < kPsChunks; b += 4)
-            if (b < nch)
-#pragma unroll
-                for (int k = b; k < b + 4; ++k) H += v[k];
-        return H;
-    };
-    const int i = c * kKC + ut;                           // this thread's column
-    const float bias = A.bias[i];
-    // the replicas of this quarter of the CTA
-    auto each = [&](auto f) {
-        for (int r = j + nch * unit; r < kRep; r += 4 * nch) f(r);
-    };
-    auto terms = [&](float v, __nv_bfloat16* x, int r) { split_bf16(v, x + size_t(c * kRep + r) * (3 * kKC) + ut, kKC); };
-    auto red = [&]() { return red_s[unit][ns++ & 1u]; };
-    const size_t xbuf = 3 * plane;                        // elements of one of the two buffers of terms
-    // the BF16 terms and the soft count partials of m_t (mf_prep_kernel), from `m`
-    auto prep = [&](const float* m, int t, __nv_bfloat16* x) {
-        each([&](int r) {
-            const float v = m[size_t(r) * npad + i];
-            terms(v, x, r);
-            float acc[1] = {i < n ? 1.f - v * v : 0.f};
-            unit_sum(acc, red(), unit);
-            if (ut == 0) __stcg(A.nbuf + (size_t(t) * kRep + r) * kPsChunks + c, acc[0]);
-        });
-        ++nb;
-        arrive(b_own);
-    };
-    // one forward step t (mf_fwd_kernel): m_{t+1} into m_next, its terms into x, P_t into P_out when that is not null
-    auto forward = [&](int t, const float* m_cur, const float* m_prev, float* m_next, float* also, __nv_bfloat16* x, float* P_out) {
-        const float beta = __ldg(A.beta + t), q = __ldg(A.q + t), u = __ldg(A.u + t), w = __ldg(A.w + t);
-        wait_cnt(a_cnt, ng * unsigned(nch), kErrA);
-        each([&](int r) {
-            const float gamma = u * sum_parts_cg(A.nbuf + (size_t(t) * kRep + r) * kPsChunks, nch) + w;
-            const size_t idx = size_t(r) * npad + i;
-            const float H = field(r);
-            const float P = H + bias + q * m_cur[idx] - gamma * m_prev[idx];
-            const float mn = i < n ? tanhf(beta * P) : 0.f;
-            m_next[idx] = mn;
-            if (also) also[idx] = mn;
-            terms(mn, x, r);
-            if (P_out) P_out[idx] = P;
-            float acc[1] = {i < n ? 1.f - mn * mn : 0.f};
-            unit_sum(acc, red(), unit);
-            if (ut == 0) __stcg(A.nbuf + (size_t(t + 1) * kRep + r) * kPsChunks + c, acc[0]);
-        });
-        ++nb;
-        arrive(b_own);
-    };
-    __syncthreads();
-    tc_fence_after();
-
-    if constexpr (!ADJOINT) {
-        // m_t in ring slot (t + 1) % 3, touched by its owner threads only; checkpoints of (m_{t-1}, m_t) every 16 steps
-        each([&](int r) {
-            const size_t idx = size_t(r) * npad + i;
-            A.ring[idx] = A.mprev[idx];
-            A.ring[plane + idx] = A.m0[idx];
-        });
-        prep(A.m0, 0, A.xm);
-        for (int t = 0; t < S; ++t) {
-            const float *prev = A.ring + size_t(t % 3) * plane, *cur = A.ring + size_t((t + 1) % 3) * plane;
-            if (t % kMfCheckpoint == 0) {
-                float* ck = A.ckpt + size_t(t / kMfCheckpoint) * 2 * plane;
-                each([&](int r) {
-                    const size_t idx = size_t(r) * npad + i;
-                    ck[idx] = prev[idx];
-                    ck[plane + idx] = cur[idx];
-                });
-            }
-            gemm(A.xm + size_t(t & 1) * xbuf);
-            forward(t, cur, prev, A.ring + size_t((t + 2) % 3) * plane, t == S - 1 ? A.m_out : nullptr,
-                    A.xm + size_t((t + 1) & 1) * xbuf, nullptr);
-        }
-    } else {
-        unsigned pbn = 0;                                 // adjoint steps so far: the buffer of their terms
-        for (int seg = (S + kMfCheckpoint - 1) / kMfCheckpoint - 1; seg >= 0; --seg) {
-            const int t0 = seg * kMfCheckpoint, t1 = min(S, t0 + kMfCheckpoint);
-            // seg_m slot k holds m_{t0 - 1 + k}
-            const float* ck = A.ckpt_in + size_t(seg) * 2 * plane;
-            each([&](int r) {
-                const size_t idx = size_t(r) * npad + i;
-                A.seg_m[idx] = ck[idx];
-                A.seg_m[plane + idx] = ck[plane + idx];
-            });
-            prep(ck + plane, t0, A.xm);
-            for (int t = t0; t < t1; ++t) {
-                const int k = t - t0;
-                gemm(A.xm + size_t(k & 1) * xbuf);
-                forward(t, A.seg_m + size_t(k + 1) * plane, A.seg_m + size_t(k) * plane, A.seg_m + size_t(k + 2) * plane, nullptr,
-                        A.xm + size_t((k + 1) & 1) * xbuf, A.seg_P + size_t(k) * plane);
-            }
-            for (int t = t1 - 1; t >= t0; --t) {
-                const int k = t - t0;
-                const bool last = t == S - 1, far = t + 2 < S;
-                // one adjoint step (mf_bwd_kernel)
-                const float beta = __ldg(A.beta + t), q1 = last ? 0.f : __ldg(A.q + t + 1), u1 = last ? 0.f : __ldg(A.u + t + 1);
-                const float u2 = far ? __ldg(A.u + t + 2) : 0.f, w2 = far ? __ldg(A.w + t + 2) : 0.f;
-                if (!last) {
-                    gemm(A.xp + size_t((pbn - 1u) & 1u) * xbuf);
-                    wait_cnt(a_cnt, ng * unsigned(nch), kErrA);
-                }
-                each([&](int r) {
-                    const float us = last ? 0.f : 2.f * u1 * sum_parts_cg(A.svec + (size_t((t + 1) % 3) * kRep + r) * kPsChunks, nch);
-                    const float g2 = far ? u2 * sum_parts_cg(A.nbuf + (size_t(t + 2) * kRep + r) * kPsChunks, nch) + w2 : 0.f;
-                    const float nt = sum_parts_cg(A.nbuf + (size_t(t) * kRep + r) * kPsChunks, nch);
-                    const size_t idx = size_t(r) * npad + i;
-                    const float mn = A.seg_m[size_t(k + 2) * plane + idx];
-                    float G;
-                    if (last) {
-                        G = A.g_m[idx];
-                    } else {
-                        const float H = field(r);
-                        G = H + q1 * A.pbar[size_t((t + 1) % 3) * plane + idx] + us * mn;
-                        if (far) G -= g2 * A.pbar[size_t((t + 2) % 3) * plane + idx];
-                    }
-                    const float abar = i < n ? G * (1.f - mn * mn) : 0.f;
-                    const float pb = beta * abar;
-                    A.pbar[size_t(t % 3) * plane + idx] = pb;
-                    terms(pb, A.xp + size_t(pbn & 1u) * xbuf, r);
-                    float acc[3] = {abar * A.seg_P[size_t(k) * plane + idx], pb * A.seg_m[size_t(k + 1) * plane + idx],
-                                    pb * A.seg_m[size_t(k) * plane + idx]};
-                    unit_sum(acc, red(), unit);
-                    if (ut == 0) {
-                        __stcg(A.svec + (size_t(t % 3) * kRep + r) * kPsChunks + c, acc[2]);
-                        float* g = A.gparts + size_t(t) * 4 * nch * kRep;
-                        g[(0 * nch + c) * kRep + r] = acc[0];
-                        g[(1 * nch + c) * kRep + r] = acc[1];
-                        g[(2 * nch + c) * kRep + r] = -acc[2] * nt;
-                        g[(3 * nch + c) * kRep + r] = -acc[2];
-                    }
-                });
-                ++pbn;
-                ++nb;
-                arrive(b_own);
-            }
-            if (seg > 0) {
-                ++ne;
-                arrive(e_cnt);
-                wait_cnt(e_cnt, ne * gridDim.x, kErrE);
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
-    }
-}
-
-// Up to 8 chunks: as above with these differences. CTA (128 rows of J, K chunk j, replica group of NR) keeps its tile of J in
-// TMEM, so that an MMA reads only its B tile from shared memory. The nch CTAs of a row block and group are a team: replica k
-// of the group is summed by its member k mod nch, 128 rows to a quarter of its 512 threads. a_cnt[team] counts the team's
-// GEMMs, b_cnt[chunk] the elementwise steps of the chunk's two teams. The sizes are compile-time constants.
-//
-// A soft count needs the sum over a chunk's two row blocks, which two teams hold: the warps publish their sums of 32 rows
-// ([replica][chunk][warp of the chunk]) and each reader applies block_sum's tree over them, bit for bit. Those sums and the
-// thread's own values are loaded while the MMAs run.
-// Before its MMAs a CTA has seen every chunk's last elementwise step, so partials, terms and sums of the step before that have
-// all been read: one buffer of partials and two of terms are enough.
-// Bound: the chain of a step, about 11000 cycles at n = 2000: counter 800, terms from L2 1450, MMAs 2200 (the mid and low
-// terms' 32 in one chain, 45 cycles each), epilogue and store 1000, release and counter 2500, partials 1000, tanh, terms and
-// sums 1000, release 1000. 512 threads with up to 128 registers, because 1024 spilled and left each thread one serial chain.
-constexpr int kTmChunks = 8;      // at most
+constexpr int kTmChunks = 12;     // at most: nch^2 CTAs of two row blocks, one per SM
 constexpr int kTmThreads = 512;
 
 // block_sum's tree over the 8 warp sums of a chunk
@@ -803,44 +430,49 @@ __device__ __forceinline__ float warps_tree(const float* parts) {
 
 template <int NCH>
 struct TmSplit {
+    static constexpr int mb = NCH <= 8 ? 1 : 2;                             // row blocks per CTA
     // replicas per group: as few as one CTA per SM allows
     static constexpr int nr = NCH <= 4 ? 16 : NCH <= 6 ? 32 : 64;
     static constexpr int rp = (nr + NCH - 1) / NCH;                         // replicas that a CTA sums, at most
-    static constexpr int grid = 2 * NCH * NCH * (kRep / nr);
+    static constexpr int grid = 2 / mb * NCH * NCH * (kRep / nr);
     // more than half of an SM's shared memory: each CTA allocates all of its SM's TMEM
-    static constexpr size_t smem = 120 * 1024;
-    static_assert(1024 + 12 * nr * 128 + 64 <= smem, "operand atoms");
+    static constexpr size_t need = 1024 + (mb - 1) * 4 * size_t(kATile) + 12 * size_t(nr) * 128 + 64;
+    static constexpr size_t smem = need > 120 * 1024 ? need : 120 * 1024;
 };
 
 template <int NCH, bool ADJOINT>
-__global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_constant__ CUtensorMap, const __grid_constant__ PsArgs A) {
+__global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_constant__ CUtensorMap mapJ, const __grid_constant__ PsArgs A) {
     using Split = TmSplit<NCH>;
-    constexpr int NR = Split::nr, rp = Split::rp, nch = NCH, npad = NCH * kKC;
+    constexpr int MB = Split::mb, NR = Split::nr, rp = Split::rp, nch = NCH, npad = NCH * kKC;
     constexpr uint32_t IDESC =
         (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(NR >> 3) << 17) | (uint32_t(kRows >> 4) << 24);
     constexpr int BT = NR * 128, CW = NR / 4;                   // bytes of a B atom; columns per epilogue warp
     constexpr uint32_t kACol = 320;                             // TMEM columns: 5 x NR accumulators, J from 320
-    constexpr int P = (rp + 3) / 4;                             // replicas per quarter of the CTA
+    constexpr int UK = 4 / MB, P = (rp + UK - 1) / UK;          // quarters per 128 rows; replicas per quarter
+    constexpr int GL = NCH <= 8 ? 8 : 16;                       // lanes per array in sums()
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ int s_ok;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, unit = tid >> 7, ut = tid & 127;
     const int n = A.n, S = A.S;
-    const int j = int(blockIdx.x) % NCH, rowi = int(blockIdx.x) / NCH % (2 * NCH), rg = int(blockIdx.x) / NCH / (2 * NCH);
-    const int c = rowi >> 1;                                    // own chunk
+    const int j = int(blockIdx.x) % NCH, team = int(blockIdx.x) / NCH % (2 / MB * NCH), rg = int(blockIdx.x) / NCH / (2 / MB * NCH);
+    const int c = MB == 1 ? team >> 1 : team;                   // own chunk
+    const int half = MB == 1 ? team & 1 : unit & 1;             // of the chunk's rows: this quarter's
+    const int row0 = MB == 1 ? team : 2 * team;                 // the CTA's first row block
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sb = smem;                                         // [3 terms][4] operand atoms
+    uint8_t* sa = smem;                                         // [4] J atoms of a second row block
+    uint8_t* sb = sa + (MB - 1) * 4 * kATile;                   // [3 terms][4] operand atoms
     uint64_t* bars = reinterpret_cast<uint64_t*>(sb + 12 * BT);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 1);
-    const uint32_t bar_done = smem_u32(bars);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
+    const uint32_t bar_done = smem_u32(bars), bar_j = smem_u32(bars + 1);
     constexpr size_t plane = size_t(kRep) * npad;
-    // per replica group: b_cnt[nch], a_cnt[2 nch]
-    unsigned* const b_cnt = A.cnt + rg * 3 * NCH * kCntStride;
-    unsigned* const a_cnt = b_cnt + (NCH + rowi) * kCntStride;
-    constexpr unsigned team = unsigned(2 * NCH);
+    unsigned* const b_cnt = A.cnt + rg * 3 * NCH * kCntStride;  // per replica group: b_cnt[nch], a_cnt[up to 2 nch]
+    unsigned* const a_cnt = b_cnt + (NCH + team) * kCntStride;
+    constexpr unsigned b_all = unsigned(2 / MB * NCH);          // arrivals per step at a b_cnt
 
     if (tid == 0) {
         s_ok = 1;
         mbar_init(bar_done, 2);
+        mbar_init(bar_j, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -855,7 +487,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
     const uint32_t tmem = *tslot, tlane = tmem + (uint32_t((warp & 3) * 32) << 16);
     {
         // warp w: rows 32 (w % 4) .., BF16 columns 64 (w / 4) .. of the tile, two to a TMEM column
-        const uint4* src = reinterpret_cast<const uint4*>(A.J + size_t(rowi * kRows + (warp & 3) * 32 + lane) * npad + j * kKC +
+        const uint4* src = reinterpret_cast<const uint4*>(A.J + size_t(row0 * kRows + (warp & 3) * 32 + lane) * npad + j * kKC +
                                                           64 * (warp >> 2));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -872,6 +504,14 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
         }
         tmem_wait_st();
         tc_fence_before();
+    }
+    if (MB == 2 && tid == 0) {
+        mbar_arrive_expect_tx(bar_j, 4 * kATile);
+        for (int a = 0; a < 4; ++a) tma_load_2d(smem_u32(sa + a * kATile), &mapJ, j * kKC + 64 * a, (row0 + 1) * kRows, bar_j);
+        if (!mbar_wait_for(bar_j, 0u, A.err, kErrFull, A.wait_ns)) {
+            mbar_wait_for(bar_j, 0u, nullptr, 0, kWaitNs);
+            s_ok = 0;
+        }
     }
     unsigned ng = 0, nb = 0;                              // GEMMs and elementwise steps so far
     uint32_t done_ph = 0u;
@@ -903,11 +543,11 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
     const uint32_t b_dst = smem_u32(sb) + uint32_t((lane >> 3) * BT + warp * 128 + (((lane & 7) ^ (warp & 7)) << 4));
     const size_t b_src = (size_t(j * kRep + rg * NR + warp) * 3) * kKC + lane * 8;
     // partials are [row block][replica][K chunk][128 rows]: where this thread's accumulator columns go, and the sums' first
-    float* const part_out = A.partial + (size_t(rowi * kRep + rg * NR + CW * (warp >> 2)) * NCH + j) * kRows + (warp & 3) * 32 + lane;
-    const float* const part_in = A.partial + size_t(rowi * kRep) * (NCH * kRows) + ut;
+    float* const part_out = A.partial + (size_t(row0 * kRep + rg * NR + CW * (warp >> 2)) * NCH + j) * kRows + (warp & 3) * 32 + lane;
+    const float* const part_in = A.partial + size_t((2 * c + half) * kRep) * (NCH * kRows) + ut;
     // partials of J tile x the three terms x[..][chunk j], of the whole team when it returns; `ahead` runs while the MMAs do
     auto gemm = [&](const __nv_bfloat16* x, auto ahead) {
-        if (tid == 0) poll(b_cnt + j * kCntStride, nb * team, kErrB);
+        if (tid == 0) poll(b_cnt + j * kCntStride, nb * b_all, kErrB);
         __syncthreads();
         const __nv_bfloat16* src = x + b_src;
 #pragma unroll
@@ -920,66 +560,81 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         // every chunk's step, for the sums that `ahead` reads
-        if (warp == 15 && lane < nch) poll(b_cnt + lane * kCntStride, nb * team, kErrB);
+        if (warp == 15 && lane < nch) poll(b_cnt + lane * kCntStride, nb * b_all, kErrB);
         const uint32_t ut0 = __shfl_sync(0xffffffffu, tmem, 0);
-        const uint64_t db = sw128_desc(smem_u32(sb));
-        auto mma = [&](uint32_t d, int term, int a, int kk, uint32_t acc) {
-            mma_f16_ta(ut0 + d, ut0 + kACol + uint32_t(8 * (4 * a + kk)), db + uint64_t((term * 4 + a) * (BT >> 4) + 2 * kk), IDESC, acc);
+        const uint64_t da = sw128_desc(smem_u32(sa)), db = sw128_desc(smem_u32(sb));
+        auto mma = [&](int mb, uint32_t d, int term, int a, int kk, uint32_t acc) {
+            const uint64_t b = db + uint64_t((term * 4 + a) * (BT >> 4) + 2 * kk);
+            if (mb == 0)
+                mma_f16_ta(ut0 + d, ut0 + kACol + uint32_t(8 * (4 * a + kk)), b, IDESC, acc);
+            else
+                mma_f16(ut0 + d, da + uint64_t(a * (kATile >> 4) + 2 * kk), b, IDESC, acc);
+        };
+        auto leading = [&](int mb) {
+            if (elect_one()) {
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) mma(mb, uint32_t(NR * a), 0, a, kk, kk != 0 ? 1u : 0u);
+                mma_commit(bar_done);
+            }
+            __syncwarp();
+        };
+        auto others = [&](int mb) {
+            if (elect_one()) {
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) {
+                        mma(mb, uint32_t(4 * NR), 1, a, kk, (a | kk) != 0 ? 1u : 0u);
+                        mma(mb, uint32_t(4 * NR), 2, a, kk, 1u);
+                    }
+                mma_commit(bar_done);
+            }
+            __syncwarp();
         };
         // the leading term's products while the other two terms are on their way; one warp issues them, another the others
         asm volatile("cp.async.wait_group 2;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         tc_fence_after();
-        if (warp == 0) {
-            if (elect_one()) {
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) mma(uint32_t(NR * a), 0, a, kk, kk != 0 ? 1u : 0u);
-                mma_commit(bar_done);
-            }
-            __syncwarp();
-        }
+        if (warp == 0) leading(0);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (warp == 1) {
-            if (elect_one()) {
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        mma(uint32_t(4 * NR), 1, a, kk, (a | kk) != 0 ? 1u : 0u);
-                        mma(uint32_t(4 * NR), 2, a, kk, 1u);
-                    }
-                mma_commit(bar_done);
-            }
-            __syncwarp();
-        }
+        if (warp == 1) others(0);
         ahead();
-        if (!mbar_wait_for(bar_done, done_ph & 1u, A.err, kErrDone, A.wait_ns)) {
-            mbar_wait_for(bar_done, done_ph & 1u, nullptr, 0, kWaitNs);
-            s_ok = 0;
-        }
-        ++done_ph;
-        tc_fence_after();
-        const uint32_t tl = tlane + uint32_t(CW * (warp >> 2));
-        constexpr int EW = CW < 8 ? CW : 8;
 #pragma unroll
-        for (int h = 0; h < CW / EW; ++h) {
-            uint32_t v[5][EW];
-#pragma unroll
-            for (int a = 0; a < 5; ++a) ps_ld(tl + uint32_t(NR * a + EW * h), v[a]);
-            tmem_wait_ld();
-#pragma unroll
-            for (int e = 0; e < EW; ++e) {
-                const float s01 = __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
-                const float s23 = __uint_as_float(v[2][e]) + __uint_as_float(v[3][e]);
-                __stcg(part_out + (EW * h + e) * (NCH * kRows), (s01 + s23) + __uint_as_float(v[4][e]));
+        for (int mb = 0; mb < MB; ++mb) {
+            if (mb) {
+                __syncthreads();                          // the accumulators of the first block have been read
+                tc_fence_after();
+                if (warp == 0) leading(1);
+                if (warp == 1) others(1);
             }
+            if (!mbar_wait_for(bar_done, done_ph & 1u, A.err, kErrDone, A.wait_ns)) {
+                mbar_wait_for(bar_done, done_ph & 1u, nullptr, 0, kWaitNs);
+                s_ok = 0;
+            }
+            ++done_ph;
+            tc_fence_after();
+            const uint32_t tl = tlane + uint32_t(CW * (warp >> 2));
+            constexpr int EW = CW < 8 ? CW : 8;
+#pragma unroll
+            for (int h = 0; h < CW / EW; ++h) {
+                uint32_t v[5][EW];
+#pragma unroll
+                for (int a = 0; a < 5; ++a) ps_ld(tl + uint32_t(NR * a + EW * h), v[a]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < EW; ++e) {
+                    const float s01 = __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
+                    const float s23 = __uint_as_float(v[2][e]) + __uint_as_float(v[3][e]);
+                    __stcg(part_out + (mb * kRep + EW * h + e) * (NCH * kRows), (s01 + s23) + __uint_as_float(v[4][e]));
+                }
+            }
+            tc_fence_before();
         }
-        tc_fence_before();
         ++ng;
         arrive(a_cnt);
         if (tid == 0) poll(a_cnt, ng * unsigned(NCH), kErrA);
@@ -999,7 +654,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
             for (int ks = 0; ks < NCH; ++ks) H[h] += v[h][ks];
         }
     };
-    const int i = rowi * kRows + ut;                      // this thread's column of m
+    const int i = c * kKC + half * kRows + ut;                      // this thread's column of m
     const bool in = i < n;
     const float bias = A.bias[i];
     // This thread's replicas. Where the last of them is none (on[P - 1] false) it repeats the first, to be computed and not
@@ -1008,15 +663,15 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
     bool on[P];
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-        const int k = unit + 4 * p;
+        const int k = unit / MB + UK * p;
         on[p] = k < rp && k * NCH + j < NR;
-        r[p] = rg * NR + (on[p] ? k : unit) * NCH + j;
+        r[p] = rg * NR + (on[p] ? k : unit / MB) * NCH + j;
     }
     auto terms = [&](float v, __nv_bfloat16* x, int r) {
-        split_bf16(v, x + (c * kRep + r) * (3 * kKC) + (rowi & 1) * kRows + ut, kKC);
+        split_bf16(v, x + (c * kRep + r) * (3 * kKC) + half * kRows + ut, kKC);
     };
     // a replica's raw sums are [chunk][warp of the chunk]
-    const int wslot = c * 8 + (rowi & 1) * 4 + (warp & 3);
+    const int wslot = c * 8 + half * 4 + (warp & 3);
     auto put = [&](float* base, float (&v)[P]) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -1026,9 +681,9 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
         for (int h = 0; h < P; ++h)
             if (lane == 0 && on[h]) __stcg(base + r[h] * (8 * NCH) + wslot, v[h]);
     };
-    // sums over the chunks, in chunk order, of up to four arrays at once: lanes 8 g .. hold the chunks of array g
+    // sums over the chunks, in chunk order, of the arrays that each GL lanes are given
     auto sums = [&](const float* mine, float (&v)[P]) {
-        const int ch0 = min(lane & 7, NCH - 1);
+        const int ch0 = min(lane & (GL - 1), NCH - 1);
         float tree[P];
 #pragma unroll
         for (int h = 0; h < P; ++h) {
@@ -1038,7 +693,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
 #pragma unroll
         for (int ch = 0; ch < NCH; ++ch)
 #pragma unroll
-            for (int h = 0; h < P; ++h) v[h] += __shfl_sync(0xffffffffu, tree[h], (lane & 24) + ch);
+            for (int h = 0; h < P; ++h) v[h] += __shfl_sync(0xffffffffu, tree[h], (lane & ~(GL - 1)) + ch);
     };
     constexpr size_t xbuf = 3 * plane, sstep = size_t(kRep) * 8 * NCH;
     // the BF16 terms and the soft count sums of m_t (mf_prep_kernel), from `m`
@@ -1155,12 +810,12 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
                             p2[h] = far ? A.pbar[size_t((t + 2) % 3) * plane + idx] : 0.f;
                         }
                         float v[P];
-                        // lanes 0 .. 7: s_{t+1}, the others: n_{t+2}; at the last steps other values, which are not used
-                        sums(lane < 8 ? A.svec + size_t((t + 1) % 3) * sstep : A.nbuf + size_t(far ? t + 2 : t) * sstep, v);
+                        // lanes 0 .. GL - 1: s_{t+1}, the others: n_{t+2}; at the last steps other values, which are not used
+                        sums(lane < GL ? A.svec + size_t((t + 1) % 3) * sstep : A.nbuf + size_t(far ? t + 2 : t) * sstep, v);
 #pragma unroll
                         for (int h = 0; h < P; ++h) {
                             s1[h] = __shfl_sync(0xffffffffu, v[h], 0);
-                            n2[h] = __shfl_sync(0xffffffffu, v[h], 8);
+                            n2[h] = __shfl_sync(0xffffffffu, v[h], GL);
                         }
                     }
                 };
@@ -1205,7 +860,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
             }
             if (t1 - t0 == 1 && seg > 0) {
                 // a last segment of one step had no GEMM behind its forward step: its terms may still be read
-                if (tid < NCH) poll(b_cnt + tid * kCntStride, nb * team, kErrB);
+                if (tid < NCH) poll(b_cnt + tid * kCntStride, nb * b_all, kErrB);
                 __syncthreads();
             }
         }
@@ -1218,26 +873,30 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
     }
 }
 
-// The schedule gradients from mf_tmem_kernel's raw sums, one warp per (step, replica): lanes 0 .. 7 hold the chunks of
-// sum abar P, 8 .. of sum pbar m_t, 16 .. of s_t, 24 .. of n_t; the same sums as mf_bwd_kernel's and mf_gsum_kernel's.
+// The schedule gradients from mf_tmem_kernel's warp sums, one warp per (step, replica): the halves of the warp hold the chunks
+// of s_t and n_t, then those of sum abar P and sum pbar m_t; the same sums as mf_bwd_kernel's and mf_gsum_kernel's.
 __global__ void mf_gsum_raw_kernel(const float* __restrict__ gparts, const float* __restrict__ nbuf, int S, int nch, float* __restrict__ gsched) {
-    const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, hi = lane >> 4;
     if (e >= S * kRep) return;
-    const int r = e % kRep, t = e / kRep, kind = lane >> 3;
-    const size_t sstep = size_t(kRep) * 8 * nch;
-    const float* src = (kind == 3 ? nbuf + size_t(t) * sstep : gparts + (size_t(t) * 3 + kind) * sstep) + r * (8 * nch);
-    const float tree = (lane & 7) < nch ? warps_tree(src + (lane & 7) * 8) : 0.f;
-    float v = 0.f;
-    for (int ch = 0; ch < nch; ++ch) v += __shfl_sync(0xffffffffu, tree, (lane & 24) + ch);
-    const float nt = __shfl_sync(0xffffffffu, v, 24);
-    float g2 = 0.f, g3 = 0.f;
+    const int r = e % kRep, t = e / kRep, ch0 = min(lane & 15, nch - 1);
+    const size_t sstep = size_t(kRep) * 8 * nch, at = size_t(r * nch + ch0) * 8;
+    const float tree = warps_tree((hi ? nbuf + size_t(t) * sstep : gparts + (size_t(t) * 3 + 2) * sstep) + at);
+    const float prod = warps_tree(gparts + (size_t(t) * 3 + hi) * sstep + at);
+    float n = 0.f, v = 0.f, g2 = 0.f, g3 = 0.f;
     for (int ch = 0; ch < nch; ++ch) {
-        const float s = __shfl_sync(0xffffffffu, tree, 16 + ch);
-        g2 = __fadd_rn(g2, __fmul_rn(-s, nt));
+        n += __shfl_sync(0xffffffffu, tree, 16 + ch);
+        v += __shfl_sync(0xffffffffu, prod, (lane & 16) + ch);
+    }
+    for (int ch = 0; ch < nch; ++ch) {
+        const float s = __shfl_sync(0xffffffffu, tree, ch);
+        g2 = __fadd_rn(g2, __fmul_rn(-s, n));
         g3 += -s;
     }
-    const float out = kind == 2 ? g2 : (kind == 3 ? g3 : v);
-    if ((lane & 7) == 0) gsched[(size_t(t) * 4 + kind) * kRep + r] = out;
+    float* const out = gsched + size_t(t) * 4 * kRep + r;
+    if ((lane & 15) == 0) {
+        out[hi * kRep] = v;
+        out[(2 + hi) * kRep] = hi ? g3 : g2;
+    }
 }
 
 bool check(cudaError_t e, const char* what, std::string* why) {
@@ -1312,35 +971,27 @@ int run_steps(MfContext* c, int t0, int t1, const float* beta, const float* q, c
 
 using PsKernel = void (*)(const CUtensorMap, const PsArgs);
 struct PsForm {
-    int grid, threads;
-    bool raw;                  // the sums are kept per warp (mf_gsum_raw_kernel)
+    int grid;
     size_t smem;
     PsKernel fwd, adj;
-    int row;                   // floats per step and replica of the soft counts and of s_t
-    int grows;                 // and of the schedule gradient's sums
 };
 template <int NCH>
 constexpr PsForm tm_form() {
-    using Split = TmSplit<NCH>;
-    return {Split::grid, kTmThreads, true, Split::smem, mf_tmem_kernel<NCH, false>, mf_tmem_kernel<NCH, true>, 8 * NCH,
-            24 * NCH};
+    return {TmSplit<NCH>::grid, TmSplit<NCH>::smem, mf_tmem_kernel<NCH, false>, mf_tmem_kernel<NCH, true>};
 }
-constexpr PsForm ps_blocks(int nch) {
-    return {nch * nch, kPsThreads, false, ps_smem(), mf_steps_kernel<false>, mf_steps_kernel<true>, kPsChunks, 4 * nch};
-}
-const PsForm kPsForms[kPsChunks] = {tm_form<1>(), tm_form<2>(), tm_form<3>(), tm_form<4>(),  tm_form<5>(),  tm_form<6>(),
-                                    tm_form<7>(), tm_form<8>(), ps_blocks(9), ps_blocks(10), ps_blocks(11), ps_blocks(12)};
+const PsForm kPsForms[kTmChunks] = {tm_form<1>(), tm_form<2>(), tm_form<3>(), tm_form<4>(),  tm_form<5>(),  tm_form<6>(),
+                                    tm_form<7>(), tm_form<8>(), tm_form<9>(), tm_form<10>(), tm_form<11>(), tm_form<12>()};
 
 size_t ps_cnt_bytes(int nch) { return size_t(12 * nch + 1) * kCntStride * sizeof(unsigned); }
 
 // The persistent form for npad columns, or null (the launch sequences) beyond twelve chunks or where its CTAs do not all fit,
-// one per SM. Measured, a forward / an adjoint step in us, launch sequences -> persistent: n = 200 8.2 / 15.3 -> 5.9 / 11.1,
-// n = 700 10.0 / 18.6 -> 5.9 / 10.5, n = 2000 9.3 / 19.4 -> 6.0 / 12.4, n = 2500 15.7 / 30.9 -> 12.4 / 27.9, n = 3072
-// 16.9 / 32.7 -> 13.0 / 28.2. J of more chunks does not fit the SMs.
+// one per SM. Measured, a forward / an adjoint step in us, launch sequences -> persistent: n = 200 8.4 / 15.2 -> 5.8 / 11.2,
+// n = 700 10.0 / 18.7 -> 5.8 / 10.4, n = 2000 9.3 / 19.4 -> 6.0 / 12.4, n = 2500 15.8 / 30.9 -> 10.8 / 20.9, n = 3072
+// 16.8 / 32.7 -> 10.6 / 20.4. J of more chunks does not fit the SMs.
 const PsForm* ps_form(int npad) {
     const int nch = npad / kKC;
     int dev = 0, sms = 0, coop = 0;
-    if (nch > kPsChunks || cudaGetDevice(&dev) != cudaSuccess ||
+    if (nch > kTmChunks || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
         return nullptr;
@@ -1349,7 +1000,7 @@ const PsForm* ps_form(int npad) {
         const void* k = reinterpret_cast<const void*>(kernel);
         int per_sm = 0;
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(f.smem)) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, f.threads, f.smem) != cudaSuccess || per_sm < 1 ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kTmThreads, f.smem) != cudaSuccess || per_sm < 1 ||
             f.grid > sms) {
             cudaGetLastError();
             return nullptr;
@@ -1361,7 +1012,6 @@ const PsForm* ps_form(int npad) {
 PsArgs ps_args(MfContext* c, int S, const float* beta, const float* q, const float* u, const float* w) {
     PsArgs a{};
     a.n = c->n;
-    a.npad = c->npad;
     a.S = S;
     a.J = c->J;
     a.bias = c->bias;
@@ -1386,8 +1036,8 @@ int ensure_steps(MfContext* c, int S, std::string* why) {
         *p = nullptr;
     }
     c->nbuf_steps = 0;
-    const size_t nbytes = size_t(S + 1) * (c->form ? c->form->row : nch(c)) * kRep * sizeof(float);
-    const size_t gbytes = size_t(S) * (c->form ? c->form->grows : 4 * nch(c)) * kRep * sizeof(float);
+    const size_t nbytes = size_t(S + 1) * (c->form ? 8 : 1) * nch(c) * kRep * sizeof(float);
+    const size_t gbytes = size_t(S) * (c->form ? 24 : 4) * nch(c) * kRep * sizeof(float);
     if (!check(cudaMalloc(&c->nbuf, nbytes), "cudaMalloc", why) || !check(cudaMemset(c->nbuf, 0, nbytes), "cudaMemset", why) ||
         !check(cudaStreamSynchronize(nullptr), "cudaMemset", why) ||
         !check(cudaMalloc(&c->gparts, gbytes), "cudaMalloc", why))
@@ -1399,7 +1049,7 @@ int ensure_steps(MfContext* c, int S, std::string* why) {
 int ps_launch(MfContext* c, PsKernel kernel, PsArgs& a, cudaStream_t st, std::string* why) {
     void* args[] = {&c->mapJ, &a};
     if (!check(cudaMemsetAsync(c->cnt, 0, ps_cnt_bytes(nch(c)), st), "clear counters", why) ||
-        !check(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(c->form->grid), dim3(c->form->threads),
+        !check(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(c->form->grid), dim3(kTmThreads),
                                            args, c->form->smem, st),
                "mean-field steps launch", why))
         return -2;
@@ -1434,8 +1084,8 @@ int mf_create(const int8_t* J, const int32_t* bias, int n, MfContext** out, std:
     const size_t plane = size_t(kRep) * npad;
     c->form = ps_form(npad);
     const size_t nbuf = c->form ? 2 : 1, kch = npad / kKC;
-    const size_t pbytes = (!c->form ? kch : c->form->raw ? kch : 2 * size_t(ps_pad(kch))) * plane * sizeof(float);
-    const size_t sbytes = 3 * (c->form ? size_t(c->form->row) : kch) * kRep * sizeof(float);
+    const size_t pbytes = kch * plane * sizeof(float);
+    const size_t sbytes = 3 * (c->form ? 8 : 1) * kch * kRep * sizeof(float);
     bool ok = check(cudaMalloc(&c->J, Jh.size() * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
               check(cudaMemcpy(c->J, Jh.data(), Jh.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice), "upload J",
                     why) &&
@@ -1692,11 +1342,7 @@ int mf_backward(MfContext* c, int S, const float* beta, const float* q, const fl
         a.gparts = c->gparts;
         rc = ps_launch(c, c->form->adj, a, st, why);
         if (rc) return rc;
-        const int ne = S * 4 * kRep;
-        if (c->form->raw)
-            mf_gsum_raw_kernel<<<(S * kRep + 7) / 8, 256, 0, st>>>(c->gparts, c->nbuf, S, nch(c), gsched);
-        else
-            mf_gsum_kernel<<<(ne + 255) / 256, 256, 0, st>>>(c->gparts, S, nch(c), gsched);
+        mf_gsum_raw_kernel<<<(S * kRep + 7) / 8, 256, 0, st>>>(c->gparts, c->nbuf, S, nch(c), gsched);
         return check(cudaGetLastError(), "mean-field gradient sum", why) ? 0 : -2;
     }
     int rc = ensure_io(c, S, why);

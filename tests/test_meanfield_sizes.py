@@ -19,7 +19,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,S", [(256, 17), (257, 33), (700, 18), (1000, 16), (1281, 1), (1500, 33), (1600, 5), (2048, 18),
-                                 (2049, 17), (3072, 2), (3073, 17)])
+                                 (2049, 17), (2800, 33), (3072, 2), (3073, 17)])
 def test_forms_vs_fp64(cuda, n, S):
     inst = I.random_kbit(n, 2, 900 + n, pzero=0.4, bmax=3)
     theta = (4.0 * math.sqrt(n), math.log(2.0), 1.0, 0.5, 1.05)
