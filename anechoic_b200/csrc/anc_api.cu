@@ -724,7 +724,7 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
 
 // Run-time tuner of the CSR pass (the plain engine on sparse instances): on the first synchronous run of an
 // instance, each compiled variant (kSparseVariantShape: rows in flight per lane group x edges per lane) runs the
-// first min(S, 64) steps of min(nchains, one wave) anneals of that run -- twice, the second launch timed with CUDA
+// first min(S, 64) steps of min(nchains, one wave) anneals of that run -- after an untimed launch of 8 steps, timed with CUDA
 // events -- and the fastest is kept for every later launch of the instance (device, batch and graph-captured
 // launches included). Every variant computes the same fields; only the time differs. The probes write into the
 // handle's own workspaces, never into the caller's outputs.
@@ -1650,7 +1650,7 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
         return rc ? cuda_fail(cudaError_t(rc), "plain engine launch") : ANC_OK;
     };
     // the CSR pass variant of the sparse launch: forced by the options, else tuned on this batch as a whole (each
-    // variant runs the first min(S, 64) steps of every sparse job, twice, the second timed) and kept for batches of
+    // variant runs the first min(S, 64) steps of every sparse job, after an untimed launch of 8) and kept for batches of
     // the same instances and anneal counts
     int sparse_variant = (o && o->sparse_variant > 0) ? o->sparse_variant - 1 : -1;
     if (nitems[0] > 0 && sparse_variant < 0) {

@@ -133,7 +133,7 @@ typedef struct {
  * run-time tuner of the plain engine's CSR pass: on an instance's first synchronous run (anc_run / anc_run_fields /
  * anc_run_batch) each compiled variant -- lane groups x edges fetched per lane before any is applied: {1, 8},
  * {1, 4}, {2, 4}, {1, 16} -- runs the first min(S, 64) steps of up to one wave of that run's anneals into the handle's
- * own workspaces (twice; the second launch is timed), and the fastest is used for every later launch of the
+ * own workspaces (after an untimed launch of 8 steps), and the fastest is used for every later launch of the
  * instance. Writes the chosen variant (-1 = not tuned yet, or not a CSR instance) and probe_us[4], each variant's
  * probe time per step in microseconds (may be NULL). */
 ANC_API int anc_sparse_tuning(const anc_instance* inst, int* variant, double* probe_us);
