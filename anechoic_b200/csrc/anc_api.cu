@@ -739,7 +739,10 @@ int tune_sparse(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
     int per_sm = 0;
     rc = plain_residency(I, P, &smem, &stream, &per_sm);
     if (rc) return rc;
-    const int np = std::max(1, std::min(nchains, per_sm * I->sms));
+    int np = std::max(1, std::min(nchains, per_sm * I->sms));
+    // a run in groups is probed in groups
+    if (I->slices && anc::sparse_groups(I->np, row_degree(I), nchains, I->sms))
+        np = std::min(nchains, std::max(np, anc::kGroupReplicas * I->sms));
     const int Sp = std::min(tb->S, 64);
     CK(I->w_spins.ensure(size_t(I->nw) * np));
     CK(I->w_sh.ensure(np));
