@@ -146,9 +146,14 @@ int pad_np(int n) { return std::max(2048, ((n + 255) / 256) * 256); }
 //            streaming 99.5 (measured 99.5 at NP = 10240 and 98 at NP = 16384: bound by its step latency, not by
 //            reading J)
 // Each engine advances a fixed number of anneals at once (per_wave); a launch of more takes further waves.
-// Least step AUTO assumes for the fp4 kernel (3.5 - 4.6 us measured up to four replica groups): a 1-bit batch that flips
-// few spins (the temperature-scaled schedules, phi about 0.11) stays on the plain engine, whose estimate is 5.9 us there.
-constexpr double kFp4FloorUs = 5.95;
+// The fp4 kernel's step is taken as at least kFp4FloorUs unless its own (planes_step_us) saves more than the set-up of its
+// operands where that is still to be done. +-1, phi 0.33, us a step plain / cluster / fp4: n = 500 4.3 / 4.9 / 3.8 for 60 anneals
+// and 4.3 / 8.5 / 4.2 for 100; n = 1100 6.6 / 4.9 / 3.8 and 6.6 / 8.5 / 4.3; n = 2000 10.3 / 4.9 / 3.9 and 10.3 / 8.5 / 4.3; up to
+// 30 anneals the cluster engine has 2.5. Batches that flip few spins (the temperature-scaled schedules, phi about 0.11 at
+// n = 2000) stay on the plain engine where its estimate is the least of the others (5.86 us there): the floor holds below
+// kFewFlips.
+constexpr double kFp4FloorUs = 5.95, kFewFlips = 0.15;
+constexpr double kPlanesSetupUs = 400.0;   // packing, workspaces and their first touch: 0.3 - 0.5 ms on an instance's first call
 constexpr double kPhiPrior = 0.25;   // flip fraction assumed before any run of these tables on this instance
 
 double plain_step_us(int n, int K, double phi) {
@@ -568,10 +573,13 @@ int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts
     int best = estimate_engines(I->n, I->K, nchains, tb->S, phi, fp4_candidate(I), engine_waves(I), est);
     const bool free_choice = !o || (o->tensor_kind == ANC_TENSOR_AUTO && o->kernel_variant == 0 && !o->profile);
     if ((free_choice || o->tensor_kind == ANC_TENSOR_PLANES) && planes_candidate(I)) {
-        // where the fp4 kernel runs, it is the planes kernel by another name: only its estimate changes, and not below
-        // kFp4Floor
+        // where the fp4 kernel runs, it is the planes kernel by another name: only its estimate changes
         const bool fp4 = fp4_candidate(I) && (!o || o->tensor_kind != ANC_TENSOR_PLANES);
-        const double t = tb->S * std::max(fp4 ? kFp4FloorUs : 0.0, anc::planes_step_us(I->n, I->info.maxabs, nchains, I->sms));
+        const double step = anc::planes_step_us(I->n, I->info.maxabs, nchains, I->sms);
+        double t = tb->S * std::max(fp4 ? kFp4FloorUs : 0.0, step);
+        const bool held = best == ANC_ENGINE_PLAIN && phi < kFewFlips;
+        if (fp4 && !held && est[best] >= 0 && tb->S * step + (I->planes4_ready ? 0.0 : kPlanesSetupUs) < est[best])
+            t = tb->S * step;
         if (t >= 0 && (est[ANC_ENGINE_TENSOR] < 0 || t < est[ANC_ENGINE_TENSOR])) {
             est[ANC_ENGINE_TENSOR] = t;
             if (est[best] < 0 || t < est[best] || best == ANC_ENGINE_TENSOR) {
@@ -825,7 +833,7 @@ int tune_kernel(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
         float ms = 0.f, best_ms = 0.f;
         for (int rep = 0; rep < 3; ++rep) {
             CK(cudaEventRecord(I->ev0, st));
-            int rc = run_device_impl(I, tb, seed, off, nprobe, &po, pout, st, Sp);
+            int rc = run_device_impl(I, tb, seed, off, nprobe, &po, pout, st, rep ? Sp : std::min(Sp, 8));
             if (rc) return rc;
             CK(cudaEventRecord(I->ev1, st));
             CK(cudaEventSynchronize(I->ev1));

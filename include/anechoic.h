@@ -146,8 +146,8 @@ ANC_API int anc_sparse_tuning(const anc_instance* inst, int* variant, double* pr
  *     fewest lanes), 1 = 8 (16 CTAs per replica group), 2 = 4 (32 CTAs), 3 = 2 (64 CTAs).
  * The first synchronous run (anc_run / anc_run_fields) that uses one of these kernels for a (device, kernel, NP, K,
  * replica groups) key not yet tuned runs each variant on the first min(S, 256) steps of that run's anneals (one wave
- * of the plain engine, every replica group of the fp4 kernel) into the handle's own workspaces -- three times, the
- * least of the last two launches timed -- and keeps variant 0 unless another probes more than 1 % faster, in which
+ * of the plain engine, every replica group of the fp4 kernel) into the handle's own workspaces -- after a launch of
+ * 8 steps twice, the lesser time counted -- and keeps variant 0 unless another probes more than 1 % faster, in which
  * case the fastest, for every later launch with that key in the process (device and
  * graph-captured launches included; anc_run_batch and anc_run_batch_noalloc use variant 0). For the key a run of
  * nchains anneals of this instance on `kernel` would use, writes the chosen variant (-1 = not tuned yet), the number
