@@ -1477,8 +1477,8 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
         if (jobs[k].inst->K == 0) sparse_anneals += jobs[k].nchains;
     auto sparse_class = [&](const anc_instance* I) {
         const bool group = I->slices && anc::sparse_groups(I->np, std::max(8.0, row_degree(I)), sparse_anneals, sms);
-        // few anneals: one launch, one anneal per SM
-        if (sparse_anneals <= 2 * sms) return 3;
+        // few anneals: one launch, one anneal at a time per SM
+        if (sparse_anneals <= anc::kBatchAlone * sms) return 3;
         return (group ? 0 : 3) + (I->np <= 2304 ? 0 : I->np <= 9216 ? 1 : 2);
     };
     KindPlan sparse_plans[kClasses];

@@ -85,6 +85,10 @@ struct PlainLaunch {
 constexpr uint32_t kEdgePad = 0x7fe0;  // padding edge of csr16 rows
 
 // Sparse jobs with unit weights and short rows run several replicas of an instance together (sparse_engine.cu).
+// A batch of uneven sparse instances with at most this many anneals per SM runs them one per SM, longest first: its largest
+// instances set the time, and those are slow beside others. 12 to 51 instances, S = 150, ms one per SM / by class: 312 anneals
+// 1.9 / 3.5, 570 3.0 / 4.8, 816 4.8 / 4.9, 1200 (in groups, sparse_groups) 6.3 / 4.1.
+constexpr int kBatchAlone = 8;
 constexpr int kGroupReplicas = 8;
 constexpr int kGroupDegree = 120;      // a row's four byte sums stay below 256
 constexpr int kGroupNp = 7936;         // a slot's byte offset fits 16 bits, padding included

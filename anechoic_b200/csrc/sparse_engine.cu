@@ -696,7 +696,7 @@ int sparse_launch(const PlainLaunch& L, int per_sm, int sms, cudaStream_t st) {
         threads = 1024;
         smem = wide_smem(L.np_max, threads);
         grid = std::min(grid, sms);
-    } else if (L.nitems <= sms || per_sm < 2 || (L.items && L.nitems <= 2 * sms)) {
+    } else if (L.nitems <= sms || per_sm < 2 || (L.items && L.nitems <= kBatchAlone * sms)) {
         // one CTA of 512 threads per SM (plain_engine.cu)
         const size_t plain = plain_smem_bytes(L.np_max, L.np_max / 32, 0, 12);
         return plain_launch(L, 0, 12, std::min(grid, sms), plain, st);

@@ -63,7 +63,7 @@ def test_forms_vs_oracle(cuda, oracle, name, build, chains, sched, wide):
 
 
 def test_batch_mixes_forms(cuda, oracle):
-    """More anneals than two per SM: groups of two sizes, weighted rows, long rows and a 20000-spin torus in one call."""
+    """More anneals than eight per SM: groups of two sizes, weighted rows, long rows and a 20000-spin torus in one call."""
     insts = [I.random_graph(500, 3000, True, 1, bmax=2), I.random_graph(3000, 9000, False, 2), _weighted(600, 3),
              _hub(400, 150), I.torus(100, 200, 4), I.torus(20, 40, 5, bmax=1)]
     counts = [333, 200, 150, 130, 3, 401]
