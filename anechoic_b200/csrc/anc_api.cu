@@ -1193,13 +1193,13 @@ int anc_instance_create_csr(int n, const int32_t* row_ptr, const int32_t* col, c
     size_t rp16_at = 0, adj16_at = 0, slices_at = 0, info_at = 0, counts_at = 0;
     bool sliced = false;
     // unit weights and np <= kEdgePad: the same rows with 16-bit edges y | [J = -1] << 15, two per word, each row padded to a
-    // whole word with the edge kEdgePad; the CSR pass then fetches half the words
+    // whole word with the edge 0x7fff; the CSR pass then fetches half the words
     bool unit = I->np <= int(anc::kEdgePad);
     for (int64_t k = 0; unit && k < nnz; ++k) unit = val[k] == 1 || val[k] == -1;
     if (unit) {
         std::vector<int32_t> rp16(size_t(n) + 1, 0);
         for (int x = 0; x < n; ++x) rp16[x + 1] = rp16[x] + (row_ptr[x + 1] - row_ptr[x] + 1) / 2;
-        std::vector<uint32_t> a16(std::max<int32_t>(rp16[n], 1), anc::kEdgePad * 0x10001u);
+        std::vector<uint32_t> a16(std::max<int32_t>(rp16[n], 1), 0x7fff7fffu);
         std::vector<int32_t> minus(n, 0);
         int longest = 0;
         for (int x = 0; x < n; ++x) {

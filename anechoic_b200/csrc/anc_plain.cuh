@@ -35,7 +35,7 @@ struct PlainJob {
     const int32_t* row_ptr;            // sparse: [n + 1] (csr16: in words of two edges)
     const uint32_t* adj;               // sparse: (y << 8) | uint8(J_xy); csr16: two 16-bit edges per word
     int csr16;                         // sparse, every J_xy = +-1 and np <= kEdgePad: edge = y | [J_xy = -1] << 15, rows
-                                       // padded to whole words with the edge kEdgePad
+                                       // padded to whole words with the skip edge 0x7fff
     const int32_t* bias;               // [n] or null
     DevTables tab;
     uint64_t seed;
@@ -82,7 +82,7 @@ struct PlainLaunch {
     int32_t* group_h;                  // sparse_group_scratch words
 };
 
-constexpr uint32_t kEdgePad = 0x7fe0;  // padding edge of csr16 rows
+constexpr uint32_t kEdgePad = 0x7fe0;  // slots of csr16 rows lie below; a skip edge has all of its bits
 
 // Sparse jobs with unit weights and short rows run several replicas of an instance together (sparse_engine.cu).
 // A batch of uneven sparse instances with at most this many anneals per SM runs them one per SM, longest first: its largest

@@ -332,13 +332,13 @@ __device__ __forceinline__ int sparse_lanes_log2(int nnz, int n) {
     return lg;
 }
 
-// One word of edges: (y << 8) | uint8(J), or with E16 two edges y | [J = -1] << 15 (y >= kEdgePad: no edge).
+// One word of edges: (y << 8) | uint8(J), or with E16 two edges y | [J = -1] << 15 (0x7fff: no edge).
 template <bool E16>
 __device__ __forceinline__ void sparse_apply(uint32_t v, int32_t m, int32_t* h) {
     if (E16) {
         const uint32_t lo = v & 0xffffu, hi = v >> 16;
-        if ((lo & 0x7fffu) < kEdgePad) atomicAdd(&h[lo & 0x7fffu], (lo >> 15) ? -m : m);
-        if ((hi & 0x7fffu) < kEdgePad) atomicAdd(&h[hi & 0x7fffu], (hi >> 15) ? -m : m);
+        if ((lo & 0x7fffu) != 0x7fffu) atomicAdd(&h[lo & 0x7fffu], (lo >> 15) ? -m : m);
+        if ((hi & 0x7fffu) != 0x7fffu) atomicAdd(&h[hi & 0x7fffu], (hi >> 15) ? -m : m);
     } else {
         atomicAdd(&h[v >> 8], m * int32_t(int8_t(v & 0xffu)));
     }

@@ -36,8 +36,8 @@ template <bool E16>
 __device__ __forceinline__ void apply_word(uint32_t v, int32_t m, int32_t* h) {
     if (E16) {
         const uint32_t lo = v & 0xffffu, hi = v >> 16;
-        if ((lo & 0x7fffu) < kEdgePad) atomicAdd(&h[lo & 0x7fffu], (lo >> 15) ? -m : m);
-        if ((hi & 0x7fffu) < kEdgePad) atomicAdd(&h[hi & 0x7fffu], (hi >> 15) ? -m : m);
+        if (~lo & kEdgePad) atomicAdd(&h[lo & 0x7fffu], (lo >> 15) ? -m : m);
+        if (~hi & kEdgePad) atomicAdd(&h[hi & 0x7fffu], (hi >> 15) ? -m : m);
     } else {
         atomicAdd(&h[v >> 8], m * int32_t(int8_t(v & 0xffu)));
     }
