@@ -130,6 +130,10 @@ __global__ void __launch_bounds__(kSThreads, 1)
     uint32_t hph = 0u, q = 0u, rph = 0u;
 
     for (int pr = 0; pr < P.npairs; ++pr) {
+        // Step m's updates are in the rows of parity (m + ph) & 1, which alternate over the S + 1 publications of every pair: a
+        // CTA that enters a pair may find others still loading the last step's updates of the pair before it, but none that
+        // still loads those of the step before that.
+        const int ph = pr & (S + 1) & 1;
         if (warp < kSDW) {
             // ---------------- decision warps ----------------
             const int g = warp >> 3, jl = (warp >> 2) & 1;
@@ -163,12 +167,13 @@ __global__ void __launch_bounds__(kSThreads, 1)
                     const uint32_t b = valid ? (up ? 0x01u : 0xFFu) : 0u;
                     dwords[k >> 2] |= b << (8 * (k & 3));
                 }
-                int8_t* dst = P.dbuf + ((drow0 + kSM) * kSNPP) + cs * kSCols + jl * RP;   // parity 1
+                const size_t row = drow0 + size_t(ph ^ 1) * kSM;                          // m = -1
+                int8_t* dst = P.dbuf + row * kSNPP + cs * kSCols + jl * RP;
 #pragma unroll
                 for (int e = 0; e < RP / 16; ++e)
                     reinterpret_cast<uint4*>(dst)[e] =
                         make_uint4(dwords[4 * e], dwords[4 * e + 1], dwords[4 * e + 2], dwords[4 * e + 3]);
-                P.nlx[(drow0 + kSM) * 256 + 2 * cs + jl] = 0;
+                P.nlx[row * 256 + 2 * cs + jl] = 0;
                 uint32_t v[16];
 #pragma unroll
                 for (int h4 = 0; h4 < RP / 16; ++h4) {
@@ -250,7 +255,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 const uint32_t lw = uint32_t(2 * twoT - 1);
                 const int32_t xs = qv - corr, twocorr = 2 * corr, c1 = twoT - 1;
                 uint64_t fm = 0, lm = 0;
-                const int par = m & 1;
+                const int par = (m + ph) & 1;
                 int8_t* dst = P.dbuf + ((drow0 + size_t(par) * kSM) * kSNPP) + cs * kSCols + jl * RP;
 #pragma unroll
                 for (int c16 = 0; c16 < RP / 16; ++c16) {
@@ -315,7 +320,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
             const int pwid = warp - kSDW;
             const uint32_t* fl = P.flags + pr * kSSlices;
             for (int m = -1; m < S; ++m) {
-                const int par = m & 1;
+                const int par = (m + ph) & 1;
                 const uint32_t target = uint32_t(m + 2);
                 uint32_t ready[4] = {0u, 0u, 0u, 0u};        // slices seen at >= target, by 32-slice window
                 for (int c = 0; c < kSChunks; ++c, ++q) {
