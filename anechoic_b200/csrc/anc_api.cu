@@ -1627,7 +1627,8 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
             L.nwj_max = kp.np_max / 32;
             L.np_min = kp.np_min;
             L.groups = ci < 3;
-            for (const Prepared& p : prep) L.clamp = L.clamp || p.hclamp > 0;
+            for (const Prepared& p : prep)
+                L.clamp = L.clamp || (p.hclamp > 0 && jobs[p.idx].inst->K == 0 && sparse_class(jobs[p.idx].inst) == ci);
             L.group_h = L.groups ? reinterpret_cast<int32_t*>(arena.p + group_at[ci]) : nullptr;
             if (e == cudaSuccess) e = cudaMemsetAsync(L.next_item, 0, sizeof(int), cst);
             if (e != cudaSuccess) return cuda_fail(e, "sparse launch");

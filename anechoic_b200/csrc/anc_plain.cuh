@@ -78,7 +78,7 @@ struct PlainLaunch {
     int dense_variant;                 // dense pass variant (dense_variants(K) of them; 0 = the default)
     int np_min;                        // sparse batches: the smallest job's np
     int groups;                        // sparse: items are groups of kGroupReplicas trials, every job has slices
-    int clamp;                         // sparse groups: some job has hclamp > 0
+    int clamp;                         // sparse groups: some job of this launch has hclamp > 0
     int32_t* group_h;                  // sparse_group_scratch words
 };
 

@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kGroupThreads, 4 / kQuads) sparse_group_kernel
         const int2 it = L.items ? L.items[item] : make_int2(0, NR * item);
         const PlainJob& job = L.items ? L.jobs[it.x] : L.job0;
         const int n = job.n, np = job.np, R = np / kLanes, RA = (n + kLanes - 1) / kLanes, S = job.tab.S, c0 = it.y + 4 * q;
-        const int32_t hclamp = job.hclamp;
+        const int32_t hclamp = job.hclamp > 0 ? job.hclamp : 0x7fffffff;     // 0: the job's fields need no clamp
         const int32_t* __restrict__ bias = job.bias;
         const uint32_t* __restrict__ row_c = job.row_counts;
         const uint2* __restrict__ slice_t = job.slice_info + (l >> 5);       // slice 8 k + l / 32
