@@ -412,8 +412,10 @@ __global__ void __launch_bounds__(kGroupThreads, 4 / kQuads) sparse_group_kernel
     constexpr int Q = kQuads, TPB = kGroupThreads, NR = kGroupReplicas;
     static_assert(Q == 2, "edges are offsets of 8 bytes a slot");
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    __shared__ int s_item, s_nl[3][NR], s_fl[NR];
+    __shared__ int s_item;
+    __shared__ uint32_t s_cnt[3][NR];          // a step's counts per replica, each below 2^16: n_lin | flips << 16
     __shared__ unsigned long long s_red[2][NR];
+    __shared__ long long s_fl[NR];             // flips so far; thread r alone uses replica r's
     const uint32_t half = uint32_t(L.np_max + 32) * 4 * Q;                   // bytes of a half of moves
     const uint32_t base = uint32_t(__cvta_generic_to_shared(smem_raw));
     int4* h = reinterpret_cast<int4*>(L.group_h) + size_t(blockIdx.x) * L.np_max * Q + threadIdx.x;
@@ -456,7 +458,7 @@ __global__ void __launch_bounds__(kGroupThreads, 4 / kQuads) sparse_group_kernel
             reinterpret_cast<uint32_t*>(smem_raw)[np * Q + tid] = 0u;
             reinterpret_cast<uint32_t*>(smem_raw + half)[np * Q + tid] = 0u;
         }
-        if (tid < 3 * NR) (&s_nl[0][0])[tid] = 0;
+        if (tid < 3 * NR) (&s_cnt[0][0])[tid] = 0u;
         if (tid < NR) s_fl[tid] = 0;
         if (tid < 2 * NR) (&s_red[0][0])[tid] = 0ull;
         __syncthreads();
@@ -493,7 +495,7 @@ __global__ void __launch_bounds__(kGroupThreads, 4 / kQuads) sparse_group_kernel
                 const int64_t kcorr = __ldg(job.tab.kcorr + t);
                 const int32_t kconst = __ldg(job.tab.kconst + t);
 #pragma unroll
-                for (int r = 0; r < 4; ++r) corr[r] = step_corr(t ? s_nl[(t + 2) % 3][4 * q + r] : 0, kcorr, kconst);
+                for (int r = 0; r < 4; ++r) corr[r] = step_corr(t ? int(s_cnt[(t + 2) % 3][4 * q + r] & 0xffffu) : 0, kcorr, kconst);
             }
             uint32_t nl = 0u, nf = 0u;                                      // a byte per replica: RA <= 31
             uint2 sn = __ldg(slice_t);
@@ -540,20 +542,19 @@ __global__ void __launch_bounds__(kGroupThreads, 4 / kQuads) sparse_group_kernel
             const uint32_t n02 = __reduce_add_sync(quad_lanes, nl & 0x00ff00ffu), n13 = __reduce_add_sync(quad_lanes, (nl >> 8) & 0x00ff00ffu);
             const uint32_t f02 = __reduce_add_sync(quad_lanes, nf & 0x00ff00ffu), f13 = __reduce_add_sync(quad_lanes, (nf >> 8) & 0x00ff00ffu);
             if (lane < Q) {
-                int* sn4 = &s_nl[t % 3][4 * q];
-                int* sf4 = &s_fl[4 * q];
-                atomicAdd(sn4, int(n02 & 0xffffu));
-                atomicAdd(sn4 + 1, int(n13 & 0xffffu));
-                atomicAdd(sn4 + 2, int(n02 >> 16));
-                atomicAdd(sn4 + 3, int(n13 >> 16));
-                atomicAdd(sf4, int(f02 & 0xffffu));
-                atomicAdd(sf4 + 1, int(f13 & 0xffffu));
-                atomicAdd(sf4 + 2, int(f02 >> 16));
-                atomicAdd(sf4 + 3, int(f13 >> 16));
+                uint32_t* sc4 = &s_cnt[t % 3][4 * q];
+                atomicAdd(sc4, (n02 & 0xffffu) | f02 << 16);
+                atomicAdd(sc4 + 1, (n13 & 0xffffu) | f13 << 16);
+                atomicAdd(sc4 + 2, n02 >> 16 | (f02 & 0xffff0000u));
+                atomicAdd(sc4 + 3, n13 >> 16 | (f13 & 0xffff0000u));
             }
-            if (tid < NR) s_nl[(t + 1) % 3][tid] = 0;       // last read two barriers ago
+            if (tid < NR) s_cnt[(t + 1) % 3][tid] = 0u;     // last read before the previous barrier
             __syncthreads();
-            if (tracer) job.out_trace[size_t(it.y + tid) * S + t] = s_nl[t % 3][tid];
+            if (tid < NR) {
+                const uint32_t sc = s_cnt[t % 3][tid];
+                if (tracer) job.out_trace[size_t(it.y + tid) * S + t] = int32_t(sc & 0xffffu);
+                s_fl[tid] += sc >> 16;
+            }
         }
         // the last step's moves into the fields, and the outputs
         const uint32_t cur = (S & 1) ? half : 0u;
