@@ -469,8 +469,8 @@ int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t 
             L.groups = 1;
             L.clamp = job.hclamp > 0;
             L.nitems = (job.ntrials + anc::kGroupReplicas - 1) / anc::kGroupReplicas;
-            const size_t words = anc::sparse_group_scratch(I->np, L.nitems, I->sms);
-            CK(I->w_group.ensure(words));
+            // for as many CTAs as any launch has, so that it never moves: a captured launch names it
+            CK(I->w_group.ensure(anc::sparse_group_scratch(I->np, 1 << 30, I->sms)));
             L.group_h = I->w_group.p;
         }
     } else {

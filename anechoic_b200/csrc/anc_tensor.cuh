@@ -8,6 +8,52 @@
 
 namespace anc {
 
+// Whether work submitted to the stream is being recorded into a CUDA graph.
+inline bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return s != cudaStreamCaptureStatusNone;
+}
+
+// A handle's device workspace, which grows with its largest call. A block that a captured launch uses is kept until the handle
+// goes, because the graph may be replayed after the workspace has grown; other blocks are freed when they are replaced.
+struct Workspace {
+    uint8_t* p = nullptr;
+    size_t bytes = 0;
+    // At least `need` bytes for a launch on st. While st is being captured nothing can be allocated: a call that needs more is
+    // refused without ending the capture.
+    cudaError_t ensure(size_t need, cudaStream_t st) {
+        const bool cap = capturing(st);
+        if (bytes < need) {
+            if (cap) return cudaErrorStreamCaptureUnsupported;
+            if (p && captured) kept.push_back(p);
+            else if (p) cudaFree(p);
+            p = nullptr;
+            bytes = 0;
+            captured = false;
+            void* q = nullptr;
+            const cudaError_t e = cudaMalloc(&q, need);
+            if (e != cudaSuccess) return e;
+            p = static_cast<uint8_t*>(q);
+            bytes = need;
+        }
+        captured = captured || cap;
+        return cudaSuccess;
+    }
+    void free() {
+        if (p) cudaFree(p);
+        for (uint8_t* k : kept) cudaFree(k);
+        *this = Workspace{};
+    }
+
+private:
+    bool captured = false;
+    std::vector<uint8_t*> kept;
+};
+
 struct TensorInstance {
     int n = 0, np = 0;
     int npp = 0;                 // permuted width of J_perm (np, or 256 x the padded rounds for the streaming kernel)
@@ -15,8 +61,7 @@ struct TensorInstance {
     std::vector<int> perm;       // slot i -> permuted index (CTA-contiguous slot slices)
     int8_t* d_J = nullptr;       // J_perm [np][np] int8 (row = y, contiguous x)
     size_t bytes = 0;
-    void* d_ws = nullptr;        // exchange buffers + error word
-    size_t ws_bytes = 0;
+    Workspace ws;                // exchange buffers + error word
     int32_t* d_bias_perm = nullptr;
     int* last_err = nullptr;     // error word of the last launch
     int last_ctas = 0, last_cluster = 0;
@@ -74,8 +119,7 @@ struct PlanesInstance {
     int n = 0, R = 0, W = 0;
     uint8_t* d_J = nullptr;      // [W][256 RP][128 RP] packed e2m1
     int32_t* d_bias = nullptr;   // bias at permuted column
-    void* d_ws = nullptr;        // error word, flags, exchange buffers
-    size_t ws_bytes = 0;
+    Workspace ws;                // error word, flags, exchange buffers
     int* last_err = nullptr;     // error word of the last launch
     int last_ctas = 0;
 };

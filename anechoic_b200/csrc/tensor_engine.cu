@@ -996,19 +996,13 @@ int res_run(TensorInstance* ti, const TensorRun& r, cudaStream_t st, std::string
     const size_t dbytes = size_t(ngroups) * 2 * kM * 2048;
     const size_t nbytes = size_t(ngroups) * 2 * kM * 128;
     const size_t need = 256 + fbytes + dbytes + nbytes + 256;
-    cudaError_t e = cudaSuccess;
-    if (ti->ws_bytes < need) {
-        if (ti->d_ws) cudaFree(ti->d_ws);
-        ti->d_ws = nullptr;
-        ti->ws_bytes = 0;
-        e = cudaMalloc(&ti->d_ws, need);
-        if (e != cudaSuccess) {
-            if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-            return -2;
-        }
-        ti->ws_bytes = need;
+    ti->last_err = nullptr;
+    cudaError_t e = ti->ws.ensure(need, st);
+    if (e != cudaSuccess) {
+        if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
+        return -2;
     }
-    uint8_t* base = static_cast<uint8_t*>(ti->d_ws);
+    uint8_t* base = ti->ws.p;
     int* err = reinterpret_cast<int*>(base);
     uint32_t* flags = reinterpret_cast<uint32_t*>(base + 256);
     int8_t* dbuf = reinterpret_cast<int8_t*>(base + 256 + ((fbytes + 255) / 256) * 256);
@@ -1110,21 +1104,15 @@ int tensor_run(TensorInstance* ti, const TensorRun& r, cudaStream_t st, std::str
     // workspace: exchange buffers, permuted bias, error word
     const size_t dbytes = size_t(groups) * 2 * kM * np;
     const size_t nlbytes = size_t(groups) * 2 * kC * kM * 4;
-    cudaError_t e = cudaSuccess;
-    if (ti->ws_bytes < dbytes + nlbytes + 256) {
-        if (ti->d_ws) cudaFree(ti->d_ws);
-        ti->d_ws = nullptr;
-        ti->ws_bytes = 0;
-        e = cudaMalloc(&ti->d_ws, dbytes + nlbytes + 256);
-        if (e != cudaSuccess) {
-            if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-            return -2;
-        }
-        ti->ws_bytes = dbytes + nlbytes + 256;
+    ti->last_err = nullptr;
+    cudaError_t e = ti->ws.ensure(dbytes + nlbytes + 256, st);
+    if (e != cudaSuccess) {
+        if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
+        return -2;
     }
-    int8_t* dbuf = static_cast<int8_t*>(ti->d_ws);
-    int32_t* nlbuf = reinterpret_cast<int32_t*>(static_cast<uint8_t*>(ti->d_ws) + dbytes);
-    int* err = reinterpret_cast<int*>(static_cast<uint8_t*>(ti->d_ws) + dbytes + nlbytes);
+    int8_t* dbuf = reinterpret_cast<int8_t*>(ti->ws.p);
+    int32_t* nlbuf = reinterpret_cast<int32_t*>(ti->ws.p + dbytes);
+    int* err = reinterpret_cast<int*>(ti->ws.p + dbytes + nlbytes);
     CUtensorMap mapA, mapB;
     if (!make_map(&mapA, dbuf, uint64_t(np), uint64_t(groups) * 2 * kM, kM) ||
         !make_map(&mapB, ti->d_J, uint64_t(np), uint64_t(np), uint32_t(16 * R))) {
@@ -1195,12 +1183,11 @@ int tensor_check_error(const int* err, cudaStream_t st, std::string* why) {
 void tensor_free_instance(TensorInstance* ti) {
     if (!ti) return;
     if (ti->d_J) cudaFree(ti->d_J);
-    if (ti->d_ws) cudaFree(ti->d_ws);
     if (ti->d_bias_perm) cudaFree(ti->d_bias_perm);
     ti->d_J = nullptr;
-    ti->d_ws = nullptr;
     ti->d_bias_perm = nullptr;
-    ti->ws_bytes = 0;
+    ti->ws.free();
+    ti->last_err = nullptr;
 }
 
 }  // namespace anc

@@ -821,18 +821,13 @@ int planes_run(PlanesInstance* pi, const TensorRun& r, cudaStream_t st, std::str
     const size_t dbytes = size_t(ngroups) * 2 * kM * (128 * c.rp);
     const size_t nbytes = size_t(ngroups) * 3 * kNlCopies * kM * 4;
     const size_t need = 256 + fbytes + nbytes + dbytes;
-    if (pi->ws_bytes < need) {
-        if (pi->d_ws) cudaFree(pi->d_ws);
-        pi->d_ws = nullptr;
-        pi->ws_bytes = 0;
-        e = cudaMalloc(&pi->d_ws, need);
-        if (e != cudaSuccess) {
-            if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-            return -2;
-        }
-        pi->ws_bytes = need;
+    pi->last_err = nullptr;
+    e = pi->ws.ensure(need, st);
+    if (e != cudaSuccess) {
+        if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
+        return -2;
     }
-    uint8_t* base = static_cast<uint8_t*>(pi->d_ws);
+    uint8_t* base = pi->ws.p;
     CUtensorMap mapJ;
     if (!make_map_2d(&mapJ, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pi->d_J, uint64_t(128) * c.rp, uint64_t(256) * c.rp * c.w,
                      128, uint32_t(c.ch))) {
@@ -898,7 +893,7 @@ int planes_run(PlanesInstance* pi, const TensorRun& r, cudaStream_t st, std::str
 void planes_free(PlanesInstance* pi) {
     if (pi->d_J) cudaFree(pi->d_J);
     if (pi->d_bias) cudaFree(pi->d_bias);
-    if (pi->d_ws) cudaFree(pi->d_ws);
+    pi->ws.free();
     *pi = PlanesInstance{};
 }
 

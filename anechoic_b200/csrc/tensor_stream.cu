@@ -555,18 +555,13 @@ int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm,
     const size_t dbytes = size_t(2) * 2 * kSM * kSNPP;
     const size_t nbytes = size_t(2) * 2 * kSM * 256;
     const size_t need = 256 + fbytes + dbytes + nbytes;
-    if (ti->ws_bytes < need) {
-        if (ti->d_ws) cudaFree(ti->d_ws);
-        ti->d_ws = nullptr;
-        ti->ws_bytes = 0;
-        e = cudaMalloc(&ti->d_ws, need);
-        if (e != cudaSuccess) {
-            if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-            return -2;
-        }
-        ti->ws_bytes = need;
+    ti->last_err = nullptr;
+    e = ti->ws.ensure(need, st);
+    if (e != cudaSuccess) {
+        if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
+        return -2;
     }
-    uint8_t* base = static_cast<uint8_t*>(ti->d_ws);
+    uint8_t* base = ti->ws.p;
     int* err = reinterpret_cast<int*>(base);
     uint32_t* flags = reinterpret_cast<uint32_t*>(base + 256);
     int8_t* dbuf = reinterpret_cast<int8_t*>(base + 256 + fbytes);

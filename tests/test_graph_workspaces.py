@@ -1,0 +1,76 @@
+"""GPU: captured anc_run_device calls and the workspaces of their handles. A larger run of the same handle after the capture
+leaves the captured call's workspaces in place, so that replays stay exact."""
+import numpy as np
+import pytest
+import torch
+
+import anechoic_b200 as A
+from anechoic_b200 import _lib, instances as I
+
+pytestmark = pytest.mark.gpu
+
+SCHED = dict(S=9, lam=1.05, ramp=True)
+SPARSE = dict(S=9, t0=6.0, t1=0.5, q=1.5, kappa=2.0, ramp=True)
+
+# name, instance, schedule, engine and operand format, anneals captured, anneals of the larger run
+CASES = {
+    "sparse groups": (lambda: I.random_graph(1000, 10000, True, 6, bmax=2), SPARSE, "auto", "auto", 1187, 2400),
+    "planes": (lambda: I.complete_pm1(2501, 4), SCHED, "auto", "auto", 100, 1300),
+    "fp4": (lambda: I.complete_pm1(2000, 4), SCHED, "tensor", "fp4", 130, 2100),
+    "int8": (lambda: I.random_kbit(2000, 4, 5, pzero=0.2, bmax=3), dict(SCHED, t0=300.0), "tensor", "int8", 130, 1100),
+    "streaming": (lambda: I.complete_pm1(6200, 4), SCHED, "auto", "auto", 130, 900),
+}
+
+
+class _Out:
+    def __init__(self, n, chains):
+        W = A.spin_words(n)
+        z = lambda *s: torch.zeros(s, dtype=torch.int64, device="cuda")
+        self.t = (z(chains, W), z(chains), z(chains), z(chains))
+
+    def launch(self, dev, tb, o, off, stream):
+        _lib.check(_lib.load().anc_run_device(dev._h, tb._h, 11, off, len(self.t[1]), o, *(x.data_ptr() for x in self.t),
+                                              None, stream.cuda_stream))
+
+    def same(self, r):
+        sp, sh, bs, fl = (x.cpu().numpy() for x in self.t)
+        return (np.array_equal(sp.view(np.uint64), r.spins) and np.array_equal(sh, r.sum_sh) and
+                np.array_equal(bs, r.sum_bs) and np.array_equal(fl, r.flips))
+
+
+def _eager(out, *args):
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        out.launch(*args, side)
+    torch.cuda.synchronize()
+
+
+def _capture(out, *args):
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        out.launch(*args, torch.cuda.current_stream())
+    return g
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_replay_after_a_larger_run(cuda, case):
+    build, sched, engine, kind, few, many = CASES[case]
+    inst = build()
+    dev, tb = A.DeviceInstance(inst), A.Tables.from_schedule(A.Schedule(**sched))
+    o = _lib.opts(engine, tensor_kind=kind)
+    ref = A.run(dev, tb, 11, 40, few, engine=engine, tensor_kind=kind)
+    out = _Out(inst.n, few)
+    _eager(out, dev, tb, o, 40)
+    g = _capture(out, dev, tb, o, 40)
+    big = A.run(dev, tb, 11, 0, many, engine=engine, tensor_kind=kind)
+    assert np.array_equal(big.spins[40:40 + few], ref.spins)
+    fill = [torch.full((1 << 18,), -1, dtype=torch.int32, device="cuda") for _ in range(64)]   # freed blocks find new owners
+    for _ in range(2):
+        for x in out.t:
+            x.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert out.same(ref)
+    assert all(int((f != -1).sum()) == 0 for f in fill)
