@@ -446,6 +446,16 @@ int tuned_variant(anc_instance* I, int kernel, int nchains);
 // Mean edges per row of a sparse instance.
 double row_degree(const anc_instance* I) { return double(I->info.nnz) / std::max(1, I->n); }
 
+// The fields of grouped launches, for as many CTAs as any launch has, so that they never move: a captured launch names them.
+// False where they do not fit or would have to be allocated during a capture (the launch then runs without groups).
+bool ensure_group_fields(anc_instance* I, cudaStream_t st) {
+    if (I->w_group.p) return true;
+    if (anc::capturing(st)) return false;
+    if (I->w_group.ensure(anc::sparse_group_scratch(I->np, 1 << 30, I->sms)) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 // One launch of the one-CTA plain engine; variant >= 0 forces the CSR pass variant (sparse instances) or the dense
 // pass variant (dense instances), else the tuned one.
 int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t st, int variant = -1) {
@@ -465,12 +475,10 @@ int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t 
     if (rc) return rc;
     if (I->K == 0) {
         L.sparse_variant = variant >= 0 ? variant : std::max(0, I->sparse_variant);
-        if (job.slices && anc::sparse_groups(I->np, row_degree(I), job.ntrials, I->sms)) {
+        if (job.slices && anc::sparse_groups(I->np, row_degree(I), job.ntrials, I->sms) && ensure_group_fields(I, st)) {
             L.groups = 1;
             L.clamp = job.hclamp > 0;
             L.nitems = (job.ntrials + anc::kGroupReplicas - 1) / anc::kGroupReplicas;
-            // for as many CTAs as any launch has, so that it never moves: a captured launch names it
-            CK(I->w_group.ensure(anc::sparse_group_scratch(I->np, 1 << 30, I->sms)));
             L.group_h = I->w_group.p;
         }
     } else {
@@ -602,32 +610,40 @@ int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts
     return best;
 }
 
-int ensure_tensor(anc_instance* I, cudaStream_t st) {
+// Set-up of the tensor engine's operands. *no_room is set when it lacked device memory, or would have had to allocate while st
+// is being captured.
+int ensure_tensor(anc_instance* I, cudaStream_t st, bool* no_room) {
     if (I->tensor_ready) return ANC_OK;
     if (I->dense.empty()) return fail(ANC_EINVAL, "the tensor engine needs dense couplings");
+    if ((*no_room = anc::capturing(st)))
+        return fail(ANC_ECUDA, "tensor engine setup: the handle's first run of it must come before a capture");
     std::string why;
     const int rc = !anc::tensor_supported(I->n, I->K, 1) || anc::stream_supported(I->n)
                        ? anc::stream_build(I->planes.p, I->K, I->nwj, I->n, &I->tensor, st, &why)
                        : anc::tensor_build_instance(I->dense.data(), I->n, &I->tensor, &why);
-    if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "tensor engine setup: %s", why.c_str());
+    *no_room = rc == anc::kNoRoom;
+    if (rc) return fail(rc == -1 ? ANC_EINVAL : ANC_ECUDA, "tensor engine setup: %s", why.c_str());
     I->tensor_ready = true;
     return ANC_OK;
 }
 
-int ensure_planes(anc_instance* I, cudaStream_t st) {
+int ensure_planes(anc_instance* I, cudaStream_t st, bool* no_room) {
     if (I->planes4_ready) return ANC_OK;
+    if ((*no_room = anc::capturing(st)))
+        return fail(ANC_ECUDA, "planes kernel setup: the handle's first run of it must come before a capture");
     std::string why;
     const int rc = anc::planes_build(I->planes.p, I->K, I->nwj, I->n, I->bias.empty() ? nullptr : I->bias.data(),
                                      I->info.maxabs, &I->planes4, st, &why);
-    if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "planes kernel setup: %s", why.c_str());
+    *no_room = rc == anc::kNoRoom;
+    if (rc) return fail(rc == -1 ? ANC_EINVAL : ANC_ECUDA, "planes kernel setup: %s", why.c_str());
     I->planes4_ready = true;
     return ANC_OK;
 }
 
 // Launch on device outputs; no synchronisation. S_probe > 0 runs only the first S_probe steps of the schedule (the
-// run-time tuners' probes).
+// run-time tuners' probes). no_room, when given, is set if the call failed for want of room (see ensure_tensor).
 int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, int nchains, const anc_run_opts* o,
-                    const OutPtrs& out, cudaStream_t st, int S_probe = 0) {
+                    const OutPtrs& out, cudaStream_t st, int S_probe = 0, bool* no_room = nullptr) {
     if (!I || !tb) return fail(ANC_EINVAL, "null handle");
     if (nchains < 1) return fail(ANC_EINVAL, "nchains must be >= 1");
     if (!out.spins || !out.sh || !out.fl) return fail(ANC_EINVAL, "spins, sum_sh and flips outputs are required");
@@ -636,7 +652,8 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
     if (rc) return rc;
     bool planes = false, streamed = false;
     const int engine = pick_engine(I, tb, nchains, o, nullptr, nullptr, &planes, &streamed);
-    if (engine == ANC_ENGINE_TENSOR) {
+    auto run_tensor = [&](bool* full) -> int {
+        *full = false;
         if (planes ? !planes_candidate(I) : !streamed && !anc::tensor_supported(I->n, I->K, nchains))
             return fail(ANC_EINVAL, "tensor engine does not support n=%d K=%d", I->n, I->K);
         const int kind = o ? o->tensor_kind : ANC_TENSOR_AUTO;
@@ -644,7 +661,7 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
             return fail(ANC_EINVAL, "tensor engine: the fp4 kernel needs NP = 2048, |J| <= 1 and max|b| + max_y sum_x "
                                     "|J_xy| < 16384");
         const bool fp4 = !planes && fp4_candidate(I) && kind != ANC_TENSOR_INT8;
-        rc = planes || fp4 ? ensure_planes(I, st) : ensure_tensor(I, st);
+        rc = planes || fp4 ? ensure_planes(I, st, full) : ensure_tensor(I, st, full);
         if (rc) return rc;
         const int forced = o ? o->kernel_variant : 0;
         if (forced > (planes ? 0 : anc::kF4Variants))
@@ -680,14 +697,24 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
         }
         std::string why;
         rc = planes || fp4 ? anc::planes_run(&I->planes4, r, st, &why) : anc::tensor_run(&I->tensor, r, st, &why);
+        *full = rc == anc::kNoRoom;
         if (rc == -3) return fail(ANC_ETIMEOUT, "tensor engine: %s", why.c_str());
-        if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "tensor engine: %s", why.c_str());
+        if (rc) return fail(rc == -1 ? ANC_EINVAL : ANC_ECUDA, "tensor engine: %s", why.c_str());
         if (planes || fp4) {
             I->tensor.last_ctas = I->planes4.last_ctas;     // the profile's geometry fields
             I->tensor.last_cluster = 1;
         }
         g_last_kernel = planes ? ANC_KERNEL_TENSOR_PLANES : fp4 ? ANC_KERNEL_TENSOR_FP4 : ANC_KERNEL_TENSOR_INT8;
         return ANC_OK;
+    };
+    if (engine == ANC_ENGINE_TENSOR) {
+        bool full = false;
+        rc = run_tensor(&full);
+        if (no_room) *no_room = full;
+        // AUTO runs the plain engine, which needs no operands or workspaces beyond the handle's, where the tensor engine's do
+        // not fit or do not exist yet in a capture; a profile or a forced variant is the tensor engine's
+        if (!full || (o && (o->engine == ANC_ENGINE_TENSOR || o->profile || o->kernel_variant))) return rc;
+        I->prof_ctas = 0;
     }
     anc::PlainJob job = make_job(I, tb, seed, off, nchains, hclamp, out);
     if (S_probe > 0) job.tab.S = std::min(job.tab.S, S_probe);
@@ -833,7 +860,9 @@ int tune_kernel(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, in
         float ms = 0.f, best_ms = 0.f;
         for (int rep = 0; rep < 3; ++rep) {
             CK(cudaEventRecord(I->ev0, st));
-            int rc = run_device_impl(I, tb, seed, off, nprobe, &po, pout, st, rep ? Sp : std::min(Sp, 8));
+            bool no_room = false;
+            int rc = run_device_impl(I, tb, seed, off, nprobe, &po, pout, st, rep ? Sp : std::min(Sp, 8), &no_room);
+            if (no_room) return ANC_OK;      // the run itself meets the same, and refuses or takes another engine
             if (rc) return rc;
             CK(cudaEventRecord(I->ev1, st));
             CK(cudaEventSynchronize(I->ev1));

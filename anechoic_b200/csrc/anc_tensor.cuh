@@ -18,6 +18,14 @@ inline bool capturing(cudaStream_t st) {
     return s != cudaStreamCaptureStatusNone;
 }
 
+// What a kernel's set-up returns when it lacks device memory, or would have to allocate during a capture: nothing has been
+// enqueued, and an engine that needs no memory of its own can run the call instead.
+constexpr int kNoRoom = -4;
+inline int setup_code(cudaError_t e) {
+    cudaGetLastError();
+    return e == cudaErrorMemoryAllocation || e == cudaErrorStreamCaptureUnsupported ? kNoRoom : -2;
+}
+
 // A handle's device workspace, which grows with its largest call. A block that a captured launch uses is kept until the handle
 // goes, because the graph may be replayed after the workspace has grown; other blocks are freed when they are replaced.
 struct Workspace {

@@ -969,8 +969,9 @@ int tensor_build_instance(const int8_t* J, int n, TensorInstance* out, std::stri
 namespace {
 
 // Permuted bias on the device (built once per instance from the caller's device bias) and its max |b|.
-int ensure_bias_perm(TensorInstance* ti, const int32_t* bias, std::string* why) {
+int ensure_bias_perm(TensorInstance* ti, const int32_t* bias, cudaStream_t st, std::string* why) {
     if (!bias || ti->d_bias_perm) return 0;
+    if (capturing(st)) return setup_code(cudaErrorStreamCaptureUnsupported);
     std::vector<int32_t> b(ti->n), bp(ti->npp, 0);
     cudaError_t e = cudaMemcpy(b.data(), bias, size_t(ti->n) * 4, cudaMemcpyDeviceToHost);
     for (int i = 0; i < ti->n && e == cudaSuccess; ++i) bp[ti->perm[i]] = b[i];
@@ -978,7 +979,9 @@ int ensure_bias_perm(TensorInstance* ti, const int32_t* bias, std::string* why) 
     if (e == cudaSuccess) e = cudaMemcpy(ti->d_bias_perm, bp.data(), size_t(ti->npp) * 4, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         if (why) *why = std::string("bias: ") + cudaGetErrorString(e);
-        return -2;
+        if (ti->d_bias_perm) cudaFree(ti->d_bias_perm);
+        ti->d_bias_perm = nullptr;
+        return setup_code(e);
     }
     return 0;
 }
@@ -1000,7 +1003,7 @@ int res_run(TensorInstance* ti, const TensorRun& r, cudaStream_t st, std::string
     cudaError_t e = ti->ws.ensure(need, st);
     if (e != cudaSuccess) {
         if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-        return -2;
+        return setup_code(e);
     }
     uint8_t* base = ti->ws.p;
     int* err = reinterpret_cast<int*>(base);
@@ -1096,7 +1099,7 @@ int tensor_wave_chains(int n, int* out) {
 
 int tensor_run(TensorInstance* ti, const TensorRun& r, cudaStream_t st, std::string* why) {
     const int np = ti->np, R = np / 256;
-    int rc0 = ensure_bias_perm(ti, r.bias, why);
+    int rc0 = ensure_bias_perm(ti, r.bias, st, why);
     if (rc0) return rc0;
     if (ti->stream) return stream_run(ti, r, r.bias ? ti->d_bias_perm : nullptr, st, why);
     if (R == 8) return res_run(ti, r, st, why);
@@ -1108,7 +1111,7 @@ int tensor_run(TensorInstance* ti, const TensorRun& r, cudaStream_t st, std::str
     cudaError_t e = ti->ws.ensure(dbytes + nlbytes + 256, st);
     if (e != cudaSuccess) {
         if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-        return -2;
+        return setup_code(e);
     }
     int8_t* dbuf = reinterpret_cast<int8_t*>(ti->ws.p);
     int32_t* nlbuf = reinterpret_cast<int32_t*>(ti->ws.p + dbytes);

@@ -795,7 +795,7 @@ int planes_build(const uint32_t* bits, int K, int nwj, int n, const int32_t* bia
     if (e != cudaSuccess) {
         if (why) *why = std::string("J planes: ") + cudaGetErrorString(e);
         planes_free(out);
-        return -2;
+        return setup_code(e);
     }
     out->n = n;
     out->R = R;
@@ -825,7 +825,7 @@ int planes_run(PlanesInstance* pi, const TensorRun& r, cudaStream_t st, std::str
     e = pi->ws.ensure(need, st);
     if (e != cudaSuccess) {
         if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-        return -2;
+        return setup_code(e);
     }
     uint8_t* base = pi->ws.p;
     CUtensorMap mapJ;

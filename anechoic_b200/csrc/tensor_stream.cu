@@ -527,7 +527,7 @@ int stream_build(const uint32_t* bits, int K, int nwj, int n, TensorInstance* ou
     if (e != cudaSuccess) {
         if (why) *why = std::string("J: ") + cudaGetErrorString(e);
         tensor_free_instance(out);
-        return -2;
+        return setup_code(e);
     }
     return 0;
 }
@@ -559,7 +559,7 @@ int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm,
     e = ti->ws.ensure(need, st);
     if (e != cudaSuccess) {
         if (why) *why = std::string("workspace: ") + cudaGetErrorString(e);
-        return -2;
+        return setup_code(e);
     }
     uint8_t* base = ti->ws.p;
     int* err = reinterpret_cast<int*>(base);

@@ -1,5 +1,6 @@
 """GPU: captured anc_run_device calls and the workspaces of their handles. A larger run of the same handle after the capture
-leaves the captured call's workspaces in place, so that replays stay exact."""
+leaves the captured call's workspaces in place, so that replays stay exact; and a handle whose workspaces do not exist yet (no
+eager call, or one with fewer anneals) can be captured under AUTO, as the engines that need none always could."""
 import numpy as np
 import pytest
 import torch
@@ -74,3 +75,25 @@ def test_replay_after_a_larger_run(cuda, case):
         torch.cuda.synchronize()
         assert out.same(ref)
     assert all(int((f != -1).sum()) == 0 for f in fill)
+
+
+@pytest.mark.parametrize("case", ["sparse groups", "planes", "streaming"])
+@pytest.mark.parametrize("before", ["nothing", "fewer anneals"])
+def test_capture_without_workspaces(cuda, case, before):
+    build, sched, engine, kind, few, many = CASES[case]
+    inst = build()
+    tb = A.Tables.from_schedule(A.Schedule(**sched))
+    o = _lib.opts(engine, tensor_kind=kind)
+    ref = A.run(A.DeviceInstance(inst), tb, 11, 0, many)       # another handle: loads the kernels
+    A.run(A.DeviceInstance(inst), tb, 11, 0, many, engine="plain")
+    dev = A.DeviceInstance(inst)
+    out = _Out(inst.n, many)
+    if before == "fewer anneals":
+        _eager(_Out(inst.n, 5), dev, tb, o, 0)
+    g = _capture(out, dev, tb, o, 0)
+    for _ in range(2):
+        for x in out.t:
+            x.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert out.same(ref)
