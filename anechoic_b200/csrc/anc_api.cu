@@ -73,14 +73,17 @@ struct DevBuf {
 };
 
 // Device memory of anc_run_batch calls. One block per device, of at most kKeepBytes, is kept between calls (allocating and
-// freeing 100 MB took up to 20 ms a call); concurrent calls allocate their own. A call has synchronised its streams before it
-// gives its block back. The kept blocks are freed with the last instance.
+// freeing 100 MB took up to 20 ms a call); concurrent calls allocate their own. A call that has synchronised its streams says
+// so (idle) and gives its block back; the block of one that failed on the way is freed, which waits for the device. The kept
+// blocks are freed with the last instance, or when a call finds no room beside one.
 class BatchMemory {
 public:
     ~BatchMemory() { give(); }
+    void idle() { idle_ = true; }
     cudaError_t take(int dev, size_t bytes) {
         give();
         dev_ = dev;
+        idle_ = false;
         std::lock_guard<std::mutex> lock(mu_);
         auto it = kept_.find(dev);
         if (it != kept_.end() && it->second.second >= bytes) {
@@ -89,7 +92,17 @@ public:
             return cudaSuccess;
         }
         n_ = std::max<size_t>(bytes, 1);
-        return cudaMalloc(&p, n_);
+        cudaError_t e = cudaMalloc(&p, n_);
+        if (e == cudaErrorMemoryAllocation && it != kept_.end()) {
+            cudaFree(it->second.first);
+            kept_.erase(it);
+            e = cudaMalloc(&p, n_);
+        }
+        if (e != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();
+        }
+        return e;
     }
     static void instance_created() {
         std::lock_guard<std::mutex> lock(mu_);
@@ -109,7 +122,7 @@ private:
         if (!p) return;
         std::lock_guard<std::mutex> lock(mu_);
         auto it = kept_.find(dev_);
-        if (n_ <= kKeepBytes && instances_ > 0 && (it == kept_.end() || it->second.second < n_)) {
+        if (idle_ && n_ <= kKeepBytes && instances_ > 0 && (it == kept_.end() || it->second.second < n_)) {
             if (it != kept_.end()) cudaFree(it->second.first);
             kept_[dev_] = {p, n_};
         } else {
@@ -119,6 +132,7 @@ private:
     }
     int dev_ = 0;
     size_t n_ = 0;
+    bool idle_ = false;
     static std::mutex mu_;
     static std::map<int, std::pair<uint8_t*, size_t>> kept_;
     static long instances_;
@@ -1461,7 +1475,12 @@ int anc_run_device(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off,
     return run_device_impl(I, tb, seed, off, nchains, o, out, reinterpret_cast<cudaStream_t>(stream));
 }
 
-int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
+}  // extern "C"
+
+namespace {
+
+// anc_run_batch; without `groups` no job runs in groups of replicas, which take device memory for their fields.
+int run_batch_impl(int njobs, const anc_job* jobs, const anc_run_opts* o, bool groups) {
     if (njobs < 1 || !jobs) return fail(ANC_EINVAL, "need jobs");
     // group by kernel kind (sparse / dense K); each group is one persistent launch with a cost-ordered work queue
     struct Prepared {
@@ -1505,7 +1524,7 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
     for (int k = 0; k < njobs; ++k)
         if (jobs[k].inst->K == 0) sparse_anneals += jobs[k].nchains;
     auto sparse_class = [&](const anc_instance* I) {
-        const bool group = I->slices && anc::sparse_groups(I->np, std::max(8.0, row_degree(I)), sparse_anneals, sms);
+        const bool group = groups && I->slices && anc::sparse_groups(I->np, std::max(8.0, row_degree(I)), sparse_anneals, sms);
         // few anneals: one launch, one anneal at a time per SM
         if (sparse_anneals <= anc::kBatchAlone * sms) return 3;
         return (group ? 0 : 3) + (I->np <= 2304 ? 0 : I->np <= 9216 ? 1 : 2);
@@ -1607,7 +1626,11 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
         if (sparse_plans[ci].np_max)
             group_at[ci] = place(4 * anc::sparse_group_scratch(sparse_plans[ci].np_max, class_first[ci + 1] - class_first[ci], sms));
     BatchMemory arena;
-    CK(arena.take(dev, need));
+    const bool grouped = group_at[0] || group_at[1] || group_at[2];
+    if (const cudaError_t e = arena.take(dev, need)) {
+        if (e == cudaErrorMemoryAllocation && grouped) return run_batch_impl(njobs, jobs, o, false);
+        return cuda_fail(e, "device memory of the batch");
+    }
     int* const counters = reinterpret_cast<int*>(arena.p + counters_at);
     int2* const d_items = reinterpret_cast<int2*>(arena.p + items_at);
     const anc::PlainJob* const d_jobs = reinterpret_cast<const anc::PlainJob*>(arena.p + jobs_at);
@@ -1628,7 +1651,9 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
         cudaStreamSynchronize(st);
         return rc;
     };
-    std::vector<uint8_t> staging(std::max(in_bytes, result_bytes));
+    // results of up to 64 MB come back in one copy; larger ones go straight to the caller's arrays
+    const bool staged = result_bytes <= (size_t(64) << 20);
+    std::vector<uint8_t> staging(std::max(in_bytes, staged ? result_bytes : 0));
     std::memcpy(staging.data(), pj.data(), sizeof(anc::PlainJob) * njobs);
     std::memcpy(staging.data() + (items_at - jobs_at), all_items.data(), sizeof(int2) * all_items.size());
     {
@@ -1712,15 +1737,16 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
             float ms[anc::kSparseVariants] = {};
             for (int rep = 0; rep < 2; ++rep) {
                 for (int k = 0; k < njobs; ++k) probe[k].tab.S = std::min(pj[k].tab.S, rep ? 64 : 8);
-                CK(cudaMemcpy(d_probe, probe.data(), sizeof(anc::PlainJob) * njobs, cudaMemcpyHostToDevice));
-                for (int v = 0; v < anc::kSparseVariants; ++v) {
-                    CK(cudaEventRecord(e0, st));
+                cudaError_t e = cudaMemcpyAsync(d_probe, probe.data(), sizeof(anc::PlainJob) * njobs, cudaMemcpyHostToDevice, st);
+                for (int v = 0; v < anc::kSparseVariants && e == cudaSuccess; ++v) {
+                    e = cudaEventRecord(e0, st);
                     const int rc = launch_kind(0, d_probe, v);
                     if (rc) return drain(rc);
-                    CK(cudaEventRecord(e1, st));
-                    CK(cudaEventSynchronize(e1));
-                    CK(cudaEventElapsedTime(&ms[v], e0, e1));
+                    if (e == cudaSuccess) e = cudaEventRecord(e1, st);
+                    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+                    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[v], e0, e1);
                 }
+                if (e != cudaSuccess) return drain(cuda_fail(e, "sparse tuner"));
             }
             for (int v = 0; v < anc::kSparseVariants; ++v)
                 if (sparse_variant < 0 || ms[v] < best) { best = ms[v]; sparse_variant = v; }
@@ -1735,14 +1761,25 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
         if (rc) return drain(rc);
     }
     if (cudaEventRecord(e1, st) != cudaSuccess) return drain(cuda_fail(cudaGetLastError(), "event"));
-    cudaError_t ce = cudaMemcpyAsync(staging.data(), arena.p, result_bytes, cudaMemcpyDeviceToHost, st);
-    for (int k = 0; k < njobs && ce == cudaSuccess; ++k)
-        if (jobs[k].trace)
-            ce = cudaMemcpyAsync(jobs[k].trace, arena.p + at[k].trace, size_t(jobs[k].nchains) * jobs[k].tb->S * 4,
-                                 cudaMemcpyDeviceToHost, st);
+    cudaError_t ce = cudaSuccess;
+    auto fetch = [&](void* to, size_t from, size_t bytes) {
+        if (to && ce == cudaSuccess) ce = cudaMemcpyAsync(to, arena.p + from, bytes, cudaMemcpyDeviceToHost, st);
+    };
+    if (staged) fetch(staging.data(), 0, result_bytes);
+    for (int k = 0; k < njobs; ++k) {
+        const anc_job& j = jobs[k];
+        const size_t c = size_t(j.nchains) * 8;
+        fetch(j.trace, at[k].trace, size_t(j.nchains) * j.tb->S * 4);
+        if (staged) continue;
+        fetch(j.spins, at[k].spins, size_t(j.inst->nw) * j.nchains * 4);
+        fetch(j.sum_sh, at[k].sh, c);
+        fetch(j.sum_bs, at[k].bs, c);
+        fetch(j.flips, at[k].fl, c);
+    }
     if (ce != cudaSuccess) return drain(cuda_fail(ce, "result copy"));
     CK(cudaStreamSynchronize(st));
-    for (int k = 0; k < njobs; ++k) {
+    arena.idle();
+    for (int k = 0; k < njobs && staged; ++k) {
         const anc_job& j = jobs[k];
         const size_t c = size_t(j.nchains) * 8;
         std::memcpy(j.spins, staging.data() + at[k].spins, size_t(j.inst->nw) * j.nchains * 4);
@@ -1756,7 +1793,10 @@ int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
     return ANC_OK;
 }
 
-}  // extern "C"
+}  // namespace
+
+extern "C" int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) { return run_batch_impl(njobs, jobs, o, true); }
+
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Allocation-free batch entry point (anc_run_batch_noalloc). Its scratch lives in one file-scope device array, and

@@ -1,7 +1,9 @@
-"""GPU: calls under AUTO with little device memory left. An engine that needs operands and workspaces gives way to one that
-needs none."""
+"""GPU: calls under AUTO and sparse batches with little device memory left, and a batch whose results are large. An engine that
+needs operands and workspaces gives way to one that needs none, and memory that the library keeps between batches is given back
+before a call is refused for want of it."""
 import contextlib
 import ctypes as C
+import gc
 
 import numpy as np
 import pytest
@@ -48,3 +50,44 @@ def test_auto_without_room_for_operands(cuda, n, K, chains):
     assert r.kernel == "plain"
     assert np.array_equal(r.spins, want.spins) and np.array_equal(r.spins, plain.spins)
     assert A.run(dev, tb, 3, 0, chains).kernel == want.kernel         # with room again, the quicker kernel
+
+
+def test_kept_batch_memory_is_given_back(cuda):
+    """A batch leaves a block of 160 MB for the next; a larger one fits only where that block was."""
+    dev = A.DeviceInstance(I.torus(10, 20, 3))
+    tb = A.Tables.from_schedule(A.Schedule(S=2000, t0=6.0, t1=0.5, q=1.5, kappa=2.0))
+    small = dict(dev=dev, tb=tb, seed=1, trial_offset=0, nchains=20000, trace=True)       # 8 KB of trace an anneal
+    large = dict(small, nchains=30000)
+    gc.collect()                             # no block is kept but this one's
+    first = A.run_batch([small])[0]
+    with _free_left(150 * MB):
+        r = A.run_batch([large])[0]
+    want = A.run_batch([large])[0]
+    assert np.array_equal(r.trace, want.trace) and np.array_equal(r.spins, want.spins)
+    assert np.array_equal(first.trace, want.trace[:20000])
+
+
+def test_batch_without_room_for_groups(cuda):
+    """Groups of replicas keep their fields in device memory (two classes here, 29 and 38 MB); without room none are formed."""
+    gc.collect()                             # the last instance takes the block kept for batches with it
+    insts = [I.random_graph(3000, 15000, True, 1), I.random_graph(7900, 40000, True, 2)]
+    tb = A.Tables.from_schedule(A.Schedule(S=20, t0=6.0, t1=0.5, q=1.5, kappa=2.0))
+    want = [A.run(A.DeviceInstance(i), tb, 4, 5000 * k, 1300) for k, i in enumerate(insts)]
+    jobs = [dict(dev=A.DeviceInstance(i), tb=tb, seed=4, trial_offset=5000 * k, nchains=1300) for k, i in enumerate(insts)]
+    with _free_left(24 * MB):
+        outs = [A.run_batch(jobs) for _ in range(2)]
+    for got in outs:
+        for a, b in zip(got, want):
+            assert np.array_equal(a.spins, b.spins) and np.array_equal(a.flips, b.flips) and np.array_equal(a.sum_sh, b.sum_sh)
+
+
+def test_results_above_the_staged_size(cuda):
+    """27000 anneals of 20000 spins return 69 MB, which go straight to the caller's arrays; their halves are staged."""
+    dev = A.DeviceInstance(I.torus(100, 200, 4, bmax=2))
+    tb = A.Tables.from_schedule(A.Schedule(S=2, t0=6.0, t1=0.5, q=1.5, kappa=2.0))
+    job = dict(dev=dev, tb=tb, seed=1, trial_offset=0, nchains=27000, trace=True)
+    whole = A.run_batch([job])[0]
+    for a in (0, 13500):
+        half = A.run_batch([dict(job, trial_offset=a, nchains=13500)])[0]
+        for name in ("spins", "sum_sh", "sum_bs", "flips", "trace"):
+            assert np.array_equal(getattr(whole, name)[a:a + 13500], getattr(half, name)), name
