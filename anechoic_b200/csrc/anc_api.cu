@@ -240,7 +240,7 @@ struct anc_instance {
     DevBuf<long long> w_prof;                     // tensor-engine phase counters (opt-in)
     DevBuf<int> w_err;                            // cluster engine's error word
     bool cluster_err_pending = false;             // a cluster launch's error word is still to be read
-    int prof_ctas = 0, prof_S = 0;
+    int prof_ctas = 0, prof_S = 0, prof_clusters = 0;
     // CSR pass variant chosen by the tuner (-1: not tuned yet) and its probe's device time per step of each variant
     int sparse_variant = -1;
     double sparse_probe_us[anc::kSparseVariants] = {};
@@ -700,9 +700,13 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
         r.prof = nullptr;
         I->prof_ctas = 0;
         if (o && o->profile) {
-            anc::TensorGeometry geo;
-            if (anc::tensor_geometry(I->n, nchains, &geo) != 0) return fail(ANC_ECUDA, "tensor geometry query failed");
-            const int ctas = std::max(geo.ctas, anc::planes_max_ctas());
+            int ctas = anc::planes_max_ctas();
+            anc::TensorGeometry geo{};
+            if (!planes && !fp4) {
+                if (anc::tensor_geometry(I->n, nchains, &geo) != 0) return fail(ANC_ECUDA, "tensor geometry query failed");
+                ctas = geo.ctas;
+            }
+            I->prof_clusters = planes || fp4 ? ctas : geo.max_active_clusters;
             CK(I->w_prof.ensure(size_t(ctas) * anc::kTensorProfSlots));
             CK(cudaMemsetAsync(I->w_prof.p, 0, size_t(ctas) * anc::kTensorProfSlots * sizeof(long long), st));
             r.prof = I->w_prof.p;
@@ -717,6 +721,7 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
         if (planes || fp4) {
             I->tensor.last_ctas = I->planes4.last_ctas;     // the profile's geometry fields
             I->tensor.last_cluster = 1;
+            if (r.prof) I->prof_ctas = I->planes4.last_ctas;
         }
         g_last_kernel = planes ? ANC_KERNEL_TENSOR_PLANES : fp4 ? ANC_KERNEL_TENSOR_FP4 : ANC_KERNEL_TENSOR_INT8;
         return ANC_OK;
@@ -976,11 +981,9 @@ int run_host_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, 
             for (int b = 0; b < I->prof_ctas; ++b) acc += double(h[size_t(b) * ns + s]);
             g_prof[slot_of[s]] = acc / I->prof_ctas / std::max(1, I->prof_S);
         }
-        anc::TensorGeometry geo;
-        anc::tensor_geometry(I->n, nchains, &geo);
         g_prof[9] = I->tensor.last_ctas;
         g_prof[10] = I->tensor.last_cluster;
-        g_prof[11] = geo.max_active_clusters;
+        g_prof[11] = I->prof_clusters;
         I->prof_ctas = 0;
     }
     float ms = 0.f;
