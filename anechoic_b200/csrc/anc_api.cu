@@ -433,7 +433,7 @@ int plain_residency(const anc_instance* I, int P, size_t* smem, bool* stream, in
 constexpr int kKinds[4] = {0, 1, 2, 4};     // CSR, then dense K = 1 / 2 / 4
 int kind_index(int K) { return K == 0 ? 0 : K == 1 ? 1 : K == 2 ? 2 : 3; }
 struct KindPlan {
-    int np_max = 0, np_min = 0, nwj_max = 0, P = 0, per_sm = 0;
+    int np_max = 0, np_min = 0, nwj_max = 0, P = 0, per_sm = 0;   // np_min: sparse classes of a batch
     size_t smem = 0;
     bool stream = false;
 };
@@ -470,6 +470,12 @@ bool ensure_group_fields(anc_instance* I, cudaStream_t st) {
     return false;
 }
 
+// The form of a sparse launch of nchains anneals.
+anc::SparseForm single_form(const anc_instance* I, int nchains, bool csr16, bool slices, int per_sm) {
+    const double degree = row_degree(I);
+    return anc::sparse_form(I->np, degree, csr16 ? degree / 2 : degree, nchains, slices, per_sm, I->sms);
+}
+
 // One launch of the one-CTA plain engine; variant >= 0 forces the CSR pass variant (sparse instances) or the dense
 // pass variant (dense instances), else the tuned one.
 int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t st, int variant = -1) {
@@ -489,8 +495,10 @@ int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t 
     if (rc) return rc;
     if (I->K == 0) {
         L.sparse_variant = variant >= 0 ? variant : std::max(0, I->sparse_variant);
-        if (job.slices && anc::sparse_groups(I->np, row_degree(I), job.ntrials, I->sms) && ensure_group_fields(I, st)) {
-            L.groups = 1;
+        L.form = single_form(I, job.ntrials, job.csr16, job.slices != nullptr, per_sm);
+        if (L.form == anc::kSparseGroups && !ensure_group_fields(I, st))
+            L.form = single_form(I, job.ntrials, job.csr16, false, per_sm);
+        if (L.form == anc::kSparseGroups) {
             L.clamp = job.hclamp > 0;
             L.nitems = (job.ntrials + anc::kGroupReplicas - 1) / anc::kGroupReplicas;
             L.group_h = I->w_group.p;
@@ -1527,9 +1535,11 @@ int run_batch_impl(int njobs, const anc_job* jobs, const anc_run_opts* o, bool g
     for (int k = 0; k < njobs; ++k)
         if (jobs[k].inst->K == 0) sparse_anneals += jobs[k].nchains;
     auto sparse_class = [&](const anc_instance* I) {
-        const bool group = groups && I->slices && anc::sparse_groups(I->np, std::max(8.0, row_degree(I)), sparse_anneals, sms);
         // few anneals: one launch, one anneal at a time per SM
         if (sparse_anneals <= anc::kBatchAlone * sms) return 3;
+        // beside others an instance's last wave of groups is not left alone (njobs > 1)
+        const bool group = groups && I->slices &&
+                           (njobs > 1 || anc::sparse_groups(I->np, std::max(8.0, row_degree(I)), sparse_anneals, sms));
         return (group ? 0 : 3) + (I->np <= 2304 ? 0 : I->np <= 9216 ? 1 : 2);
     };
     KindPlan sparse_plans[kClasses];
@@ -1682,11 +1692,10 @@ int run_batch_impl(int njobs, const anc_job* jobs, const anc_run_opts* o, bool g
             L.next_item = counters + 4 + ci;
             L.np_max = kp.np_max;
             L.nwj_max = kp.np_max / 32;
-            L.np_min = kp.np_min;
-            L.groups = ci < 3;
+            L.form = ci < 3 ? anc::kSparseGroups : anc::sparse_batch_form(kp.np_max, kp.np_min, L.nitems, kp.per_sm, sms);
             for (const Prepared& p : prep)
                 L.clamp = L.clamp || (p.hclamp > 0 && jobs[p.idx].inst->K == 0 && sparse_class(jobs[p.idx].inst) == ci);
-            L.group_h = L.groups ? reinterpret_cast<int32_t*>(arena.p + group_at[ci]) : nullptr;
+            L.group_h = ci < 3 ? reinterpret_cast<int32_t*>(arena.p + group_at[ci]) : nullptr;
             if (e == cudaSuccess) e = cudaMemsetAsync(L.next_item, 0, sizeof(int), cst);
             if (e != cudaSuccess) return cuda_fail(e, "sparse launch");
             const int rc = anc::sparse_launch(L, kp.per_sm, sms, cst);
@@ -1946,6 +1955,7 @@ extern "C" int anc_run_batch_noalloc(int njobs, const anc_device_job* jobs, void
         L.np_max = kp.np_max;
         L.nwj_max = kp.nwj_max;
         L.stream = kp.stream ? 1 : 0;
+        if (K == 0) L.form = anc::sparse_batch_form(kp.np_max, 0, cnt, kp.per_sm, sms);
         const int rc = K == 0 ? anc::sparse_launch(L, kp.per_sm, sms, st)
                               : anc::plain_launch(L, K, kp.P, std::max(1, std::min(cnt, kp.per_sm * sms)), kp.smem, st);
         if (rc) return cuda_fail(cudaError_t(rc), "plain engine launch");

@@ -76,10 +76,19 @@ struct PlainLaunch {
     int stream;                        // 1: dense counts go into the fields set by set (one result buffer)
     int sparse_variant;                // CSR pass variant (kSparseVariants index; 0 = rows 1 x edges 8 per lane)
     int dense_variant;                 // dense pass variant (dense_variants(K) of them; 0 = the default)
-    int np_min;                        // sparse batches: the smallest job's np
-    int groups;                        // sparse: items are groups of kGroupReplicas trials, every job has slices
+    int form;                          // sparse: SparseForm
     int clamp;                         // sparse groups: some job of this launch has hclamp > 0
     int32_t* group_h;                  // sparse_group_scratch words
+};
+
+// Forms of the sparse launch (sparse_engine.cu).
+enum SparseForm : int {
+    kSparseOne,       // one CTA of 512 threads per SM
+    kSparseWide,      // one CTA of 1024 threads per SM
+    kSparseHalf,      // two CTAs of 512 threads per SM, draws made ahead as in the wide form
+    kSparseNarrow,    // several CTAs of 256 threads per SM
+    kSparseGroups,    // items are groups of kGroupReplicas trials; every job has slices
+    kSparseForms
 };
 
 constexpr uint32_t kEdgePad = 0x7fe0;  // slots of csr16 rows lie below; a skip edge has all of its bits
@@ -127,11 +136,15 @@ inline size_t plain_smem_plan(int np_max, int nwj_max, int K, int P, bool* strea
 }
 
 // Host launchers; they return a cudaError_t value. Sparse jobs (K = 0, sparse_engine.cu): co-resident CTAs per SM of the
-// several-anneals-per-SM form, and the launch, which runs one anneal per SM when the anneals are no more than the SMs.
+// narrow form, and the launch in the form L.form.
 int sparse_max_blocks_per_sm(int np_max, int* out);
 int sparse_launch(const PlainLaunch& L, int per_sm, int sms, cudaStream_t stream);
 size_t sparse_group_scratch(int np_max, int nitems, int sms);   // words of L.group_h
-bool sparse_groups(int np, double degree, int64_t anneals, int sms);   // whether a launch of so many anneals runs in groups
+// Whether anneals of an instance with slices and this many edges per row run in groups, the form of a launch of one instance
+// (slices: it may run in groups; words: fetched per row), and that of a batch's class of other than groups.
+bool sparse_groups(int np, double degree, int64_t anneals, int sms);
+SparseForm sparse_form(int np, double degree, double words, int anneals, bool slices, int per_sm, int sms);
+SparseForm sparse_batch_form(int np_max, int np_min, int nitems, int per_sm, int sms);
 // Dense jobs (plain_engine.cu)
 int plain_launch(const PlainLaunch& L, int K, int P, int grid, size_t smem, cudaStream_t stream);
 int plain_max_blocks_per_sm(int K, int P, size_t smem, int* out, bool stream = false);

@@ -2,15 +2,16 @@
 // and queue structures and the reference lines), in four forms. A step is a chain of dependent phases, so what bounds a
 // launch depends on how many anneals share an SM (B200, us per step, R = 2000 spins of mean degree 20, phi 0.25):
 //
-// one CTA of 512 threads per SM (plain_kernel, plain_engine.cu): up to one anneal per SM and NP <= 4096. 4.0 for 148.
-// sparse_wide_kernel: one anneal per SM above NP = 4096, or two per SM. 8 warps own the RNG lanes and make the next step's
-//   draws while the others decide the current step's slots, which then need not follow the lanes' rounds. 20000-spin torus:
-//   13.8 for up to 148 anneals (16.1 on the CTA of 512 threads); 296 anneals of R: 5.8 (8.0 in two waves before).
-// sparse_kernel: four or more anneals per SM, 256 threads each, one per RNG lane, at most 64 registers and 6.25 bytes of
-//   shared memory per slot. Every warp keeps its own flip list, so a step takes two CTA barriers. 600 anneals of R: 14.2
-//   (19.7 before); bound by issue slots (72 % busy), most of them in applying edges.
-// sparse_group_kernel: eight replicas of an instance per CTA with pulled, packed updates (below): 2368 anneals of R: 23.2
-//   (63.3 before, 43 in sparse_kernel); it needs unit weights and rows of at most kGroupDegree edges.
+// kSparseOne, one CTA of 512 threads per SM (plain_kernel, plain_engine.cu): up to one anneal per SM and NP <= 4096. 4.0 for 148.
+// kSparseWide and kSparseHalf (sparse_wide_kernel): one CTA of 1024 threads or two of 512. 8 warps own the RNG lanes and make the
+//   next step's draws while the others decide the current step's slots, which then need not follow the lanes' rounds.
+//   20000-spin torus: 13.8 for up to 148 anneals (16.1 on the CTA of 512 threads); 296 anneals of R: 5.8 (8.0 in two waves).
+// kSparseNarrow (sparse_kernel): several anneals per SM, 256 threads each, one per RNG lane, at most 64 registers and 6.25 bytes
+//   of shared memory per slot. Every warp keeps its own flip list, so a step takes two CTA barriers. 600 anneals of R: 14.2
+//   (19.7 in waves of one per SM); bound by issue slots (72 % busy), most of them in applying edges.
+// kSparseGroups (sparse_group_kernel): eight replicas of an instance per CTA with pulled, packed updates (below): 2368 anneals of
+//   R: 23.2 (63.3 in waves of one per SM, 43 in the narrow form); it needs unit weights and rows of at most kGroupDegree edges.
+// sparse_form picks one by the anneals per SM, the size and the row length.
 #include <algorithm>
 
 #include "anc_plain.cuh"
@@ -641,11 +642,11 @@ size_t wide_smem(int np, int tw) {
 }
 
 constexpr size_t kSmemLimit = 224 * 1024;
+bool wide_fits(int np) { return wide_smem(np, 1024) <= kSmemLimit; }
+bool half_fits(int np) { return 2 * (wide_smem(np, 512) + 2048) <= kSmemLimit; }
 size_t group_smem(int np) { return size_t(np + 32) * 2 * kGroupReplicas; }
-int group_ctas(int np, int nitems, int sms) {
-    const int per_sm = int(std::min<size_t>(1024 / kGroupThreads, kSmemLimit / (group_smem(np) + 1024)));
-    return std::min(nitems, per_sm * sms);
-}
+int group_per_sm(int np) { return int(std::min<size_t>(1024 / kGroupThreads, kSmemLimit / (group_smem(np) + 1024))); }
+int group_ctas(int np, int nitems, int sms) { return std::min(nitems, group_per_sm(np) * sms); }
 
 }  // namespace
 
@@ -668,50 +669,85 @@ size_t sparse_group_scratch(int np_max, int nitems, int sms) {
     return size_t(np_max) * kGroupReplicas * group_ctas(np_max, nitems, sms);
 }
 
-// Groups take over where they are the quickest (us per step, groups / sparse_kernel): degree 20, n = 2000: 18.2 / 14.2 for 600
-// anneals, 22.4 / 22.5 for 1200, 23.2 / 43 for 2368; degree 4: 14.6 / 10.2 for 1200, 20.7 / 18.5 for 2400; degree 48, n = 800:
-// 11.0 / 35 for 600 (phi near 1). A batch counts all its anneals and always passes a degree of at least 8: mixed with others
-// the short rows gain too (51 instances: 41 ms, against 46 with the short ones in sparse_kernel).
+// Where groups are the quickest form: from about five or six anneals per SM with long rows, where every CTA has few groups' worth
+// of gathers to hide behind each other, else from eight. us per step, groups / narrow form: degree 20, n = 2000: 21.8 / 18.4 for
+// 900 anneals, 21.9 / 26.3 for 1184, 41 / 44 for 2400; degree 32, n = 2000: 23 / 23 for 740 and 23 / 26 for 900; degree 48,
+// n = 4000: 54 / 51 for 740, 55 / 64 for 1184; degree 4: 14.6 / 10.2 for 1200 at n = 2000. Above NP = 7072 an SM holds one group
+// CTA, so a launch of several waves pays only if the last is nearly full: n = 7900, degree 20: 66 / 81 for 1184 anneals,
+// 129 / 109 for 1600. A batch counts all its anneals and passes a degree of at least 8: mixed with others the short rows gain
+// too (51 instances: 41 ms, against 46 with the short ones in the narrow form).
 bool sparse_groups(int np, double degree, int64_t anneals, int sms) {
-    return np <= kGroupNp && (degree >= 32.0 ? anneals > 2 * sms : degree >= 8.0 && anneals >= 8 * sms);
+    if (np > kGroupNp || degree < 8.0 || anneals < (degree >= 48.0 ? 6 : degree >= 32.0 ? 5 : 8) * int64_t(sms)) return false;
+    const int64_t groups = (anneals + kGroupReplicas - 1) / kGroupReplicas, waves = (groups + sms - 1) / sms;
+    return waves == 1 || group_per_sm(np) > 1 || 10 * groups >= 8 * sms * waves;
+}
+
+// The other forms, us per step, one / wide / half / narrow (B200, phi 0.25; - where it does not fit):
+//   one anneal per SM: the wide form gains above NP = 4096, n = 5500 .. 20000: 14 .. 41 / 11 .. 33 at degree 4;
+//   two: half where two fit (NP <= 10880), n = 2000, degree 20: 8.7 / 8.7 / 6.2 / 9, else wide in two waves: n = 12000,
+//     degree 20: 42 / 34 / - / 45;
+//   three: narrow, n = 10000, degree 20: 54 / 44 / 44 / 42, except that long rows of 32-bit edges make three of its CTAs slower
+//     than two halves while few SMs have three: n = 800, 80 edges, 310 anneals: 15.4 / 16 / 14.6 / 18;
+//   more: narrow where four CTAs fit (NP <= 8448) and rows are short, n = 7900, degree 20, 592 anneals: 58 / 50 / 42 / 40;
+//     with long rows its warps wait for one another's atomics: degree 80, 740 anneals: 134 / 112 / 106 / 138. Three per SM
+//     fill their waves less: n = 10000, degree 20, 592 anneals: 72 / 59 / 53 / 74; n = 12000, degree 32: 109 / 88 / - / 126 and
+//     degree 4: 46 / 42 / - / 43, 1184 anneals 92 / 84 / - / 71. Two per SM never gain on wide: n = 16000, 1184 anneals:
+//     129 / 108 / - / 114 at degree 4, 410 / 334 / - / 495 at degree 80.
+SparseForm sparse_form(int np, double degree, double words, int anneals, bool slices, int per_sm, int sms) {
+    if (slices && sparse_groups(np, degree, anneals, sms)) return kSparseGroups;
+    const bool wide = wide_fits(np), half = half_fits(np);
+    if (wide && np > 4096 && (anneals <= sms || per_sm < 3)) return kSparseWide;
+    if (anneals <= sms || per_sm < 2) return kSparseOne;
+    if (anneals <= 2 * sms) return half ? kSparseHalf : wide ? kSparseWide : kSparseOne;
+    if (anneals <= 3 * sms) return half && words >= 64.0 && 2 * anneals <= 5 * sms ? kSparseHalf : kSparseNarrow;
+    if (per_sm < 4 && half) return degree >= 16.0 ? kSparseHalf : kSparseNarrow;
+    if (per_sm < 4 && wide) return degree >= (anneals <= 5 * sms ? 12.0 : 24.0) ? kSparseWide : kSparseNarrow;
+    return np > 4096 && half && degree >= 48.0 ? kSparseHalf : kSparseNarrow;
+}
+
+// A batch's instances of one class: those of some size alone on their SMs, few anneals one by one (kBatchAlone), many in the
+// narrow form where at least three fit (above).
+SparseForm sparse_batch_form(int np_max, int np_min, int nitems, int per_sm, int sms) {
+    const bool mixed = np_min <= 4096;        // some of the sizes gain from the smaller CTA
+    if (wide_fits(np_max) && np_max > 4096 && !mixed && (nitems <= sms || per_sm < 3)) return kSparseWide;
+    return nitems <= kBatchAlone * sms || per_sm < 3 ? kSparseOne : kSparseNarrow;
 }
 
 int sparse_launch(const PlainLaunch& L, int per_sm, int sms, cudaStream_t st) {
     if (L.np_max / kLanes > 32 * kMaxChunks) return int(cudaErrorInvalidValue);
     const int v = L.sparse_variant;
-    if (L.groups) {
-        SparseFn fn = L.clamp ? group_fn<true>(v) : group_fn<false>(v);
-        const size_t smem = group_smem(L.np_max);
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return int(e);
-        fn<<<group_ctas(L.np_max, L.nitems, sms), kGroupThreads, smem, st>>>(L);
-        return int(cudaGetLastError());
-    }
     SparseFn fn = nullptr;
     int grid = L.nitems, threads = 0;
     size_t smem = 0;
-    const bool wide = wide_smem(L.np_max, 1024) <= kSmemLimit;
-    const bool mixed = L.items && L.np_min <= 4096;        // a batch of sizes of which some gain from the smaller CTA
-    if (wide && L.np_max > 4096 && !mixed && (L.nitems <= sms || per_sm < 2)) {
-        fn = wide_fn<1024>(v);
-        threads = 1024;
-        smem = wide_smem(L.np_max, threads);
-        grid = std::min(grid, sms);
-    } else if (L.nitems <= sms || per_sm < 2 || (L.items && L.nitems <= kBatchAlone * sms)) {
-        // one CTA of 512 threads per SM (plain_engine.cu)
-        const size_t plain = plain_smem_bytes(L.np_max, L.np_max / 32, 0, 12);
-        return plain_launch(L, 0, 12, std::min(grid, sms), plain, st);
-    } else if (!L.items && L.nitems <= 2 * sms && 2 * (wide_smem(L.np_max, 512) + 2048) <= kSmemLimit) {
-        fn = wide_fn<512>(v);
-        threads = 512;
-        smem = wide_smem(L.np_max, threads);
-    } else {
-        fn = narrow_fn(v);
-        threads = kNarrow;
-        smem = narrow_smem(L.np_max);
-        grid = std::min(grid, per_sm * sms);
+    switch (L.form) {
+        case kSparseGroups:
+            fn = L.clamp ? group_fn<true>(v) : group_fn<false>(v);
+            threads = kGroupThreads;
+            smem = group_smem(L.np_max);
+            grid = group_ctas(L.np_max, L.nitems, sms);
+            break;
+        case kSparseWide:
+            fn = wide_fn<1024>(v);
+            threads = 1024;
+            smem = wide_smem(L.np_max, threads);
+            grid = std::min(grid, sms);
+            break;
+        case kSparseHalf:
+            fn = wide_fn<512>(v);
+            threads = 512;
+            smem = wide_smem(L.np_max, threads);
+            grid = std::min(grid, 2 * sms);
+            break;
+        case kSparseNarrow:
+            fn = narrow_fn(v);
+            threads = kNarrow;
+            smem = narrow_smem(L.np_max);
+            grid = std::min(grid, per_sm * sms);
+            break;
+        default:      // plain_engine.cu
+            return plain_launch(L, 0, 12, std::min(grid, sms), plain_smem_bytes(L.np_max, L.np_max / 32, 0, 12), st);
     }
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return int(e);
     fn<<<grid, threads, smem, st>>>(L);
     return int(cudaGetLastError());
