@@ -241,8 +241,10 @@ struct anc_instance {
     DevBuf<int> w_err;                            // cluster engine's error word
     bool cluster_err_pending = false;             // a cluster launch's error word is still to be read
     int prof_ctas = 0, prof_S = 0, prof_clusters = 0;
-    // CSR pass variant chosen by the tuner (-1: not tuned yet) and its probe's device time per step of each variant
-    int sparse_variant = -1;
+    // CSR pass variant chosen by the tuner for each form of the sparse launch (-1: not tuned yet), the form tuned last (-1: none)
+    // and that probe's device time per step of each variant
+    int sparse_variant[anc::kSparseForms] = {-1, -1, -1, -1, -1};
+    int sparse_tuned = -1;
     double sparse_probe_us[anc::kSparseVariants] = {};
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -477,8 +479,8 @@ anc::SparseForm single_form(const anc_instance* I, int nchains, bool csr16, bool
 }
 
 // One launch of the one-CTA plain engine; variant >= 0 forces the CSR pass variant (sparse instances) or the dense
-// pass variant (dense instances), else the tuned one.
-int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t st, int variant = -1) {
+// pass variant (dense instances), else the tuned one; form >= 0 forces the form of a sparse launch.
+int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t st, int variant = -1, int form = -1) {
     anc::PlainLaunch L{};
     L.job0 = job;
     L.jobs = nullptr;
@@ -494,10 +496,10 @@ int launch_plain_single(anc_instance* I, const anc::PlainJob& job, cudaStream_t 
     int rc = plain_residency(I, P, &smem, &stream, &per_sm);
     if (rc) return rc;
     if (I->K == 0) {
-        L.sparse_variant = variant >= 0 ? variant : std::max(0, I->sparse_variant);
-        L.form = single_form(I, job.ntrials, job.csr16, job.slices != nullptr, per_sm);
+        L.form = form >= 0 ? form : single_form(I, job.ntrials, job.csr16, job.slices != nullptr, per_sm);
         if (L.form == anc::kSparseGroups && !ensure_group_fields(I, st))
             L.form = single_form(I, job.ntrials, job.csr16, false, per_sm);
+        L.sparse_variant = variant >= 0 ? variant : std::max(0, I->sparse_variant[L.form]);
         if (L.form == anc::kSparseGroups) {
             L.clamp = job.hclamp > 0;
             L.nitems = (job.ntrials + anc::kGroupReplicas - 1) / anc::kGroupReplicas;
@@ -784,52 +786,57 @@ int run_device_impl(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off
     return rc;
 }
 
-// Run-time tuner of the CSR pass (the plain engine on sparse instances): on the first synchronous run of an
-// instance, each compiled variant (kSparseVariantShape: rows in flight per lane group x edges per lane) runs the
-// first min(S, 64) steps of min(nchains, one wave) anneals of that run -- after an untimed launch of 8 steps, timed with CUDA
-// events -- and the fastest is kept for every later launch of the instance (device, batch and graph-captured
-// launches included). Every variant computes the same fields; only the time differs. The probes write into the
-// handle's own workspaces, never into the caller's outputs.
+// Run-time tuner of the CSR pass (the plain engine on sparse instances): on an instance's first synchronous run in a form of
+// the sparse launch, each compiled variant (kSparseVariantShape: rows in flight per lane group x edges per lane; in groups the
+// words of a row in flight) runs the first steps of min(nchains, one wave) anneals of that run in that form -- after an
+// untimed launch of 4 steps, timed with CUDA events -- and the fastest is kept for every later launch of the instance in that
+// form (device and graph-captured launches included). 64 steps with one anneal per SM, fewer as more share one (at least 12),
+// so that the probe takes no longer: n = 4000, degree 40, 450 anneals: 3 ms of a first call that 64 steps made 12 ms long. Every
+// variant computes the same fields; only the time differs. The probes write into the handle's own workspaces, never into the
+// caller's outputs.
 int tune_sparse(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, int nchains, const anc_run_opts* o) {
-    if (I->K != 0 || I->sparse_variant >= 0) return ANC_OK;
+    if (I->K != 0) return ANC_OK;
     int32_t hclamp = 0;
     int rc = resolve_clamp(I, tb, o, &hclamp);
     if (rc) return rc;
-    const int P = plain_P(I->np);
     bool stream = false;
     size_t smem = 0;
     int per_sm = 0;
-    rc = plain_residency(I, P, &smem, &stream, &per_sm);
+    rc = plain_residency(I, plain_P(I->np), &smem, &stream, &per_sm);
     if (rc) return rc;
-    int np = std::max(1, std::min(nchains, per_sm * I->sms));
-    // a run in groups is probed in groups
-    if (I->slices && anc::sparse_groups(I->np, row_degree(I), nchains, I->sms))
-        np = std::min(nchains, std::max(np, anc::kGroupReplicas * I->sms));
-    const int Sp = std::min(tb->S, 64);
+    const int edges = o ? o->kernel_variant : 0;          // a forced edge format
+    const bool csr16 = I->csr16 && edges != 1;
+    int form = single_form(I, nchains, csr16, I->slices && !edges, per_sm);
+    if (form == anc::kSparseGroups && !ensure_group_fields(I, I->stream)) form = single_form(I, nchains, csr16, false, per_sm);
+    if (I->sparse_variant[form] >= 0) return ANC_OK;
+    const int np = std::min(nchains, anc::sparse_wave(anc::SparseForm(form), per_sm, I->sms));
+    const int Sp = std::min(tb->S, np <= I->sms ? 64 : std::max(12, 48 * I->sms / np));
     CK(I->w_spins.ensure(size_t(I->nw) * np));
     CK(I->w_sh.ensure(np));
     CK(I->w_bs.ensure(np));
     CK(I->w_fl.ensure(np));
     OutPtrs out{I->w_spins.p, I->w_sh.p, I->w_bs.p, I->w_fl.p, nullptr, nullptr};
     anc::PlainJob job = make_job(I, tb, seed, off, np, hclamp, out);
-    job.tab.S = Sp;
     cudaStream_t st = I->stream;
+    double us[anc::kSparseVariants] = {};
     int best = 0;
     for (int v = 0; v < anc::kSparseVariants; ++v) {
         float ms = 0.f;
         for (int rep = 0; rep < 2; ++rep) {
-            job.tab.S = rep ? Sp : std::min(Sp, 8);       // the first launch loads the kernel and the caches
+            job.tab.S = rep ? Sp : std::min(Sp, 4);       // the first launch loads the kernel and the caches
             CK(cudaEventRecord(I->ev0, st));
-            rc = launch_plain_single(I, job, st, v);
+            rc = launch_plain_single(I, job, st, v, form);
             if (rc) return rc;
             CK(cudaEventRecord(I->ev1, st));
             CK(cudaEventSynchronize(I->ev1));
             CK(cudaEventElapsedTime(&ms, I->ev0, I->ev1));
         }
-        I->sparse_probe_us[v] = 1000.0 * double(ms) / Sp;
-        if (I->sparse_probe_us[v] < I->sparse_probe_us[best]) best = v;
+        us[v] = 1000.0 * double(ms) / Sp;
+        if (us[v] < us[best]) best = v;
     }
-    I->sparse_variant = best;
+    I->sparse_variant[form] = best;
+    I->sparse_tuned = form;
+    std::copy(us, us + anc::kSparseVariants, I->sparse_probe_us);
     return ANC_OK;
 }
 
@@ -1073,7 +1080,7 @@ const char* anc_version(void) { return "anechoic-b200 0.1 (sm_100a)"; }
 double anc_last_device_ms(void) { return g_dev_ms; }
 int anc_sparse_tuning(const anc_instance* I, int* variant, double* probe_us) {
     if (!I) return fail(ANC_EINVAL, "null handle");
-    if (variant) *variant = I->K == 0 ? I->sparse_variant : -1;
+    if (variant) *variant = I->sparse_tuned < 0 ? -1 : I->sparse_variant[I->sparse_tuned];
     if (probe_us)
         for (int v = 0; v < anc::kSparseVariants; ++v) probe_us[v] = I->sparse_probe_us[v];
     return ANC_OK;

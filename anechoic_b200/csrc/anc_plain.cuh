@@ -144,6 +144,7 @@ size_t sparse_group_scratch(int np_max, int nitems, int sms);   // words of L.gr
 // (slices: it may run in groups; words: fetched per row), and that of a batch's class of other than groups.
 bool sparse_groups(int np, double degree, int64_t anneals, int sms);
 SparseForm sparse_form(int np, double degree, double words, int anneals, bool slices, int per_sm, int sms);
+int sparse_wave(SparseForm form, int per_sm, int sms);      // anneals of a wave, as the tuner probes it
 SparseForm sparse_batch_form(int np_max, int np_min, int nitems, int per_sm, int sms);
 // Dense jobs (plain_engine.cu)
 int plain_launch(const PlainLaunch& L, int K, int P, int grid, size_t smem, cudaStream_t stream);

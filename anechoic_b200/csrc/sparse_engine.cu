@@ -705,6 +705,15 @@ SparseForm sparse_form(int np, double degree, double words, int anneals, bool sl
     return np > 4096 && half && degree >= 48.0 ? kSparseHalf : kSparseNarrow;
 }
 
+int sparse_wave(SparseForm form, int per_sm, int sms) {
+    switch (form) {
+        case kSparseHalf: return 2 * sms;
+        case kSparseNarrow: return per_sm * sms;
+        case kSparseGroups: return kGroupReplicas * sms;      // of a CTA per SM
+        default: return sms;
+    }
+}
+
 // A batch's instances of one class: those of some size alone on their SMs, few anneals one by one (kBatchAlone), many in the
 // narrow form where at least three fit (above).
 SparseForm sparse_batch_form(int np_max, int np_min, int nitems, int per_sm, int sms) {

@@ -130,12 +130,14 @@ typedef struct {
 } anc_run_opts;
 
 /* No counterpart in the reference (its kernel geometry is fixed per build by flags, sca_gpu_bias.cu:637-644). The
- * run-time tuner of the plain engine's CSR pass: on an instance's first synchronous run (anc_run / anc_run_fields /
- * anc_run_batch) each compiled variant -- lane groups x edges fetched per lane before any is applied: {1, 8},
- * {1, 4}, {2, 4}, {1, 16} -- runs the first min(S, 64) steps of up to one wave of that run's anneals into the handle's
- * own workspaces (after an untimed launch of 8 steps), and the fastest is used for every later launch of the
- * instance. Writes the chosen variant (-1 = not tuned yet, or not a CSR instance) and probe_us[4], each variant's
- * probe time per step in microseconds (may be NULL). */
+ * run-time tuner of the plain engine's CSR pass. The pass runs in one of five forms, by the anneals per SM, the size and the
+ * row length. On an instance's first synchronous run (anc_run / anc_run_fields) in a form each compiled variant -- lane
+ * groups x edges fetched per lane before any is applied: {1, 8}, {1, 4}, {2, 4}, {1, 16}; in groups of replicas 4, 2, 3 or 6
+ * words of a row in flight -- runs the first min(S, 64) steps (fewer, at least 12, as more anneals share an SM) of up to one
+ * wave of that run's anneals into the handle's own workspaces (after an untimed launch of 4 steps), and the fastest is used for every later launch of the instance
+ * in that form. Writes the variant chosen for the form tuned last (-1 = none yet, or not a CSR instance) and probe_us[4], each
+ * variant's probe time per step there in microseconds (may be NULL). anc_run_batch tunes each composition of a batch as a
+ * whole. */
 ANC_API int anc_sparse_tuning(const anc_instance* inst, int* variant, double* probe_us);
 
 /* No counterpart in the reference (its tile shapes and depths are fixed per build by flags, sca_gpu_bias.cu:637-644).
