@@ -10,6 +10,7 @@
 
 #include "anc_meanfield.cuh"
 #include "anc_ptx.cuh"
+#include "anc_tensor.cuh"
 
 namespace anc {
 
@@ -29,6 +30,7 @@ struct MfContext {
     float* seg_P = nullptr;           // [kMfCheckpoint][64][npad]
     float* pbar = nullptr;            // [3][64][npad] ring of pbar_t
     float* svec = nullptr;            // [3][nch][64] ring of s_t, per 256-column chunk
+    Workspace steps;                  // nbuf and gparts
     float* nbuf = nullptr;            // [S + 1][nch][64] soft counts n_t, per 256-column chunk
     float* gparts = nullptr;          // [S][4][nch][64] per-chunk schedule-gradient sums
     int nbuf_steps = 0;
@@ -873,6 +875,16 @@ __global__ void __launch_bounds__(kTmThreads, 1) mf_tmem_kernel(const __grid_con
     }
 }
 
+// J as int8 [n][n] -> its transpose in BF16, padded with zeros to [npad][npad].
+__global__ void mf_pack_kernel(const int8_t* __restrict__ J, int n, int npad, __nv_bfloat16* __restrict__ out) {
+    __shared__ int8_t tile[32][33];
+    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tx = threadIdx.x;
+    for (int i = threadIdx.y; i < 32; i += 8)
+        tile[i][tx] = x0 + i < n && y0 + tx < n ? J[size_t(x0 + i) * n + y0 + tx] : int8_t(0);
+    __syncthreads();
+    for (int i = threadIdx.y; i < 32; i += 8) out[size_t(y0 + i) * npad + x0 + tx] = __float2bfloat16(float(tile[tx][i]));
+}
+
 // The schedule gradients from mf_tmem_kernel's warp sums, one warp per (step, replica): the halves of the warp hold the chunks
 // of s_t and n_t, then those of sum abar P and sum pbar m_t; the same sums as mf_bwd_kernel's and mf_gsum_kernel's.
 __global__ void mf_gsum_raw_kernel(const float* __restrict__ gparts, const float* __restrict__ nbuf, int S, int nch, float* __restrict__ gsched) {
@@ -990,23 +1002,15 @@ size_t ps_cnt_bytes(int nch) { return size_t(12 * nch + 1) * kCntStride * sizeof
 // 16.8 / 32.7 -> 10.6 / 20.4. J of more chunks does not fit the SMs.
 const PsForm* ps_form(int npad) {
     const int nch = npad / kKC;
-    int dev = 0, sms = 0, coop = 0;
+    int dev = 0, sms = 0, coop = 0, optin = 0;
     if (nch > kTmChunks || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
         return nullptr;
+    // the launch bounds leave each CTA the registers of its SM; 1 KB for the kernels' static shared memory
     const PsForm& f = kPsForms[nch - 1];
-    for (PsKernel kernel : {f.fwd, f.adj}) {
-        const void* k = reinterpret_cast<const void*>(kernel);
-        int per_sm = 0;
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(f.smem)) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kTmThreads, f.smem) != cudaSuccess || per_sm < 1 ||
-            f.grid > sms) {
-            cudaGetLastError();
-            return nullptr;
-        }
-    }
-    return &f;
+    return f.grid <= sms && f.smem + 1024 <= size_t(optin) ? &f : nullptr;
 }
 
 PsArgs ps_args(MfContext* c, int S, const float* beta, const float* q, const float* u, const float* w) {
@@ -1029,26 +1033,30 @@ PsArgs ps_args(MfContext* c, int S, const float* beta, const float* q, const flo
     return a;
 }
 
-int ensure_steps(MfContext* c, int S, std::string* why) {
-    if (S <= c->nbuf_steps) return 0;
-    for (float** p : {&c->nbuf, &c->gparts}) {
-        if (*p) cudaFree(*p);
-        *p = nullptr;
+// Soft counts and gradient sums for S steps of a launch on st, in one block.
+int ensure_steps(MfContext* c, int S, cudaStream_t st, std::string* why) {
+    const int cap = std::max(S, c->nbuf_steps);
+    const size_t nbytes = size_t(cap + 1) * (c->form ? 8 : 1) * nch(c) * kRep * sizeof(float);
+    const size_t gbytes = size_t(cap) * (c->form ? 24 : 4) * nch(c) * kRep * sizeof(float);
+    const cudaError_t e = c->steps.ensure(nbytes + gbytes, st);
+    if (e != cudaSuccess) {
+        if (!c->steps.p) c->nbuf_steps = 0;
+        setup_code(e);
+        return check(e, "cudaMalloc", why) ? 0 : -2;
     }
-    c->nbuf_steps = 0;
-    const size_t nbytes = size_t(S + 1) * (c->form ? 8 : 1) * nch(c) * kRep * sizeof(float);
-    const size_t gbytes = size_t(S) * (c->form ? 24 : 4) * nch(c) * kRep * sizeof(float);
-    if (!check(cudaMalloc(&c->nbuf, nbytes), "cudaMalloc", why) || !check(cudaMemset(c->nbuf, 0, nbytes), "cudaMemset", why) ||
-        !check(cudaStreamSynchronize(nullptr), "cudaMemset", why) ||
-        !check(cudaMalloc(&c->gparts, gbytes), "cudaMalloc", why))
-        return -2;
-    c->nbuf_steps = S;
+    c->nbuf = reinterpret_cast<float*>(c->steps.p);
+    c->gparts = reinterpret_cast<float*>(c->steps.p + nbytes);
+    c->nbuf_steps = cap;
     return 0;
 }
 
 int ps_launch(MfContext* c, PsKernel kernel, PsArgs& a, cudaStream_t st, std::string* why) {
     void* args[] = {&c->mapJ, &a};
-    if (!check(cudaMemsetAsync(c->cnt, 0, ps_cnt_bytes(nch(c)), st), "clear counters", why) ||
+    // a size's kernel is loaded by its first launch, not with every context (3 ms each)
+    if (!check(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(c->form->smem)),
+               "kernel attributes", why) ||
+        !check(cudaMemsetAsync(c->cnt, 0, ps_cnt_bytes(nch(c)), st), "clear counters", why) ||
         !check(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(c->form->grid), dim3(kTmThreads),
                                            args, c->form->smem, st),
                "mean-field steps launch", why))
@@ -1069,15 +1077,6 @@ int mf_create(const int8_t* J, const int32_t* bias, int n, MfContext** out, std:
     c->n = n;
     c->npad = ((n + 255) / 256) * 256;
     const int npad = c->npad;
-    std::vector<__nv_bfloat16> Jh(size_t(npad) * npad, __float2bfloat16(0.f));
-    __nv_bfloat16 as_bf16[256];
-    for (int v = 0; v < 256; ++v) as_bf16[v] = __float2bfloat16(float(int8_t(v)));
-    constexpr int kBlock = 64;                 // the transpose in blocks that stay in the cache
-    for (int x0 = 0; x0 < n; x0 += kBlock)
-        for (int y0 = 0; y0 < n; y0 += kBlock)
-            for (int y = y0; y < std::min(n, y0 + kBlock); ++y)
-                for (int x = x0; x < std::min(n, x0 + kBlock); ++x)
-                    Jh[size_t(y) * npad + x] = as_bf16[uint8_t(J[size_t(x) * n + y])];
     std::vector<float> bh(npad, 0.f);
     if (bias)
         for (int i = 0; i < n; ++i) bh[i] = float(bias[i]);
@@ -1086,9 +1085,7 @@ int mf_create(const int8_t* J, const int32_t* bias, int n, MfContext** out, std:
     const size_t nbuf = c->form ? 2 : 1, kch = npad / kKC;
     const size_t pbytes = kch * plane * sizeof(float);
     const size_t sbytes = 3 * (c->form ? 8 : 1) * kch * kRep * sizeof(float);
-    bool ok = check(cudaMalloc(&c->J, Jh.size() * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
-              check(cudaMemcpy(c->J, Jh.data(), Jh.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice), "upload J",
-                    why) &&
+    bool ok = check(cudaMalloc(&c->J, size_t(npad) * npad * sizeof(__nv_bfloat16)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->bias, npad * sizeof(float)), "cudaMalloc", why) &&
               check(cudaMemcpy(c->bias, bh.data(), npad * sizeof(float), cudaMemcpyHostToDevice), "upload bias", why) &&
               check(cudaMalloc(&c->partial, pbytes), "cudaMalloc", why) &&
@@ -1099,12 +1096,16 @@ int mf_create(const int8_t* J, const int32_t* bias, int n, MfContext** out, std:
               check(cudaMalloc(&c->seg_P, kMfCheckpoint * plane * sizeof(float)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->pbar, 3 * plane * sizeof(float)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->svec, sbytes), "cudaMalloc", why) &&
-              check(cudaMemset(c->partial, 0, pbytes), "cudaMemset", why) &&
-              check(cudaMemset(c->svec, 0, sbytes), "cudaMemset", why) &&
-              check(cudaStreamSynchronize(nullptr), "cudaMemset", why) &&
               check(cudaMalloc(&c->cnt, ps_cnt_bytes(kch)), "cudaMalloc", why) &&
               check(cudaMalloc(&c->err, sizeof(int)), "cudaMalloc", why) &&
               check(cudaMemset(c->err, 0, sizeof(int)), "cudaMemset", why);
+    // J goes up as it is, into `partial` (npad^2 bytes), and is padded and transposed there
+    int8_t* raw = reinterpret_cast<int8_t*>(c->partial);
+    ok = ok && check(cudaMemcpy(raw, J, size_t(n) * n, cudaMemcpyHostToDevice), "upload J", why);
+    if (ok) {
+        mf_pack_kernel<<<dim3(npad / 32, npad / 32), dim3(32, 8)>>>(raw, n, npad, c->J);
+        ok = check(cudaGetLastError(), "pack J", why) && check(cudaStreamSynchronize(nullptr), "pack J", why);
+    }
     if (ok) {
         ok = make_map_2d(&c->mapJ, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c->J, npad, npad, 64, kRows);
         for (int k = 0; k < 3 && ok; ++k)
@@ -1112,7 +1113,7 @@ int mf_create(const int8_t* J, const int32_t* bias, int n, MfContext** out, std:
                  make_map_2d(&c->mapXp[k], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c->xp + k * plane, npad, kRep, 64, kRep);
         if (!ok && why) *why = "cuTensorMapEncodeTiled failed";
     }
-    if (ok)
+    if (ok && !c->form)
         ok = check(cudaFuncSetAttribute(mf_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm_smem())),
                    "GEMM attributes", why) &&
              check(cudaStreamCreateWithFlags(&c->cap, cudaStreamNonBlocking), "capture stream", why);
@@ -1225,8 +1226,8 @@ int backward_body(MfContext* c, int S, const float* beta, const float* q, const 
 }
 
 // Internal buffers for S steps (allocated outside any capture; graphs recorded on older buffers are dropped).
-int ensure_io(MfContext* c, int S, std::string* why) {
-    int rc = ensure_steps(c, S, why);
+int ensure_io(MfContext* c, int S, cudaStream_t st, std::string* why) {
+    int rc = ensure_steps(c, S, st, why);
     if (rc) return rc;
     if (S <= c->io_steps) return 0;
     for (float** p : {&c->sched_i, &c->m0_i, &c->mprev_i, &c->mout_i, &c->gm_i, &c->ckpt_i, &c->gs_i}) {
@@ -1294,7 +1295,7 @@ int mf_forward(MfContext* c, int S, const float* beta, const float* q, const flo
         return -1;
     }
     if (c->form) {
-        int rc = ensure_steps(c, S, why);
+        int rc = ensure_steps(c, S, st, why);
         if (rc) return rc;
         PsArgs a = ps_args(c, S, beta, q, u, w);
         a.m0 = m0;
@@ -1304,7 +1305,7 @@ int mf_forward(MfContext* c, int S, const float* beta, const float* q, const flo
         a.m_out = m_out;
         return ps_launch(c, c->form->fwd, a, st, why);
     }
-    int rc = ensure_io(c, S, why);
+    int rc = ensure_io(c, S, st, why);
     if (rc) return rc;
     const size_t plane = size_t(kRep) * c->npad, nseg = (S + kMfCheckpoint - 1) / kMfCheckpoint;
     rc = ensure_graph(c, &c->fwd_exec, &c->fwd_S, S, [&](cudaStream_t cs) {
@@ -1330,7 +1331,7 @@ int mf_backward(MfContext* c, int S, const float* beta, const float* q, const fl
         return -1;
     }
     if (c->form) {
-        int rc = ensure_steps(c, S, why);
+        int rc = ensure_steps(c, S, st, why);
         if (rc) return rc;
         PsArgs a = ps_args(c, S, beta, q, u, w);
         a.ckpt_in = ckpt;
@@ -1345,7 +1346,7 @@ int mf_backward(MfContext* c, int S, const float* beta, const float* q, const fl
         mf_gsum_raw_kernel<<<(S * kRep + 7) / 8, 256, 0, st>>>(c->gparts, c->nbuf, S, nch(c), gsched);
         return check(cudaGetLastError(), "mean-field gradient sum", why) ? 0 : -2;
     }
-    int rc = ensure_io(c, S, why);
+    int rc = ensure_io(c, S, st, why);
     if (rc) return rc;
     const size_t plane = size_t(kRep) * c->npad, nseg = (S + kMfCheckpoint - 1) / kMfCheckpoint;
     rc = ensure_graph(c, &c->bwd_exec, &c->bwd_S, S, [&](cudaStream_t cs) {
@@ -1401,7 +1402,7 @@ void mf_destroy(MfContext* c) {
     for (void* p : {static_cast<void*>(c->J), static_cast<void*>(c->bias), static_cast<void*>(c->partial),
                     static_cast<void*>(c->mring), static_cast<void*>(c->xm), static_cast<void*>(c->xp),
                     static_cast<void*>(c->seg_m), static_cast<void*>(c->seg_P), static_cast<void*>(c->pbar),
-                    static_cast<void*>(c->svec), static_cast<void*>(c->nbuf), static_cast<void*>(c->gparts),
+                    static_cast<void*>(c->svec),
                     static_cast<void*>(c->cnt), static_cast<void*>(c->err)})
         if (p) cudaFree(p);
     delete c;

@@ -97,3 +97,37 @@ def test_capture_without_workspaces(cuda, case, before):
         g.replay()
         torch.cuda.synchronize()
         assert out.same(ref)
+
+
+def test_meanfield_replay_after_more_steps(cuda):
+    """The relaxation's kernels of up to 3072 spins can be captured after an eager call; a longer call in between moves nothing."""
+    import math
+    from anechoic_b200.meanfield import CHECKPOINT, MeanField, SoftSchedule, initial_magnetisations
+    mf, S = MeanField(I.complete_pm1(900, 4)), 20
+    theta = torch.tensor([20.0, math.log(6.0), 3.0, 0.0, 1.05], dtype=torch.float64)
+    sched = lambda S: torch.stack(list(SoftSchedule(S=S).vectors(theta))).detach().to("cuda", torch.float32).contiguous()
+    s20, s300 = sched(S), sched(300)
+    m0 = mf.pad(initial_magnetisations(900, 64, 1))
+    g = mf.pad(torch.randn((64, 900), generator=torch.Generator().manual_seed(2)))
+    prev = torch.ones_like(m0)
+    want, ck = mf.forward_raw(s20, m0, prev)
+    wg = mf.backward_raw(s20, ck, g)
+    out, gs, ck2 = torch.empty_like(want), torch.empty_like(wg), torch.empty_like(ck)
+    L = _lib.load()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        st = torch.cuda.current_stream().cuda_stream
+        _lib.check(L.anc_mf_forward(mf._h, S, s20.data_ptr(), m0.data_ptr(), prev.data_ptr(), ck2.data_ptr(), out.data_ptr(), st))
+        _lib.check(L.anc_mf_backward(mf._h, S, s20.data_ptr(), ck2.data_ptr(), g.data_ptr(), gs.data_ptr(), st))
+    long_m, long_ck = mf.forward_raw(s300, m0, prev)
+    mf.backward_raw(s300, long_ck, g)
+    assert long_ck.shape[0] == math.ceil(300 / CHECKPOINT)
+    fill = [torch.full((1 << 18,), -1, dtype=torch.int32, device="cuda") for _ in range(64)]
+    for _ in range(2):
+        for x in (out, gs, ck2):
+            x.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and torch.equal(gs, wg) and torch.equal(ck2, ck)
+    assert all(int((f != -1).sum()) == 0 for f in fill)
