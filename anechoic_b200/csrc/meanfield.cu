@@ -36,6 +36,7 @@ struct MfContext {
     int nbuf_steps = 0;
     int* err = nullptr;               // device error word
     const PsForm* form = nullptr;   // the persistent form, null: the launch sequences
+    bool loaded[2] = {false, false};  // its forward and adjoint kernels' attributes are set
     unsigned* cnt = nullptr;          // the persistent form's counters
     uint64_t wait_ns = ptx::kWaitNs;  // limit of each device wait before the kernel gives up (recorded in the graphs)
     CUtensorMap mapJ, mapXm[3], mapXp[3];
@@ -1052,11 +1053,14 @@ int ensure_steps(MfContext* c, int S, cudaStream_t st, std::string* why) {
 
 int ps_launch(MfContext* c, PsKernel kernel, PsArgs& a, cudaStream_t st, std::string* why) {
     void* args[] = {&c->mapJ, &a};
-    // a size's kernel is loaded by its first launch, not with every context (3 ms each)
-    if (!check(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(c->form->smem)),
-               "kernel attributes", why) ||
-        !check(cudaMemsetAsync(c->cnt, 0, ps_cnt_bytes(nch(c)), st), "clear counters", why) ||
+    // a size's kernel is loaded by a context's first launch of it, not with every context (3 ms each)
+    bool& loaded = c->loaded[kernel == c->form->adj];
+    if (!loaded && !check(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(c->form->smem)),
+                          "kernel attributes", why))
+        return -2;
+    loaded = true;
+    if (!check(cudaMemsetAsync(c->cnt, 0, ps_cnt_bytes(nch(c)), st), "clear counters", why) ||
         !check(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(c->form->grid), dim3(kTmThreads),
                                            args, c->form->smem, st),
                "mean-field steps launch", why))
