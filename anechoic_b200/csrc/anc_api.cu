@@ -607,10 +607,10 @@ int pick_engine(anc_instance* I, anc_tables* tb, int nchains, const anc_run_opts
     if ((free_choice || o->tensor_kind == ANC_TENSOR_PLANES) && planes_candidate(I)) {
         // where the fp4 kernel runs, it is the planes kernel by another name: only its estimate changes
         const bool fp4 = fp4_candidate(I) && (!o || o->tensor_kind != ANC_TENSOR_PLANES);
-        const double step = anc::planes_step_us(I->n, I->info.maxabs, nchains, I->sms);
-        double t = tb->S * std::max(fp4 ? kFp4FloorUs : 0.0, step);
+        const double step = anc::planes_step_us(I->n, I->info.maxabs, nchains, I->sms);    // < 0: too few SMs
+        double t = step < 0 ? -1.0 : tb->S * std::max(fp4 ? kFp4FloorUs : 0.0, step);
         const bool held = best == ANC_ENGINE_PLAIN && phi < kFewFlips;
-        if (fp4 && !held && est[best] >= 0 && tb->S * step + (I->planes4_ready ? 0.0 : kPlanesSetupUs) < est[best])
+        if (fp4 && step >= 0 && !held && est[best] >= 0 && tb->S * step + (I->planes4_ready ? 0.0 : kPlanesSetupUs) < est[best])
             t = tb->S * step;
         if (t >= 0 && (est[ANC_ENGINE_TENSOR] < 0 || t < est[ANC_ENGINE_TENSOR])) {
             est[ANC_ENGINE_TENSOR] = t;
