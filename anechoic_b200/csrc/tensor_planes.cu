@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             dst[8] = clock64() - loop0;
         }
     }
-    cp_async_wait(0);     // no copy may land in shared memory the CTA has released
+    cp_async_wait_all();  // no copy may land in shared memory the CTA has released
     __syncthreads();
     if (warp == kMmaWarp) {
         tc_fence_after();
