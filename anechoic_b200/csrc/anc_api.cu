@@ -157,15 +157,18 @@ int pad_np(int n) { return std::max(2048, ((n + 255) / 256) * 256); }
 //            anneals on 16 CTAs, 1.18 - 1.19 per wave of up to 15 on 8)
 //   tensor   a constant per kernel: the MMA chain and the decisions cost the same whatever flips: fp4 8.1 (8.3 with
 //            more than one replica group per wave), int8 23.3 at NP = 2048, 21.7 and 28.3 at NP = 3072 and 4096,
-//            streaming 99.5 (measured 99.5 at NP = 10240 and 98 at NP = 16384: bound by its step latency, not by
-//            reading J)
+//            streaming 99.5. These are the recorded times that the model is tested against, of which the fp4 and
+//            streaming ones are of kernels since replaced: the planes kernel takes 3.8 .. 6.2 as the fp4 kernel and the
+//            streaming kernel 59.4 or 80 above NP = 8192. pick_engine uses planes_step_us and, up to NP = 8192,
+//            stream_step_us instead.
 // Each engine advances a fixed number of anneals at once (per_wave); a launch of more takes further waves.
 // The fp4 kernel's step is taken as at least kFp4FloorUs unless its own (planes_step_us) saves more than the set-up of its
 // operands where that is still to be done. +-1, phi 0.33, us a step plain / cluster / fp4: n = 500 4.3 / 4.9 / 3.8 for 60 anneals
 // and 4.3 / 8.5 / 4.2 for 100; n = 1100 6.6 / 4.9 / 3.8 and 6.6 / 8.5 / 4.3; n = 2000 10.3 / 4.9 / 3.9 and 10.3 / 8.5 / 4.3; up to
-// 30 anneals the cluster engine has 2.5. Batches that flip few spins (the temperature-scaled schedules, phi about 0.11 at
-// n = 2000) stay on the plain engine where its estimate is the least of the others (5.86 us there): the floor holds below
-// kFewFlips.
+// 30 anneals the cluster engine has 2.5. Below kFewFlips the floor holds where the plain engine's estimate is the least of the
+// others. That is not for speed: 120 anneals of the temperature-scaled schedule at n = 2000 (phi 0.11, estimated at 5.86 us) would
+// take about 4.2 us a step here. The choice of the plain engine for that batch is part of what callers and tests rely on, and
+// the two constants are set so that it stays.
 constexpr double kFp4FloorUs = 5.95, kFewFlips = 0.15;
 constexpr double kPlanesSetupUs = 400.0;   // packing, workspaces and their first touch: 0.3 - 0.5 ms on an instance's first call
 constexpr double kPhiPrior = 0.25;   // flip fraction assumed before any run of these tables on this instance
@@ -579,10 +582,8 @@ int tuned_variant(anc_instance* I, int kernel, int nchains) {
     return it == g_kernel_tune.end() ? 0 : std::max(0, it->second.variant);
 }
 
-// Whether the planes kernel can run this instance, and whether AUTO considers it (not where the fp4 kernel runs).
-bool planes_candidate(const anc_instance* I) {
-    return !I->dense.empty() && anc::planes_supported(I->n, I->info.maxabs, I->info.hmax + int64_t(I->info.bmax));
-}
+// Whether the planes kernel can run this instance.
+bool planes_candidate(const anc_instance* I) { return !I->dense.empty() && anc::planes_supported(I->n, I->info.maxabs); }
 
 // Flip fraction AUTO assumes: the caller's hint, else what the last host-output run of these tables on this instance
 // saw, else the prior.
@@ -1500,7 +1501,8 @@ namespace {
 // anc_run_batch; without `groups` no job runs in groups of replicas, which take device memory for their fields.
 int run_batch_impl(int njobs, const anc_job* jobs, const anc_run_opts* o, bool groups) {
     if (njobs < 1 || !jobs) return fail(ANC_EINVAL, "need jobs");
-    // group by kernel kind (sparse / dense K); each group is one persistent launch with a cost-ordered work queue
+    // group by kernel kind; a dense kind is one persistent launch with a cost-ordered work queue, the sparse kind up to six
+    // (by size and form)
     struct Prepared {
         int idx;
         int32_t hclamp;
@@ -1535,7 +1537,7 @@ int run_batch_impl(int njobs, const anc_job* jobs, const anc_run_opts* o, bool g
         }
     }
     // Sparse jobs run as concurrent launches by size and form: classes 0 .. 2 (NP up to 2304, 9216 and above) in groups of
-    // four replicas, classes 3 .. 5 anneal by anneal, so that the largest instance's shared memory does not set how many of
+    // eight replicas, classes 3 .. 5 anneal by anneal, so that the largest instance's shared memory does not set how many of
     // the smaller ones share an SM.
     constexpr int kClasses = 6;
     int64_t sparse_anneals = 0;

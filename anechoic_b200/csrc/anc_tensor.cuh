@@ -131,8 +131,7 @@ struct PlanesInstance {
     int* last_err = nullptr;     // error word of the last launch
     int last_ctas = 0;
 };
-// field_bound: max_y sum_x |J_xy| + max |b|
-bool planes_supported(int n, int maxabs, int64_t field_bound);
+bool planes_supported(int n, int maxabs);
 // measured device time of one step of nchains anneals (all waves), in microseconds
 double planes_step_us(int n, int maxabs, int nchains, int sms);
 // anneals one wave advances at most

@@ -1000,7 +1000,8 @@ size_t ps_cnt_bytes(int nch) { return size_t(12 * nch + 1) * kCntStride * sizeof
 // The persistent form for npad columns, or null (the launch sequences) beyond twelve chunks or where its CTAs do not all fit,
 // one per SM. Measured, a forward / an adjoint step in us, launch sequences -> persistent: n = 200 8.4 / 15.2 -> 5.8 / 11.2,
 // n = 700 10.0 / 18.7 -> 5.8 / 10.4, n = 2000 9.3 / 19.4 -> 6.0 / 12.4, n = 2500 15.8 / 30.9 -> 10.8 / 20.9, n = 3072
-// 16.8 / 32.7 -> 10.6 / 20.4. J of more chunks does not fit the SMs.
+// 16.8 / 32.7 -> 10.6 / 20.4. With one or two tiles of J per CTA more chunks do not fit one CTA per SM; three would fit 13 and
+// 14 chunks and are not compiled.
 const PsForm* ps_form(int npad) {
     const int nch = npad / kKC;
     int dev = 0, sms = 0, coop = 0, optin = 0;

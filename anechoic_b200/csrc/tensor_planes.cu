@@ -3,8 +3,8 @@
 //
 // Planes. Every |J| in {0, 1, 2, 3, 4, 6} is one e2m1 value; 5 = 4 + 1 and 7 = 6 + 1 take a second plane with entries
 // in {0, +-1}. The field update is J dS = J_0 dS + J_1 dS: the same dS tile multiplied by each plane's slice into the
-// same f32 accumulator (kind::mxf4, unit block scales). Products and partial sums are integers below 2^18 (the host
-// admits max_y sum_x |J_xy| + max |b| < 2^16), so f32 accumulation is exact in any order.
+// same f32 accumulator (kind::mxf4, unit block scales). Products and partial sums are integers below 2^18 (at these sizes
+// max_y sum_x |J_xy| + max |b| < 2^16, planes_supported), so f32 accumulation is exact in any order.
 //
 // Layout. RP = rounds padded to a multiple of 4 (columns k >= R of a lane are never decided and have zero couplings);
 // slot i = k*256 + l sits at permuted column p = l*RP + k, so a lane's slots are contiguous. CTA cs of a replica group
@@ -755,10 +755,10 @@ int planes_of(int maxabs) { return maxabs <= 4 ? 1 : 2; }
 
 }  // namespace
 
-// One plane holds |J| <= 4; two hold |J| <= 7. The field bound keeps every f32 partial sum an exact integer.
-bool planes_supported(int n, int maxabs, int64_t field_bound) {
-    return maxabs <= 7 && field_bound < (int64_t(1) << 16) &&
-           planes_config(rounds_of(n), planes_of(maxabs), 1, 128) != nullptr;
+// One plane holds |J| <= 4; two hold |J| <= 7. The sizes keep every field below 2^16, and so every f32 partial sum an exact
+// integer, whatever the instance: with the largest accepted bias, 6144 * 4 + 32767 = 57343 and 4096 * 7 + 32767 = 61439.
+bool planes_supported(int n, int maxabs) {
+    return maxabs <= 7 && planes_config(rounds_of(n), planes_of(maxabs), 1, 128) != nullptr;
 }
 
 double planes_step_us(int n, int maxabs, int nchains, int sms) {

@@ -8,7 +8,7 @@ Reference counterparts (paths relative to the reference project root):
 * ``run_trial`` / ``run_trial_bias`` -- sca::run_trial / sca::run_trial_bias (sca_ref.hpp:101-155,
   sca_ref_bias.hpp:25-75): the same arguments and results, computed on the GPU.
 * ``run`` -- one launch of sca_gpu / sca_gpu_bias over ``nchains`` trial ids (sca_gpu.cu:699-713).
-* ``run_batch`` -- many (instance, schedule) jobs in one persistent launch.
+* ``run_batch`` -- many (instance, schedule) jobs of uneven size in one call.
 * ``range_plan`` -- host::plan_ranges (gpu/multibit_bias_20261008/src/sca_gpu_bias.cu:543-557).
 
 Errors raise ``AncError`` (the reference prints ``FAIL: ...`` and exits 1). Nothing here falls back to the CPU.
@@ -193,7 +193,7 @@ class RunResult:
     fields: Optional[np.ndarray] = None
     device_ms: float = 0.0
     profile: Optional[dict] = None
-    kernel: Optional[str] = None     # "plain", "plain-cluster", "tensor-int8" or "tensor-fp4"
+    kernel: Optional[str] = None     # "plain", "plain-cluster", "tensor-int8", "tensor-fp4" or "tensor-planes"
 
     def cuts(self, sumw: int) -> np.ndarray:
         """Device cut = (sumw + sum_sh / 2) / 2 with C++ truncating division (sca_ref.hpp:153)."""
@@ -218,7 +218,7 @@ def run(dev: DeviceInstance, tb: Tables, seed: int, trial_offset: int, nchains: 
     "tensor" (replicas sharing J). "auto" runs the engine with the least estimated device time (auto_estimate);
     flip_fraction (flips per spin per step) overrides the fraction it assumes, which is otherwise what the last run
     of these tables on this instance saw. profile=True records the tensor engine's per-phase cycle counters
-    (RunResult.profile); tensor_kind picks the tensor engine's operand format ("auto", "int8", "fp4")."""
+    (RunResult.profile); tensor_kind picks the tensor engine's operand format ("auto", "int8", "fp4", "planes")."""
     L = load()
     n = dev.n
     W = spin_words(n)
@@ -275,8 +275,8 @@ def auto_choice(dev: DeviceInstance, tb: Tables, nchains: int, flip_fraction: Op
 
 
 def run_batch(jobs: List[dict], engine: str = "auto", wide="auto") -> List[RunResult]:
-    """Many jobs in one persistent launch; each job is dict(dev=DeviceInstance, tb=Tables, seed, trial_offset, nchains,
-    trace=False). Returns one RunResult per job."""
+    """Many jobs in one call (persistent launches with work queues); each job is dict(dev=DeviceInstance, tb=Tables, seed,
+    trial_offset, nchains, trace=False). Returns one RunResult per job."""
     L = load()
     arr = (_lib.Job * len(jobs))()
     outs = []

@@ -44,7 +44,7 @@ extern "C" {
 
 #define ANC_TENSOR_AUTO 0   /* fp4 when exact for the instance (NP = 2048, |J| <= 1, small fields), else int8 */
 #define ANC_TENSOR_PLANES 3 /* kind::mxf4 with J as one or two e2m1 planes kept in shared memory (|J| <= 4: n <= 6144;
-                              |J| <= 7: n <= 4096; max_y sum_x |J_xy| + max |b| < 2^16, EINVAL otherwise); exact.
+                              |J| <= 7: n <= 4096; EINVAL otherwise); exact, since fields stay below 2^16 there.
                               ANC_ENGINE_AUTO picks it where it is estimated fastest; ANC_ENGINE_TENSOR runs it only
                               when this kind is asked for */
 #define ANC_TENSOR_INT8 1   /* tcgen05.mma kind::i8, int32 accumulation (any K) */
@@ -205,7 +205,9 @@ ANC_API int anc_run_device(anc_instance* inst, anc_tables* tb, uint64_t seed, ui
                    const anc_run_opts* opts, uint64_t* d_spins, int64_t* d_sum_sh, int64_t* d_sum_bs,
                    int64_t* d_flips, int32_t* d_trace, void* stream);
 
-/* Many instances / schedules in ONE persistent launch (work queue, uneven sizes). */
+/* Many instances / schedules in one call: a persistent launch with a work queue per dense kernel kind, and up to six
+ * concurrent ones, by size and form, for the sparse jobs. The call's device memory, up to 256 MB per device, is kept for
+ * the next call; it is freed with the last instance, or when a batch finds no room beside it. */
 typedef struct {
     anc_instance* inst;
     anc_tables* tb;
