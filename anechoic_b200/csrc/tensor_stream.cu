@@ -13,7 +13,8 @@
 //     n_lin partials (256 bytes per replica: 2 per slice).
 //   1 MMA warp: per dS chunk, 4 x 2 tcgen05.mma kind::i8 (M 128 replicas, N 2 RP columns, K 32) into each group's
 //     int32 field accumulator; per n_lin chunk 4 x 2 i8 MMAs against a ones row into the n_lin accumulators.
-// Every wait is bounded (2 s); on expiry the kernel records an error code and skips the remaining work.
+// Every wait is bounded (the wait limit, 2 s by default); on expiry the kernel records an error code, skips the remaining work
+// and waits for what it has in flight.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -71,6 +72,7 @@ struct StreamParams {
     int32_t* out_trace;
     int32_t* out_h;
     int* err;
+    uint64_t wait_ns;                   // limit of each wait
     long long* prof;
 };
 
@@ -86,8 +88,9 @@ __global__ void __launch_bounds__(kSThreads, 1)
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* stages = smem;                                 // kSStages x (dS0, dS1, J)
     uint8_t* ones = stages + kSStages * kSStage;            // 2 KB: row 0 = 128 x int8(1)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(ones + 2048);   // full[4], empty[4], hready, init, fields read
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSStages + 3);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ones + 2048);   // full[4], empty[4], hready, init, fields read, drain
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSStages + 4);
+    __shared__ uint32_t s_issued[kSStages];                 // chunks issued to each stage
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cs = int(blockIdx.x);
@@ -98,16 +101,18 @@ __global__ void __launch_bounds__(kSThreads, 1)
     const uint32_t bar_init = smem_u32(bars + 2 * kSStages + 1);   // decision warps: fields of a new pair set
     // decision warps: the fields of step m have been read, so step m's tiles may now be accumulated (other slices
     // can publish step m before this CTA has read the fields it decides step m from)
-    const uint32_t bar_rd = smem_u32(bars + 2 * kSStages + 2);
+    const uint32_t bar_rd = smem_u32(bars + 2 * kSStages + 2), bar_fin = smem_u32(bars + 2 * kSStages + 3);
 
     if (tid == 0) {
         for (int s = 0; s < kSStages; ++s) {
             mbar_init(bar_full + 8 * s, 1);
             mbar_init(bar_empty + 8 * s, 1);
+            s_issued[s] = 0u;
         }
         mbar_init(bar_h, 1);
         mbar_init(bar_init, 1);
         mbar_init(bar_rd, 1);
+        mbar_init(bar_fin, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < 2048; i += blockDim.x) ones[i] = i < 128 ? 1 : 0;
@@ -206,7 +211,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 const int t = m < S ? m : S - 1;
                 const int32_t fourT = __ldg(P.fourT + t), qv = __ldg(P.q + t), kconst = __ldg(P.kconst + t);
                 const int64_t kcorr = __ldg(P.kcorr + t);
-                if (!err_set(err)) mbar_wait(bar_h, hph & 1u, err, kErrHready);
+                if (!err_set(err)) mbar_wait_for(bar_h, hph & 1u, err, kErrHready, P.wait_ns);
                 ++hph;
                 tc_fence_after();
                 if (prof) { const long long t1 = clock64(); pa += t1 - t0; t0 = t1; }
@@ -330,7 +335,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                     const uint32_t u = q / kSStages;
                     const long long w0 = prof ? clock64() : 0;
                     if (u >= 1) {
-                        const int w = lane == 0 ? (mbar_wait(bar_empty + 8 * s, (u - 1) & 1u, err, kErrEmpty) ? 1 : 0) : 1;
+                        const int w = lane == 0 ? (mbar_wait_for(bar_empty + 8 * s, (u - 1) & 1u, err, kErrEmpty, P.wait_ns) ? 1 : 0) : 1;
                         if (!__shfl_sync(0xffffffffu, w, 0)) continue;
                     }
                     uint8_t* st_base = stages + size_t(s) * kSStage;
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(fl + 32 * wdw + lane) : "memory");
                             ready[wdw] = __ballot_sync(0xffffffffu, v >= target);
                             if ((ready[wdw] & need) == need) { ok = true; break; }
-                            if ((k & 63u) == 0 && __shfl_sync(0xffffffffu, globaltimer() - t0 > kWaitNs, 0)) {
+                            if (((k & 63u) == 0 || P.wait_ns == 0) && __shfl_sync(0xffffffffu, globaltimer() - t0 >= P.wait_ns, 0)) {
                                 if (lane == 0) atomicCAS(err, 0, kErrFlag);
                                 break;
                             }
@@ -375,6 +380,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                             tma_load_2d(smem_u32(st_base), &mapNL, x, ay0, bar_full + 8 * s);
                             tma_load_2d(smem_u32(st_base + kSTile), &mapNL, x, ay1, bar_full + 8 * s);
                         }
+                        atomicMax(&s_issued[s], u + 1);
                     }
                     __syncwarp();
                 }
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
         } else if (warp == kSMmaWarp) {
             // ---------------- MMA warp: converged, one elected lane issues (as a loop run by one lane, an MMA takes about
             // 80 cycles to issue: its operands move to uniform registers one by one) ----------------
-            const bool iok = !err_set(err) && mbar_wait(bar_init, uint32_t(pr) & 1u, err, kErrInit);
+            const bool iok = !err_set(err) && mbar_wait_for(bar_init, uint32_t(pr) & 1u, err, kErrInit, P.wait_ns);
             (void)__all_sync(0xffffffffu, iok);
             tc_fence_after();
             const uint32_t utmem = __shfl_sync(0xffffffffu, tmem, 0);
@@ -393,7 +399,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 const long long t0 = prof ? clock64() : 0;
                 bool ok = __all_sync(0xffffffffu, !err_set(err));
                 if (m >= 0) {
-                    ok = ok && __all_sync(0xffffffffu, mbar_wait(bar_rd, rph & 1u, err, kErrRead));
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait_for(bar_rd, rph & 1u, err, kErrRead, P.wait_ns));
                     ++rph;
                     tc_fence_after();
                 }
@@ -401,7 +407,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 for (int c = 0; c < kSChunks; ++c, ++q) {
                     const uint32_t s = q % kSStages;
                     const long long w0 = prof ? clock64() : 0;
-                    ok = ok && __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, (q / kSStages) & 1u, err, kErrFull));
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait_for(bar_full + 8 * s, (q / kSStages) & 1u, err, kErrFull, P.wait_ns));
                     if (prof) pa += clock64() - w0;
                     tc_fence_after();
                     if (lead) {
@@ -421,7 +427,8 @@ __global__ void __launch_bounds__(kSThreads, 1)
                                 mma_i8(utmem + 272u, d0 + uint64_t(kSTile >> 4), bo + uint64_t(2 * kk), IDESC_NL, 1u);
                             }
                         }
-                        mma_commit(bar_empty + 8 * s);
+                        // a stage is free again only once its copies were seen: none is issued on top of one in flight
+                        if (ok) mma_commit(bar_empty + 8 * s);
                     }
                     __syncwarp();
                 }
@@ -438,8 +445,14 @@ __global__ void __launch_bounds__(kSThreads, 1)
         if (warp == kSMmaWarp && lane == 0) { dst[5] = pa; dst[6] = pb; dst[8] = clock64() - t_loop0; }
         if (warp == kSDW && lane == 0) dst[7] = pa;
     }
-    // on the normal path every copy has landed before the MMA thread's last wait and every MMA has completed before
-    // the decision warps' last wait on bar_h; the barrier orders the TMEM dealloc after both
+    // Before shared memory and TMEM go away every copy issued has landed and every MMA has completed, also where a wait gave up.
+    // A stage's last copies are those of its phase s_issued - 1: a phase is issued only once the one before was consumed.
+    if (warp == kSMmaWarp && elect_one()) {
+        mma_commit(bar_fin);
+        mbar_wait_for(bar_fin, 0u, nullptr, 0, kWaitNs);
+    }
+    __syncthreads();
+    if (tid < kSStages && s_issued[tid] > 0) mbar_wait_for(bar_full + 8 * tid, (s_issued[tid] - 1) & 1u, nullptr, 0, kWaitNs);
     __syncthreads();
     if (warp == kSMmaWarp) {
         tc_fence_after();
@@ -447,7 +460,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
     }
 }
 
-size_t stream_smem_bytes(uint32_t stage) { return 1024 + size_t(kSStages) * stage + 2048 + (2 * kSStages + 3) * 8 + 16; }
+size_t stream_smem_bytes(uint32_t stage) { return 1024 + size_t(kSStages) * stage + 2048 + (2 * kSStages + 4) * 8 + 16; }
 
 using StreamKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const StreamParams);
 struct StreamConfig {
@@ -610,6 +623,7 @@ int stream_run(TensorInstance* ti, const TensorRun& r, const int32_t* bias_perm,
     P.out_trace = r.out_trace;
     P.out_h = r.out_h;
     P.err = err;
+    P.wait_ns = r.wait_ns;
     P.prof = r.prof;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
