@@ -19,20 +19,31 @@ MB = 1 << 20
 
 @contextlib.contextmanager
 def _free_left(target):
-    """Holds device memory, straight from the driver, so that between `target` and `target` + 2 MB are free."""
+    """Takes device memory straight from the driver until none is left (freed pieces that it holds back included), then gives
+    `target` bytes back."""
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     cuda = C.CDLL("libcuda.so.1")
     held = []
     try:
         for step in (4096 * MB, 256 * MB, 16 * MB, 2 * MB):
-            while torch.cuda.mem_get_info()[0] - step >= target:
+            p = C.c_uint64()
+            while cuda.cuMemAlloc_v2(C.byref(p), C.c_size_t(step)) == 0:
+                held.append((step, p))
                 p = C.c_uint64()
-                assert cuda.cuMemAlloc_v2(C.byref(p), C.c_size_t(step)) == 0
-                held.append(p)
+        given = 0
+        while held and given < target:
+            step, p = held.pop()
+            cuda.cuMemFree_v2(p)
+            given += step
+            while given > target:                    # the part of a large block that is too much
+                p = C.c_uint64()
+                assert cuda.cuMemAlloc_v2(C.byref(p), C.c_size_t(2 * MB)) == 0
+                held.append((2 * MB, p))
+                given -= 2 * MB
         yield
     finally:
-        for p in held:
+        for _, p in held:
             cuda.cuMemFree_v2(p)
 
 
@@ -45,7 +56,7 @@ def test_auto_without_room_for_operands(cuda, n, K, chains):
     assert want.kernel != "plain"
     plain = A.run(A.DeviceInstance(inst), tb, 3, 0, chains, engine="plain")     # its kernels are loaded
     dev = A.DeviceInstance(inst)
-    with _free_left(9 * MB):
+    with _free_left(8 * MB):
         r = A.run(dev, tb, 3, 0, chains)
     assert r.kernel == "plain"
     assert np.array_equal(r.spins, want.spins) and np.array_equal(r.spins, plain.spins)
