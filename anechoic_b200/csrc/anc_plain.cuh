@@ -114,6 +114,16 @@ constexpr int kSparseVariantShape[kSparseVariants][2] = {{1, 8}, {1, 4}, {2, 4},
 constexpr int kDenseVariantsMax = 3;
 inline int dense_variants(int K, bool stream) { return stream ? 1 : K == 1 ? 3 : K == 2 ? 2 : 1; }
 
+// Lets every launch of fn have as much dynamic shared memory as an SM can give. The attribute belongs to the function, so a
+// launch that set it to its own need could find it lowered by another thread's before it is made.
+template <class F>
+inline cudaError_t allow_max_smem(F fn) {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, fn);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - int(a.sharedSizeBytes));
+}
+
 // Shared-memory bytes for a launch (P = counter planes).
 inline size_t plain_smem_bytes(int np_max, int nwj_max, int K, int P, bool stream = false) {
     const size_t C = (K <= 1 || stream) ? 1 : size_t(2 * (K - 1));

@@ -919,7 +919,7 @@ __global__ void __cluster_dims__(CR, 1, 1) __launch_bounds__(cluster_threads(CR)
 template <int K, int P, bool SPARSE, bool STREAM = false, int SB = 1, int SE = 8, int DV = 0>
 int launch_t(const PlainLaunch& L, int grid, size_t smem, cudaStream_t st) {
     auto fn = plain_kernel<K, P, SPARSE, STREAM, SB, SE, DV>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_max_smem(fn);
     if (e != cudaSuccess) return int(e);
     fn<<<grid, T, smem, st>>>(L);
     return int(cudaGetLastError());
@@ -928,7 +928,7 @@ int launch_t(const PlainLaunch& L, int grid, size_t smem, cudaStream_t st) {
 template <int K, int P, bool SPARSE, bool STREAM = false>
 int occ_t(size_t smem, int* out) {
     auto fn = plain_kernel<K, P, SPARSE, STREAM>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_max_smem(fn);
     if (e != cudaSuccess) return int(e);
     return int(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, T, smem));
 }

@@ -655,7 +655,7 @@ int sparse_max_blocks_per_sm(int np_max, int* out) {
     int least = 1 << 30;
     for (int v = 0; v < kSparseVariants; ++v) {
         SparseFn fn = narrow_fn(v);
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(narrow_smem(np_max)));
+        cudaError_t e = allow_max_smem(fn);
         int b = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kNarrow, narrow_smem(np_max));
         if (e != cudaSuccess) return int(e);
@@ -756,7 +756,7 @@ int sparse_launch(const PlainLaunch& L, int per_sm, int sms, cudaStream_t st) {
         default:      // plain_engine.cu
             return plain_launch(L, 0, 12, std::min(grid, sms), plain_smem_bytes(L.np_max, L.np_max / 32, 0, 12), st);
     }
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const cudaError_t e = allow_max_smem(fn);
     if (e != cudaSuccess) return int(e);
     fn<<<grid, threads, smem, st>>>(L);
     return int(cudaGetLastError());
