@@ -11,6 +11,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -50,6 +51,18 @@ int fail(int code, const char* fmt, ...) {
 
 int cuda_fail(cudaError_t e, const char* what) {
     return fail(ANC_ECUDA, "%s: %s", what, cudaGetErrorString(e));
+}
+
+// An entry point's body: a failed host allocation becomes a status, since no C++ exception may cross the ABI.
+template <class F>
+int guarded(F body) {
+    try {
+        return body();
+    } catch (const std::bad_alloc&) {
+        return fail(ANC_ECUDA, "out of host memory");
+    } catch (const std::exception& e) {
+        return fail(ANC_ECUDA, "%s", e.what());
+    }
 }
 
 #define CK(call)                                                   \
@@ -1021,12 +1034,14 @@ struct anc_meanfield {
 
 int anc_mf_create(const int8_t* J, int n, const int32_t* bias, anc_meanfield** out) {
     if (!J || n < 1 || !out) return fail(ANC_EINVAL, "anc_mf_create: J, n >= 1 and out are required");
-    std::string why;
-    anc::MfContext* c = nullptr;
-    const int rc = anc::mf_create(J, bias, n, &c, &why);
-    if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "mean-field setup: %s", why.c_str());
-    *out = new anc_meanfield{c};
-    return ANC_OK;
+    return guarded([&] {
+        std::string why;
+        anc::MfContext* c = nullptr;
+        const int rc = anc::mf_create(J, bias, n, &c, &why);
+        if (rc) return fail(rc == -2 ? ANC_ECUDA : ANC_EINVAL, "mean-field setup: %s", why.c_str());
+        *out = new anc_meanfield{c};
+        return ANC_OK;
+    });
 }
 
 int anc_mf_npad(const anc_meanfield* mf) { return mf && mf->ctx ? anc::mf_npad(mf->ctx) : 0; }
@@ -1127,7 +1142,7 @@ int anc_last_kernel(void) { return g_last_kernel; }
 int anc_np(int n) { return pad_np(n); }
 int anc_spin_words(int n) { return pad_np(n) / 64; }
 
-int anc_instance_create(const int8_t* J, int n, int kbits, const int32_t* bias, anc_instance** out) {
+static int create_dense(const int8_t* J, int n, int kbits, const int32_t* bias, anc_instance** out) {
     if (!out) return fail(ANC_EINVAL, "out is null");
     *out = nullptr;
     if (!J || n < 1 || n > 65536) return fail(ANC_EINVAL, "need J and 1 <= n <= 65536");
@@ -1192,8 +1207,8 @@ int anc_instance_create(const int8_t* J, int n, int kbits, const int32_t* bias, 
     return ANC_OK;
 }
 
-int anc_instance_create_csr(int n, const int32_t* row_ptr, const int32_t* col, const int8_t* val, const int32_t* bias,
-                            anc_instance** out) {
+static int create_csr(int n, const int32_t* row_ptr, const int32_t* col, const int8_t* val, const int32_t* bias,
+                      anc_instance** out) {
     if (!out) return fail(ANC_EINVAL, "out is null");
     *out = nullptr;
     if (!row_ptr || n < 1 || n > (1 << 24)) return fail(ANC_EINVAL, "need row_ptr and 1 <= n < 2^24");
@@ -1332,6 +1347,15 @@ int anc_instance_create_csr(int n, const int32_t* row_ptr, const int32_t* col, c
     }
     *out = I.release();
     return ANC_OK;
+}
+
+int anc_instance_create(const int8_t* J, int n, int kbits, const int32_t* bias, anc_instance** out) {
+    return guarded([&] { return create_dense(J, n, kbits, bias, out); });
+}
+
+int anc_instance_create_csr(int n, const int32_t* row_ptr, const int32_t* col, const int8_t* val, const int32_t* bias,
+                            anc_instance** out) {
+    return guarded([&] { return create_csr(n, row_ptr, col, val, bias, out); });
 }
 
 int anc_instance_get_info(const anc_instance* I, anc_instance_info* info) {
@@ -1475,14 +1499,14 @@ int anc_auto_choice(anc_instance* I, anc_tables* tb, int nchains, const anc_run_
 
 int anc_run(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, int nchains, const anc_run_opts* o,
             uint64_t* spins, int64_t* sum_sh, int64_t* sum_bs, int64_t* flips, int32_t* trace) {
-    return run_host_impl(I, tb, seed, off, nchains, o, spins, sum_sh, sum_bs, flips, trace, nullptr);
+    return guarded([&] { return run_host_impl(I, tb, seed, off, nchains, o, spins, sum_sh, sum_bs, flips, trace, nullptr); });
 }
 
 int anc_run_fields(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, int nchains, const anc_run_opts* o,
                    uint64_t* spins, int64_t* sum_sh, int64_t* sum_bs, int64_t* flips, int32_t* trace,
                    int32_t* fields) {
     if (!fields) return fail(ANC_EINVAL, "fields output required");
-    return run_host_impl(I, tb, seed, off, nchains, o, spins, sum_sh, sum_bs, flips, trace, fields);
+    return guarded([&] { return run_host_impl(I, tb, seed, off, nchains, o, spins, sum_sh, sum_bs, flips, trace, fields); });
 }
 
 int anc_run_device(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off, int nchains, const anc_run_opts* o,
@@ -1491,7 +1515,7 @@ int anc_run_device(anc_instance* I, anc_tables* tb, uint64_t seed, uint32_t off,
     OutPtrs out{reinterpret_cast<uint32_t*>(d_spins), reinterpret_cast<long long*>(d_sum_sh),
                 reinterpret_cast<long long*>(d_sum_bs), reinterpret_cast<long long*>(d_flips), d_trace, nullptr};
     if (!d_sum_bs) return fail(ANC_EINVAL, "sum_bs output required on the device path");
-    return run_device_impl(I, tb, seed, off, nchains, o, out, reinterpret_cast<cudaStream_t>(stream));
+    return guarded([&] { return run_device_impl(I, tb, seed, off, nchains, o, out, reinterpret_cast<cudaStream_t>(stream)); });
 }
 
 }  // extern "C"
@@ -1816,7 +1840,9 @@ int run_batch_impl(int njobs, const anc_job* jobs, const anc_run_opts* o, bool g
 
 }  // namespace
 
-extern "C" int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) { return run_batch_impl(njobs, jobs, o, true); }
+extern "C" int anc_run_batch(int njobs, const anc_job* jobs, const anc_run_opts* o) {
+    return guarded([&] { return run_batch_impl(njobs, jobs, o, true); });
+}
 
 
 // ---------------------------------------------------------------------------------------------------------------------
