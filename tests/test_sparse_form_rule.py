@@ -38,8 +38,8 @@ def test_forms_at_the_lines(cuda, oracle, n, degree, unit, chains):
     assert np.array_equal(r.fields[chains - 1], inst.fields(r.spins[chains - 1]))
 
 
-@pytest.mark.parametrize("n,degree,unit,chains", [(2000, 40, True, 310), (7900, 80, True, 310), (7900, 20, True, 1200),
-                                                  (16000, 20, True, 444), (10000, 80, True, 592), (800, 80, False, 310)])
+@pytest.mark.parametrize("n,degree,unit,chains", [(2000, 40, True, 310), (4000, 80, True, 310), (7900, 20, True, 1200),
+                                                  (16000, 20, True, 444), (10000, 48, True, 592), (800, 80, False, 310)])
 def test_not_slower_than_waves_of_one_per_sm(cuda, n, degree, unit, chains):
     inst = _graph(n, degree, unit)
     dev, tb = A.DeviceInstance(inst), A.Tables.from_schedule(A.Schedule(**SCHED, S=150))
